@@ -10,14 +10,15 @@ import sys
 PACKAGE_DIR = os.path.dirname(os.path.abspath(__file__))
 REPO_DIR = os.path.dirname(PACKAGE_DIR)
 CSRC = os.path.join(PACKAGE_DIR, "csrc")
-SOURCES = [os.path.join(CSRC, "engine.cu"), os.path.join(CSRC, "noalloc.cu"), os.path.join(CSRC, "server.cpp"),
-           os.path.join(CSRC, "format.cpp"), os.path.join(CSRC, "reader.cpp")]
-DEPENDS = SOURCES + [os.path.join(CSRC, f) for f in ("pw_device.cuh", "pw_kernels.cuh", "pw_score16.cuh", "pw_band.cuh", "pw_band16.cuh", "pw_tiles.cuh", "pw_plan.h", "pw_finish.cuh", "pw_host.h", "server.cpp")] + [
+SOURCES = [os.path.join(CSRC, f) for f in (
+    "engine.cu", "noalloc.cu", "score16_linear.cu", "score16_affine.cu", "score16_dual.cu",
+    "server.cpp", "format.cpp", "reader.cpp")]
+DEPENDS = SOURCES + [os.path.join(CSRC, f) for f in ("score16_variants.h", "pw_device.cuh", "pw_kernels.cuh", "pw_score16.cuh", "pw_band.cuh", "pw_band16.cuh", "pw_tiles.cuh", "pw_plan.h", "pw_finish.cuh", "pw_host.h", "server.cpp")] + [
     os.path.join(REPO_DIR, "include", "paswas_b200.h")]
 LIBRARY = os.path.join(PACKAGE_DIR, "libpaswas_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
-              "-Xcompiler", "-fPIC", "-shared", "-lpthread", "-Xptxas", "-O3"]
+              "-Xcompiler", "-fPIC", "-shared", "-lpthread", "-Xptxas", "-O3", "--threads", "0"]
 
 
 HITBUILD_SRC = os.path.join(CSRC, "hitbuild.c")

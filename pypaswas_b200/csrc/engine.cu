@@ -31,7 +31,7 @@
 
 #include "../../include/paswas_b200.h"
 #include "pw_kernels.cuh"
-#include "pw_score16.cuh"
+#include "score16_variants.h"
 #include "pw_band.cuh"
 #include "pw_tiles.cuh"
 #include "pw_band16.cuh"
@@ -260,7 +260,7 @@ struct pw_engine {
     HostBuf<uint8_t> h_stage;           // page-locked staging of the other per-set uploads (Staged)
     int64_t free_mem = 0;    // free device memory plus this engine's kept wave buffers, as last queried
     double free_mem_t = -1;  // wall_ms() of that query
-    DevBuf chain_items, chain_info, chain_prog, chain_max, chain_ring_off, chain_ring, chain_abort, p1_items, p1_grid;
+    DevBuf chain_info, chain_prog, chain_max, chain_ring_off, chain_ring, chain_abort, p1_items, p1_grid;
     // plan of the 16-bit score phase (work items, classes, chain queue), kept
     // on the device and reused while inputs, scoring, flags and tuning stay
     struct {
@@ -1044,39 +1044,46 @@ static std::vector<uint32_t> class_cost_order(const std::vector<int>& cls, const
 
 
 // ------------------------------------------------------------ 16-bit phase 1
-template <int S, bool AFF, bool MULTI, bool DL>
-static cudaError_t launch_s16(pw_engine* e, Score16Args A) {
-    auto kern = score16_kernel<S, AFF, MULTI, DL>;
-    const int smem = 4 * (S / 4) * A.alpha1 * prof_entry_bytes<DL>();
-    if (smem > 48 * 1024) {
-        cudaError_t c = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (c != cudaSuccess) return c;
-    }
-    int per_sm = 0;
-    cudaError_t c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
-    if (c != cudaSuccess) return c;
-    per_sm = std::max(1, std::min(per_sm, 16));
-    int grid = std::min(grid_cap(e, per_sm), (A.n_items + 3) / 4);
-    PW_LAUNCH(kern, std::max(grid, 1), 128, smem, e->stream, A);
-    e->launches++;
-    return cudaGetLastError();
+// The profile layout of the 16-bit sweep (Form16, pw_score16.cuh).  Up to 8
+// codes (DNA) no two residues' 128-bit entries meet in a bank group.  Above,
+// measured on proteins (20 residues): the linear sweep, which loads most per
+// clock, 701 x 701 proteins in 22.3 ms with 32-bit entries, 23.0 with 64-bit
+// and 25.2 with 128-bit ones; the affine sweep, 200 x 2000, 24.0 ms with
+// 64-bit, 25.4 with 32-bit and 24.0 with 128-bit entries (6 x 50,000: 4.55,
+// 4.97 and 4.71).
+static int s16_form(const pw_engine* e, bool trans, bool dual) {
+    const int alpha1 = (trans ? e->pr.alpha_t : e->pr.alpha) + 1;
+    if (dual) return kDual;
+    if (alpha1 <= 8) return kPair128;
+    return e->affine ? kPair64 : kPair32;
 }
 
-template <bool DL>
-static cudaError_t launch_s16_class(pw_engine* e, int cls, bool affine, const Score16Args& A) {
-    if (affine) {
-        if (cls == kS16) return launch_s16<16, true, false, DL>(e, A);
-        if (cls == kS24) return launch_s16<24, true, false, DL>(e, A);
-        if (cls == kS32) return launch_s16<32, true, false, DL>(e, A);
-        return launch_s16<32, true, true, DL>(e, A);
+static Score16Kernel s16_kernel(const pw_engine* e, int form, int rows, int alpha1) {
+    if (form == kDual) return score16_dual(e->affine != 0, rows, alpha1);
+    return e->affine ? score16_affine(form, rows, alpha1) : score16_linear(form, rows, alpha1);
+}
+
+// Resident blocks per SM of a kernel (its shared memory allowed first).
+static cudaError_t s16_blocks(const Score16Kernel& k, int* per_sm) {
+    if (!k.kern) return cudaErrorInvalidValue;
+    if (k.smem > 48 * 1024) {
+        cudaError_t c = cudaFuncSetAttribute(k.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem);
+        if (c != cudaSuccess) return c;
     }
-    if (cls == kS16) return launch_s16<16, false, false, DL>(e, A);
-    if (cls == kS24) return launch_s16<24, false, false, DL>(e, A);
-    if (cls == kS32) return launch_s16<32, false, false, DL>(e, A);
-    if (cls == kS40) return launch_s16<40, false, false, DL>(e, A);
-    if (cls == kS48) return launch_s16<48, false, false, DL>(e, A);
-    if (cls == kS64) return launch_s16<64, false, false, DL>(e, A);
-    return launch_s16<32, false, true, DL>(e, A);
+    cudaError_t c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k.kern, 128, k.smem);
+    *per_sm = std::max(1, std::min(*per_sm, 16));
+    return c;
+}
+
+static cudaError_t launch_s16(pw_engine* e, int form, int rows, const Score16Args& A) {
+    const Score16Kernel k = s16_kernel(e, form, rows, A.alpha1);
+    int per_sm = 0;
+    cudaError_t c = s16_blocks(k, &per_sm);
+    if (c != cudaSuccess) return c;
+    const int grid = std::max(1, std::min(grid_cap(e, per_sm), (A.n_items - A.item_base + 3) / 4));
+    PW_LAUNCH(k.kern, grid, 128, k.smem, e->stream, A);
+    e->launches++;
+    return cudaGetLastError();
 }
 
 // Plans the multi-strip launch.  Items whose sweep cost (columns x strips)
@@ -1101,53 +1108,32 @@ static int setup_chains(pw_engine* e, const std::vector<WorkItem>& items, int i0
     const int64_t permille = e->tune[PW_TUNE_CHAIN_MIN] > 0 ? e->tune[PW_TUNE_CHAIN_MIN] : 500;
     ChainPlan plan;
     plan_chain_queue(nstr, xm4, warps, permille, kChainLead, plan);
-    std::vector<WorkItem> q(plan.queue.size());
-    std::vector<int4> info(plan.queue.size());
-    for (size_t k = 0; k < plan.queue.size(); ++k) {
+    const size_t nq = plan.queue.size();
+    std::vector<int4> info(nq);
+    for (size_t k = 0; k < nq; ++k) {
         const PlanEntry& p = plan.queue[k];
-        q[k] = items[i0 + p.item];
-        info[k] = make_int4(p.chain, p.strip, p.pred, 0);
+        info[k] = make_int4(p.chain, p.strip, p.pred, p.item);
     }
     std::vector<int64_t> ring_off(std::max<size_t>(plan.chain_xm4.size(), 1), 0);
     int64_t ring_elems = 0;
     for (size_t c = 0; c < plan.chain_xm4.size(); ++c) {
         ring_off[c] = ring_elems;
-        ring_elems += 2 * plan.chain_xm4[c] * kWarp;
+        ring_elems += 2 * (e->affine ? ring_row<true>((int)plan.chain_xm4[c]) : ring_row<false>((int)plan.chain_xm4[c]));
     }
     cudaError_t c;
-    if ((c = upload(e, e->chain_items, q)) != cudaSuccess) return cuda_fail(e, c, "upload chain items");
     if ((c = upload(e, e->chain_info, info)) != cudaSuccess) return cuda_fail(e, c, "upload chain info");
-    e->h_chain_info = info;
+    e->h_chain_info.swap(info);
     if ((c = upload(e, e->chain_ring_off, ring_off)) != cudaSuccess) return cuda_fail(e, c, "upload ring offsets");
     // one progress flag per entry, plus one that no entry ever sets (PW_TUNE_STALL_TEST)
-    if ((c = e->chain_prog.reserve(e->stream, (q.size() + 1) * sizeof(int))) != cudaSuccess)
+    if ((c = e->chain_prog.reserve(e->stream, (nq + 1) * sizeof(int))) != cudaSuccess)
         return cuda_fail(e, c, "alloc chain progress");
-    if ((c = e->chain_max.reserve(e->stream, q.size() * kWarp * sizeof(uint32_t))) != cudaSuccess)
+    if ((c = e->chain_max.reserve(e->stream, nq * kWarp * sizeof(uint32_t))) != cudaSuccess)
         return cuda_fail(e, c, "alloc chain maxima");
     if ((c = e->chain_ring.reserve(e->stream, (size_t)std::max<int64_t>(ring_elems, 1) * sizeof(uint4))) != cudaSuccess)
         return cuda_fail(e, c, "alloc chain ring");
     if ((c = e->chain_abort.reserve(e->stream, sizeof(int))) != cudaSuccess) return cuda_fail(e, c, "alloc chain status");
-    *n_entries = (int)q.size();
+    *n_entries = (int)nq;
     return PW_OK;
-}
-
-template <int S, bool AFF, bool DL>
-static cudaError_t launch_s16_chain(pw_engine* e, Score16Args A) {
-    auto kern = score16_chain_kernel<S, AFF, DL>;
-    // the four warps' profiles, then (affine) their prefetch rings of the row above
-    const int smem = chain_profile_bytes<S, DL>(A.alpha1) + (AFF ? 4 * kPre * kWarp * (int)sizeof(uint4) : 0);
-    if (smem > 48 * 1024) {
-        cudaError_t c = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (c != cudaSuccess) return c;
-    }
-    int per_sm = 0;
-    cudaError_t c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem);
-    if (c != cudaSuccess) return c;
-    per_sm = std::max(1, std::min(per_sm, 16));
-    const int grid = std::max(1, std::min(grid_cap(e, per_sm), (A.n_items - A.item_base + 3) / 4));
-    PW_LAUNCH(kern, grid, 128, smem, e->stream, A);
-    e->launches++;
-    return cudaGetLastError();
 }
 
 // Cell-slot cost of an orientation: strips are paired in length order (one
@@ -1294,15 +1280,10 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
         if (P1.chained) {
             int per_sm = 0;
             const int a1 = (trans ? pr.alpha_t : pr.alpha) + 1;
-            const int smem = (dual ? chain_profile_bytes<32, true>(a1) : chain_profile_bytes<32, false>(a1)) +
-                             (e->affine ? 4 * kPre * kWarp * (int)sizeof(uint4) : 0);
-            auto kern = e->affine ? (dual ? score16_chain_kernel<32, true, true> : score16_chain_kernel<32, true, false>)
-                                  : (dual ? score16_chain_kernel<32, false, true> : score16_chain_kernel<32, false, false>);
-            if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            if ((c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem)) != cudaSuccess)
+            if ((c = s16_blocks(s16_kernel(e, s16_form(e, trans, dual), -1, a1), &per_sm)) != cudaSuccess)
                 return cuda_fail(e, c, "occupancy");
             const int rc = setup_chains(e, it2, begin[kS32Multi], begin[kS32Multi + 1], strip_len,
-                                        grid_cap(e, std::max(1, std::min(per_sm, 16))) * 4, &P1.n_chain_items);
+                                        grid_cap(e, per_sm) * 4, &P1.n_chain_items);
             if (rc != PW_OK) return rc;
         }
         P1.trans = trans;
@@ -1342,14 +1323,14 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
     S.dim = e->dim;
     S.gap = (int)e->gap;
     S.ext = (int)e->ext;
-    S.ge = S.gap + S.ext;
+    const int form = s16_form(e, trans, dual);
     S.pair_max = A32.pair_max;
     S.stride_strip = trans ? nt : 1;
     S.stride_lane = trans ? 1 : nt;
     S.pad_code = S.alpha1 - 1;
     S.wait_ns = wait_limit(e);
     if (begin[kS32Multi + 1] > begin[kS32Multi]) {
-        const int64_t slot = (int64_t)P1.xm_multi * kWarp;
+        const int64_t slot = 2 * (e->affine ? ring_row<true>(P1.xm_multi) : ring_row<false>(P1.xm_multi));
         if ((c = e->bnd_pool.reserve(e->stream, (size_t)slot * e->sm_count * 16 * 4 * sizeof(uint4))) != cudaSuccess)
             return cuda_fail(e, c, "alloc boundary pool");
         S.bnd_pool = e->bnd_pool.as<uint4>();
@@ -1393,7 +1374,7 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
         if (k == kS32Multi && chained) {
             // the queue in consecutive segments, one launch each (PW_TUNE_SEGMENT):
             // every strip's predecessor is in the same or an earlier segment
-            S.items = e->chain_items.as<WorkItem>();
+            S.items = e->p1_items.as<WorkItem>() + begin[k];
             S.counter = e->counter.as<int>() + k;
             const int total = S.n_chain_items;
             const int seg = e->tune[PW_TUNE_SEGMENT] > 0 ? (int)std::min<int64_t>(e->tune[PW_TUNE_SEGMENT], total)
@@ -1403,8 +1384,7 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
                 S.n_items = std::min(total, base + std::max(seg, 1));
                 if (base > 0 && (c = cudaMemsetAsync(S.counter, 0, sizeof(int), e->stream)) != cudaSuccess)
                     return cuda_fail(e, c, "reset counter");
-                c = e->affine ? (dual ? launch_s16_chain<32, true, true>(e, S) : launch_s16_chain<32, true, false>(e, S))
-                              : (dual ? launch_s16_chain<32, false, true>(e, S) : launch_s16_chain<32, false, false>(e, S));
+                c = launch_s16(e, form, -1, S);
                 if (c != cudaSuccess) return cuda_fail(e, c, "score16 chain launch");
                 inf.score_launches++;
             }
@@ -1413,8 +1393,9 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
         S.items = e->p1_items.as<WorkItem>() + begin[k];
         S.n_items = n;
         S.counter = e->counter.as<int>() + k;
+        S.item_base = 0;
         S.grid_strips = nullptr;
-        c = dual ? launch_s16_class<true>(e, k, e->affine, S) : launch_s16_class<false>(e, k, e->affine, S);
+        c = launch_s16(e, form, k == kS32Multi ? 0 : class_S(k), S);
         if (c != cudaSuccess) return cuda_fail(e, c, "score16 launch");
         inf.score_launches++;
     }
@@ -1428,7 +1409,8 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
         S.grid_n_lane = trans ? nt : nq;
         S.n_items = (int)((int64_t)np_ * P1.n_groups);
         S.counter = e->counter.as<int>() + k;
-        c = dual ? launch_s16_class<true>(e, k, e->affine, S) : launch_s16_class<false>(e, k, e->affine, S);
+        S.item_base = 0;
+        c = launch_s16(e, form, class_S(k), S);
         if (c != cudaSuccess) return cuda_fail(e, c, "score16 launch");
         inf.score_launches++;
     }

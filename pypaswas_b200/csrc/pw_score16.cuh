@@ -6,11 +6,21 @@
 // which update two cells per instruction at the rate of one 32-bit update.
 // A warp aligns two "strip" sequences (low and high halves) against up to 32
 // "lane" sequences, one per lane.  Both halves of a lane read the same lane
-// residue, so the strip profile stores ready-made 16x2 score pairs: one
-// 128-bit shared-memory load yields the scores of four strip rows for both
-// strip sequences.  Which input set provides the strips and which the lanes
-// is chosen per run by the host (pair maxima are symmetric in the two
-// sequences, so either orientation gives the same maxima).
+// residue, so the strip profile stores ready-made 16x2 score pairs.  Which
+// input set provides the strips and which the lanes is chosen per run by the
+// host (pair maxima are symmetric in the two sequences, so either orientation
+// gives the same maxima).
+//
+// What bounds it: the DPX instructions, 64 lanes a clock and SM on the ALU
+// pipe.  A packed add (__vadd2) issues beside them on the FMA pipe at the same
+// rate (measured: 64 lanes alone, 120 when it alternates with a DPX add-max),
+// so the adds that need no maximum of their own leave the ALU pipe:
+//   linear  diagonal + score; 2 DPX + 1 add a row pair (3 DPX before);
+//           registers only, 6 warps a scheduler: 6.2 clocks a row, 7.5 before
+//   affine  diagonal + score and M + gap + ext, with the floor at 0 in the
+//           three-way maximum of B instead of in M; 3 DPX + 2 adds (5 DPX
+//           before); 9.0 clocks a row, 12.4 before
+// (plus half a three-way maximum a row for the pair maximum in both).
 //
 // Overflow: with every score in [-127, 127], no 16-bit operation can exceed
 // 32767 while all cell values stay below kOvf16 (32640 = 32767 - 127).  A pair
@@ -29,8 +39,19 @@ __device__ __forceinline__ uint32_t pack16x2(int lo, int hi) {
     return ((uint32_t)lo & 0xffffu) | ((uint32_t)hi << 16);
 }
 
+// The profile's layout: which load fetches the scores of a lane's residue.
+//   kPair128  one uint4 holds 4 rows (16x2 words): for alphabets whose
+//             residues' uint4 fall into different bank groups (8 codes)
+//   kPair64   one uint2 holds 2 rows: with more residues a quarter warp's
+//             128-bit loads meet in a bank group about twice (20 amino acids),
+//             a half warp's 64-bit loads less often
+//   kDual     the dual-lane form: one uint2 holds 4 rows of plain 16-bit scores
+//   kPair32   one word holds a row: no two residues of up to 32 share a bank
+enum Form16 { kPair128 = 0, kPair64 = 1, kDual = 2, kPair32 = 3 };
+
 struct Score16Args {
     const WorkItem* items;   // target = strip A, index = strip B (or -1), first/lanes index the lane order
+                             // (chained launch: the items that the queue entries name)
     int n_items;
     int* counter;
     const uint8_t* lane_codes;   // compact lane-alphabet codes, 16-aligned, pad-coded tail
@@ -42,16 +63,16 @@ struct Score16Args {
     const int32_t* strip_len;
     const int8_t* cmat;          // [(alpha + 1) * dim] scores lane residue x strip residue
     int alpha1, dim;
-    int gap, ext, ge;
+    int gap, ext;
     float* pair_max;
     int64_t stride_strip, stride_lane;  // pair_max[strip * stride_strip + lane * stride_lane]
     uint4* bnd_pool;
-    int64_t bnd_slot;            // uint4 elements per warp slot (xmax4 * 32)
+    int64_t bnd_slot;            // uint4 elements per warp slot (two boundary rows, see ring_row)
     // multi-strip launch with chains (score16_chain_kernel): per queue entry
-    // (chain, strip, queue index of the chain's previous strip); strip -1 marks
-    // a whole item swept by one warp with its boundary in bnd_pool
+    // (chain, strip, queue index of the chain's previous strip, item); strip -1
+    // marks a whole item swept by one warp with its boundary in bnd_pool
     const int4* chain;
-    const int64_t* ring_off;     // per chain: its two boundary rows (xm4 * 32 uint4 each) in `ring`
+    const int64_t* ring_off;     // per chain: its two boundary rows (ring_row uint4 each) in `ring`
     uint4* ring;
     int* progress;               // per queue entry: columns whose boundary row is written (kChainDone when finished)
     uint32_t* run_max;           // per queue entry x 32 lanes: running 16x2 maximum of the chain so far
@@ -71,62 +92,83 @@ struct Score16Args {
     int grid_n_lane;             // lane sequences in the sorted order
 };
 
-// Profile of strip rows [y0, y0 + S): for row group g (4 rows) and lane
-// residue a, one uint4 holds the 16x2 scores of the 4 rows, strip A in the low
-// halves and strip B in the high halves.  Rows past a strip's end get -128.
-// Affine sweeps store score + gap_open in the halves (see sweep16).
-template <int S>
-__device__ __forceinline__ void build_profile16(uint4* prof, const int8_t* cmat, const uint8_t* ra,
+// Rows a profile entry holds, entry bytes, and entries a residue: a residue's
+// entries lie together, so that a column's loads differ by constants, and one
+// entry of padding makes their number odd, so that residues differ in bank
+// group as their codes do.
+template <int FORM>
+__host__ __device__ constexpr int prof_rows() { return FORM == kPair32 ? 1 : FORM == kPair64 ? 2 : 4; }
+template <int FORM>
+__host__ __device__ constexpr int prof_entry_bytes() {
+    return FORM == kPair128 ? (int)sizeof(uint4) : FORM == kPair32 ? (int)sizeof(uint32_t) : (int)sizeof(uint2);
+}
+template <int S, int FORM>
+__host__ __device__ constexpr int prof_stride() { return (S / prof_rows<FORM>()) | 1; }
+
+// Bytes of one warp's profile (a multiple of 16) and of a block's four.
+template <int S, int FORM>
+__host__ __device__ constexpr int warp_profile_bytes(int alpha1) {
+    return (alpha1 * prof_stride<S, FORM>() * prof_entry_bytes<FORM>() + 15) & ~15;
+}
+template <int S, int FORM>
+__host__ __device__ constexpr int block_profile_bytes(int alpha1) { return 4 * warp_profile_bytes<S, FORM>(alpha1); }
+
+// Profile of strip rows [y0, y0 + S): the scores of lane residue a, strip A in
+// the low halves and strip B in the high halves (dual-lane form: strip A's
+// plain 16-bit scores).  Rows past a strip's end get -128.
+template <int S, int FORM>
+__device__ __forceinline__ void build_profile16(unsigned char* prof, const int8_t* cmat, const uint8_t* ra,
                                                 const uint8_t* rb, int y0, int la, int lb, int alpha1, int dim,
-                                                int shift, int lane) {
-    const int n = (S / 4) * alpha1;
+                                                int lane) {
+    constexpr int R = prof_rows<FORM>(), G = S / R, stride = prof_stride<S, FORM>();
+    const int n = G * alpha1;
     for (int idx = lane; idx < n; idx += kWarp) {
-        const int g = idx / alpha1, a = idx % alpha1;
+        const int a = idx / G, g = idx % G;
         uint32_t w[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int y = y0 + 4 * g + k;
+        for (int k = 0; k < R; ++k) {
+            const int y = y0 + R * g + k;
             const int sa = y < la ? (int)cmat[a * dim + ra[y]] : -128;
-            const int sb = y < lb ? (int)cmat[a * dim + rb[y]] : -128;
-            w[k] = pack16x2(sa + shift, sb + shift);
+            if constexpr (FORM == kDual) {
+                w[k] = (uint32_t)sa;
+            } else {
+                const int sb = y < lb ? (int)cmat[a * dim + rb[y]] : -128;
+                w[k] = pack16x2(sa, sb);
+            }
         }
-        prof[idx] = make_uint4(w[0], w[1], w[2], w[3]);
+        if constexpr (FORM == kPair128)
+            ((uint4*)prof)[a * stride + g] = make_uint4(w[0], w[1], w[2], w[3]);
+        else if constexpr (FORM == kPair32)
+            ((uint32_t*)prof)[a * stride + g] = w[0];
+        else if constexpr (FORM == kPair64)
+            ((uint2*)prof)[a * stride + g] = make_uint2(w[0], w[1]);
+        else
+            ((uint2*)prof)[a * stride + g] = make_uint2(pack16x2((int)w[0], (int)w[1]), pack16x2((int)w[2], (int)w[3]));
     }
 }
 
-// Dual-lane form: one strip sequence against two lane sequences per lane (the
-// lanes' own group in the low halves, the next 32-lane group in the high
-// halves).  The halves then read different lane residues, so the profile
-// holds plain 16-bit scores, [row group][lane residue] -> 4 rows in a uint2,
-// and the sweep interleaves the two residues' words with byte permutes.
-template <int S>
-__device__ __forceinline__ void build_profile16_dual(uint2* prof, const int8_t* cmat, const uint8_t* ra, int y0,
-                                                     int la, int alpha1, int dim, int shift, int lane) {
-    const int n = (S / 4) * alpha1;
-    for (int idx = lane; idx < n; idx += kWarp) {
-        const int g = idx / alpha1, a = idx % alpha1;
-        int v[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int y = y0 + 4 * g + k;
-            v[k] = (y < la ? (int)cmat[a * dim + ra[y]] : -128) + shift;
-        }
-        prof[idx] = make_uint2(pack16x2(v[0], v[1]), pack16x2(v[2], v[3]));
-    }
-}
-
-// The 16x2 scores of rows 4g .. 4g + 3: profile entries `ia` (low halves) and
-// `ib` (high halves; the dual-lane form only).
-template <bool DL>
-__device__ __forceinline__ void fetch16(const void* prof, int ia, int ib, uint32_t (&sc)[4]) {
-    if constexpr (!DL) {
-        const uint4 w = ((const uint4*)prof)[ia];
+// The 16x2 scores of rows 4g .. 4g + 3 from the entries of the lane's residue
+// (low halves; `pb`: the high halves' residue, the dual-lane form only, whose
+// halves read different residues and are interleaved with byte permutes).
+template <int FORM>
+__device__ __forceinline__ void fetch16(const void* pa, const void* pb, int g, uint32_t (&sc)[4]) {
+    if constexpr (FORM == kPair128) {
+        const uint4 w = ((const uint4*)pa)[g];
         sc[0] = w.x;
         sc[1] = w.y;
         sc[2] = w.z;
         sc[3] = w.w;
+    } else if constexpr (FORM == kPair32) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sc[k] = ((const uint32_t*)pa)[4 * g + k];
+    } else if constexpr (FORM == kPair64) {
+        const uint2 u = ((const uint2*)pa)[2 * g], v = ((const uint2*)pa)[2 * g + 1];
+        sc[0] = u.x;
+        sc[1] = u.y;
+        sc[2] = v.x;
+        sc[3] = v.y;
     } else {
-        const uint2 lo = ((const uint2*)prof)[ia], hi = ((const uint2*)prof)[ib];
+        const uint2 lo = ((const uint2*)pa)[g], hi = ((const uint2*)pb)[g];
         sc[0] = __byte_perm(lo.x, hi.x, 0x5410);
         sc[1] = __byte_perm(lo.x, hi.x, 0x7632);
         sc[2] = __byte_perm(lo.y, hi.y, 0x5410);
@@ -134,149 +176,64 @@ __device__ __forceinline__ void fetch16(const void* prof, int ia, int ib, uint32
     }
 }
 
-template <bool DL>
-__host__ __device__ constexpr int prof_entry_bytes() { return DL ? (int)sizeof(uint2) : (int)sizeof(uint4); }
-
-// Bytes of the four warps' profiles of a 128-thread block, rounded to 16.
-template <int S, bool DL>
-__host__ __device__ constexpr int chain_profile_bytes(int alpha1) {
-    return (4 * (S / 4) * alpha1 * prof_entry_bytes<DL>() + 15) & ~15;
-}
-
-// This warp's profile in shared memory (typed offsets keep the address a
-// 32-bit shared-window computation).
-template <int S, bool DL>
-__device__ __forceinline__ void* warp_profile(unsigned char* smem, int wib, int alpha1) {
-    if constexpr (DL) return (uint2*)smem + wib * ((S / 4) * alpha1);
-    else return (uint4*)smem + wib * ((S / 4) * alpha1);
-}
-
-// One lane, two pairs (strip A / strip B against the lane sequence).
-//   linear: H = max(diag + s, left + gap, up + gap, 0)                 3 DPX / row
-//   affine: carries Mg = M + gap_open (gap_open = gap + ext):
-//     M  = max(Bdiag + s, 0)          Mg = M + ge  (profile holds s + ge,
-//     so Mg = max(Bdiag + (s + ge), ge) in one instruction)
-//     Y  = max(Yup + ext, Mg_up)      strip-axis gap chain
-//     X  = max(Xleft + ext, Mg_left)  sweep-axis gap chain
-//     B  = max(Mg - ge, Y, X)          as max(M, Y, X)                 5 DPX / row
-//
-// Dual-lane form (DL): the high halves sweep a second lane sequence (qc2,
-// lq42) against the same strip; the column loop runs to the longer of the two
-// and a sequence past its end reads padding codes (pad4), which cannot raise
-// its maximum.
-template <int S, bool AFFINE, bool DL>
-__device__ __forceinline__ void sweep16(const uint8_t* qc, int lq4, const uint8_t* qc2, int lq42, uint32_t pad4,
-                                        const void* prof, int alpha1, int gap, int ext, int ge, bool has_up,
-                                        bool has_down, uint4* bnd, uint32_t& mx) {
-    const uint32_t g2 = pack16(gap), e2 = pack16(ext), ge2 = pack16(ge), nge2 = pack16(-ge);
-    auto word = [&](const uint8_t* q, int lim, int x4) -> uint32_t {
-        return !DL || x4 < lim ? *(const uint32_t*)(q + x4) : pad4;
-    };
-    const int lqa = lq4;  // the low halves' own columns
-    if constexpr (DL) lq4 = lq4 > lq42 ? lq4 : lq42;
-    if constexpr (!AFFINE) {
-        uint32_t H[S];
+// One column of a linear strip: H of the previous column in, of this one out.
+//   H = max(diag + s, left + gap, up + gap, 0)
+template <int S, int FORM>
+__device__ __forceinline__ void column16_linear(uint32_t (&H)[S], uint32_t diag, uint32_t up, const void* pa,
+                                                const void* pb, uint32_t g2, uint32_t& mx) {
 #pragma unroll
-        for (int r = 0; r < S; ++r) H[r] = 0;
-        uint32_t hb_prev = 0;
-        // the code word of the next 4 columns and the boundary value of the
-        // next column are loaded one step ahead (their latency hides behind a
-        // column of arithmetic)
-        uint32_t cw_next = lq4 > 0 ? word(qc, lqa, 0) : 0u;
-        uint32_t cw2_next = DL && lq4 > 0 ? word(qc2, lq42, 0) : 0u;
-        uint32_t up_next = has_up && lq4 > 0 ? bnd[0].x : 0u;
-        for (int x4 = 0; x4 < lq4; x4 += 4) {
-            const uint32_t cw = cw_next, cw2 = cw2_next;
-            if (x4 + 4 < lq4) {
-                cw_next = word(qc, lqa, x4 + 4);
-                if constexpr (DL) cw2_next = word(qc2, lq42, x4 + 4);
-            }
+    for (int g = 0; g < S / 4; ++g) {
+        uint32_t sc[4];
+        fetch16<FORM>(pa, pb, g, sc);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int x = x4 + j;
-                const int a = (cw >> (8 * j)) & 0xff;
-                const int a2 = DL ? (cw2 >> (8 * j)) & 0xff : 0;
-                uint32_t up = up_next;
-                if (has_up && x + 1 < lq4) up_next = bnd[(int64_t)(x + 1) * kWarp].x;
-                uint32_t diag = hb_prev;
-                hb_prev = up;
-#pragma unroll
-                for (int g = 0; g < S / 4; ++g) {
-                    uint32_t sc[4];
-                    fetch16<DL>(prof, g * alpha1 + a, g * alpha1 + a2, sc);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int r = 4 * g + k;
-                        const uint32_t left = H[r];
-                        uint32_t t = __viaddmax_s16x2(diag, sc[k], kNeg16x2);   // diag + s
-                        t = __viaddmax_s16x2(left, g2, t);                      // max(left + gap, .)
-                        const uint32_t h = __viaddmax_s16x2_relu(up, g2, t);    // max(up + gap, ., 0)
-                        diag = left;
-                        H[r] = h;
-                        up = h;
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < S; r += 2) mx = __vimax3_s16x2(mx, H[r], H[r + 1]);
-                if (has_down) bnd[(int64_t)x * kWarp].x = H[S - 1];
-            }
-        }
-    } else {
-        // Zl[r] = max(X + ext, M + gap_open) of the previous column: exactly
-        // this column's X (the sweep-axis gap chain), one row array instead of
-        // two (X and M + gap_open); M = 0 and X = -inf left of the matrix
-        uint32_t Zl[S], Bl[S];
-#pragma unroll
-        for (int r = 0; r < S; ++r) {
-            Zl[r] = ge2;
-            Bl[r] = 0;
-        }
-        uint32_t bb_prev = 0;
-        uint32_t cw_next = lq4 > 0 ? word(qc, lqa, 0) : 0u;
-        uint32_t cw2_next = DL && lq4 > 0 ? word(qc2, lq42, 0) : 0u;
-        uint4 v_next = has_up && lq4 > 0 ? bnd[0] : make_uint4(ge2, kNeg16x2, 0u, 0u);
-        uint4 v_next2 = has_up && lq4 > 1 ? bnd[kWarp] : make_uint4(ge2, kNeg16x2, 0u, 0u);
-        for (int x4 = 0; x4 < lq4; x4 += 4) {
-            const uint32_t cw = cw_next, cw2 = cw2_next;
-            if (x4 + 4 < lq4) {
-                cw_next = word(qc, lqa, x4 + 4);
-                if constexpr (DL) cw2_next = word(qc2, lq42, x4 + 4);
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int x = x4 + j;
-                const int a = (cw >> (8 * j)) & 0xff;
-                const int a2 = DL ? (cw2 >> (8 * j)) & 0xff : 0;
-                const uint4 v = v_next;
-                v_next = v_next2;
-                if (has_up && x + 2 < lq4) v_next2 = bnd[(int64_t)(x + 2) * kWarp];
-                uint32_t mgup = v.x, yup = v.y, bup = v.z;
-                uint32_t bdiag = bb_prev;
-                bb_prev = bup;
-#pragma unroll
-                for (int g = 0; g < S / 4; ++g) {
-                    uint32_t sc[4];
-                    fetch16<DL>(prof, g * alpha1 + a, g * alpha1 + a2, sc);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int r = 4 * g + k;
-                        const uint32_t mg = __viaddmax_s16x2(bdiag, sc[k], ge2);   // M + ge
-                        const uint32_t y = __viaddmax_s16x2(yup, e2, mgup);
-                        const uint32_t xg = Zl[r];
-                        const uint32_t bst = __vimax3_s16x2(__viaddmax_s16x2(mg, nge2, kNeg16x2), y, xg);
-                        Zl[r] = __viaddmax_s16x2(xg, e2, mg);
-                        bdiag = Bl[r];
-                        Bl[r] = bst;
-                        mgup = mg;
-                        yup = y;
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < S; r += 2) mx = __vimax3_s16x2(mx, Bl[r], Bl[r + 1]);
-                if (has_down) bnd[(int64_t)x * kWarp] = make_uint4(mgup, yup, Bl[S - 1], 0u);
-            }
+        for (int k = 0; k < 4; ++k) {
+            const int r = 4 * g + k;
+            const uint32_t left = H[r];
+            uint32_t h = __viaddmax_s16x2(left, g2, __vadd2(diag, sc[k]));
+            h = __viaddmax_s16x2_relu(up, g2, h);
+            diag = left;
+            H[r] = h;
+            up = h;
         }
     }
+#pragma unroll
+    for (int r = 0; r < S; r += 2) mx = __vimax3_s16x2(mx, H[r], H[r + 1]);
+}
+
+// One column of an affine strip.
+//   M  = Bdiag + s
+//   Y  = max(Yup + ext, Mg_up)      strip-axis gap chain, Mg = M + gap + ext
+//   X  = Zl                         sweep-axis gap chain, computed a column ago:
+//                                   Zl = max(X + ext, Mg) is the next column's X
+//   B  = max(M, Y, X, 0)
+// The reference floors M at 0 before the gaps open from it; a gap opened from
+// a floored M is negative, as is one opened from the M below 0 here, and what
+// is negative never reaches B >= 0, so every B is the same.
+// In: Zl, Bl of the previous column, the first row's Y (y) and the diagonal B.
+// Out: this column's; in y the Y of the row below the strip.
+template <int S, int FORM>
+__device__ __forceinline__ void column16_affine(uint32_t (&Zl)[S], uint32_t (&Bl)[S], uint32_t bdiag, uint32_t& y,
+                                                const void* pa, const void* pb, uint32_t e2, uint32_t ge2,
+                                                uint32_t& mx) {
+#pragma unroll
+    for (int g = 0; g < S / 4; ++g) {
+        uint32_t sc[4];
+        fetch16<FORM>(pa, pb, g, sc);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int r = 4 * g + k;
+            const uint32_t m = __vadd2(bdiag, sc[k]);
+            const uint32_t xg = Zl[r];
+            const uint32_t bst = __vimax3_s16x2_relu(m, y, xg);
+            const uint32_t mg = __vadd2(m, ge2);
+            Zl[r] = __viaddmax_s16x2(xg, e2, mg);
+            y = __viaddmax_s16x2(y, e2, mg);
+            bdiag = Bl[r];
+            Bl[r] = bst;
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < S; r += 2) mx = __vimax3_s16x2(mx, Bl[r], Bl[r + 1]);
 }
 
 // ------------------------------------------------------------ chained strips
@@ -314,12 +271,19 @@ constexpr int kChainLead = 64;
 constexpr int kChainNeed = 40;
 // Default bound of one wait (PW_TUNE_WAIT_NS overrides it per launch).
 constexpr unsigned long long kChainWaitNs = 2000000000ull;
-// Columns of the ring row above that the affine chained sweep keeps in
-// flight: each lane copies its own 16-byte entry into a per-warp shared-memory
-// ring with cp.async, kPre - 1 columns ahead of the column it computes (within
-// the kChainNeed columns the chain wait guarantees).
-constexpr int kPre = 8;
-static_assert(kPre - 1 < kChainNeed - 4, "prefetched columns must be published");
+// Boundary rows: per block of four columns and lane 16 bytes (linear: H of the
+// strip's last row) or 32 (affine: B of the last row and Y of the row below
+// it, which is all that the next strip needs), so that a lane stores and loads
+// a block with one or two 128-bit accesses.
+template <bool AFFINE>
+__host__ __device__ constexpr int64_t ring_row(int xm4) { return (int64_t)(xm4 / 4) * kWarp * (AFFINE ? 2 : 1); }
+// The affine sweep keeps the row above kPreBlocks - 1 column blocks in flight:
+// each lane copies its own two entries into a per-warp shared-memory ring with
+// cp.async (within the kChainNeed columns the chain wait guarantees); the
+// linear sweep loads its one entry a block ahead into registers.
+constexpr int kPreBlocks = 3;
+constexpr int kPreBytes = kPreBlocks * 2 * kWarp * (int)sizeof(uint4);  // per warp
+static_assert(4 * kPreBlocks <= kChainNeed, "prefetched columns must be published");
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
@@ -374,90 +338,85 @@ __device__ __forceinline__ void chain_publish(int* flag, int v) {
     if ((threadIdx.x & 31) == 0) st_release_gpu(flag, v);
 }
 
-// sweep16 for one strip of a chain.  The column loop runs to the warp's
-// longest lane (xm4, warp-uniform); a lane past its own sequence sweeps
-// padding-code columns, which cannot raise its maximum.  Returns false when a
-// wait gave up.
-template <int S, bool AFFINE, bool DL>
-__device__ __forceinline__ bool sweep16_chain(const uint8_t* qc, int lq4, const uint8_t* qc2, int lq42, int xm4,
-                                              uint32_t pad4, const void* prof, int alpha1, int gap, int ext, int ge,
-                                              bool has_up, bool has_down, const uint4* ring_in, uint4* ring_out,
-                                              const int* prog_in, int* prog_out, int* abort_flag,
-                                              unsigned long long wait_ns, uint4* pre, uint32_t& mx) {
-    const uint32_t g2 = pack16(gap), e2 = pack16(ext), ge2 = pack16(ge), nge2 = pack16(-ge);
-    int avail = 0;  // columns of the predecessor known to be published
-    auto need_cols = [&](int upto) -> bool {  // columns [0, upto) of ring_in readable
-        if (!has_up || avail >= upto) return true;
+// One strip of an item: a lane, two pairs (strip A / strip B against the lane
+// sequence).  The column loop runs to the warp's longest lane (xm4,
+// warp-uniform); a lane past its own sequence sweeps padding-code columns,
+// which cannot raise its maximum (in the dual-lane form the high halves'
+// second lane sequence, qc2 / lq42, likewise).  BND: the strip may have a strip
+// above (has_up, its last row in row_in) and one below (has_down, row_out);
+// with prog_in / prog_out they run on other warps.  Returns false when a wait
+// gave up.
+template <int S, bool AFFINE, int FORM, bool BND>
+__device__ __forceinline__ bool sweep16(const uint8_t* qc, int lq4, const uint8_t* qc2, int lq42, int xm4,
+                                        uint32_t pad4, const unsigned char* prof, int gap, int ext, bool has_up,
+                                        bool has_down, const uint4* row_in, uint4* row_out, const int* prog_in,
+                                        int* prog_out, int* abort_flag, unsigned long long wait_ns, uint4* pre,
+                                        uint32_t& mx) {
+    constexpr bool DL = FORM == kDual;
+    constexpr int kResidue = prof_stride<S, FORM>() * prof_entry_bytes<FORM>();  // profile bytes a residue
+    const uint32_t g2 = pack16(gap), e2 = pack16(ext), ge2 = pack16(gap + ext);
+    int avail = 0;  // columns of the strip above known to be published
+    auto need_cols = [&](int upto) -> bool {  // columns [0, upto) of row_in readable
+        if (!BND || !prog_in || avail >= upto) return true;
         avail = chain_wait(prog_in, upto, abort_flag, wait_ns);
         return avail >= 0;
     };
     auto code_word = [&](int x4) -> uint32_t { return x4 < lq4 ? *(const uint32_t*)(qc + x4) : pad4; };
     auto code_word2 = [&](int x4) -> uint32_t { return DL && x4 < lq42 ? *(const uint32_t*)(qc2 + x4) : pad4; };
     if (!need_cols(min(kChainLead, xm4))) return false;
+    // the code words of the next 4 columns and the row above's entries are
+    // loaded ahead (their latency hides behind the columns' arithmetic)
+    uint32_t cw_next = code_word(0), cw2_next = code_word2(0);
+    uint32_t prev = 0;  // the row above, one column back: the first row's diagonal
     if constexpr (!AFFINE) {
         uint32_t H[S];
 #pragma unroll
         for (int r = 0; r < S; ++r) H[r] = 0;
-        uint32_t hb_prev = 0;
-        uint32_t cw_next = xm4 > 0 ? code_word(0) : pad4;
-        uint32_t cw2_next = DL && xm4 > 0 ? code_word2(0) : pad4;
-        uint32_t up_next = has_up && xm4 > 0 ? __ldcg(&ring_in[0]).x : 0u;
+        uint4 in_next = BND && has_up && xm4 > 0 ? __ldcg(row_in) : make_uint4(0u, 0u, 0u, 0u);
         for (int x4 = 0; x4 < xm4; x4 += 4) {
             if (!need_cols(min(x4 + kChainNeed, xm4))) return false;
             const uint32_t cw = cw_next, cw2 = cw2_next;
-            if (x4 + 4 < xm4) {
-                cw_next = code_word(x4 + 4);
-                if constexpr (DL) cw2_next = code_word2(x4 + 4);
-            }
+            const uint4 in = in_next;
+            cw_next = code_word(x4 + 4);
+            if constexpr (DL) cw2_next = code_word2(x4 + 4);
+            if (BND && has_up && x4 + 4 < xm4) in_next = __ldcg(row_in + (x4 / 4 + 1) * kWarp);
+            uint32_t out[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const int x = x4 + j;
-                const int a = (cw >> (8 * j)) & 0xff;
-                const int a2 = DL ? (cw2 >> (8 * j)) & 0xff : 0;
-                uint32_t up = up_next;
-                if (has_up && x + 1 < xm4) up_next = __ldcg(&ring_in[(int64_t)(x + 1) * kWarp]).x;
-                uint32_t diag = hb_prev;
-                hb_prev = up;
-#pragma unroll
-                for (int g = 0; g < S / 4; ++g) {
-                    uint32_t sc[4];
-                    fetch16<DL>(prof, g * alpha1 + a, g * alpha1 + a2, sc);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int r = 4 * g + k;
-                        const uint32_t left = H[r];
-                        uint32_t t = __viaddmax_s16x2(diag, sc[k], kNeg16x2);
-                        t = __viaddmax_s16x2(left, g2, t);
-                        const uint32_t h = __viaddmax_s16x2_relu(up, g2, t);
-                        diag = left;
-                        H[r] = h;
-                        up = h;
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < S; r += 2) mx = __vimax3_s16x2(mx, H[r], H[r + 1]);
-                if (has_down) __stcg(&ring_out[(int64_t)x * kWarp], make_uint4(H[S - 1], 0u, 0u, 0u));
+                const void* pa = prof + ((cw >> (8 * j)) & 0xff) * kResidue;
+                const void* pb = DL ? prof + ((cw2 >> (8 * j)) & 0xff) * kResidue : pa;
+                const uint32_t up = j == 0 ? in.x : j == 1 ? in.y : j == 2 ? in.z : in.w;
+                column16_linear<S, FORM>(H, prev, up, pa, pb, g2, mx);
+                prev = up;
+                out[j] = H[S - 1];
             }
-            if (has_down && (((x4 + 4) % kChainPublish) == 0 || x4 + 4 >= xm4)) chain_publish(prog_out, x4 + 4);
+            if (BND && has_down) {
+                __stcg(row_out + (x4 / 4) * kWarp, make_uint4(out[0], out[1], out[2], out[3]));
+                if (prog_out && (((x4 + 4) % kChainPublish) == 0 || x4 + 4 >= xm4)) chain_publish(prog_out, x4 + 4);
+            }
         }
     } else {
-        uint32_t Zl[S], Bl[S];  // as in sweep16
+        // left of and above the matrix: M = 0, X and Y = -inf.
+        // Zl[r] = max(X + ext, M + gap + ext) of the previous column: exactly
+        // this column's X, one row array instead of two
+        uint32_t Zl[S], Bl[S];
 #pragma unroll
         for (int r = 0; r < S; ++r) {
             Zl[r] = ge2;
             Bl[r] = 0;
         }
-        uint32_t bb_prev = 0;
-        uint32_t cw_next = xm4 > 0 ? code_word(0) : pad4;
-        uint32_t cw2_next = DL && xm4 > 0 ? code_word2(0) : pad4;
-        // this lane's entries of the ring row above: slot k % kPre holds column k
         uint4* my = pre + (threadIdx.x & 31);
-        if (has_up) {
-#pragma unroll
-            for (int k = 0; k < kPre - 1; ++k) {
-                if (k < xm4) cp_async16(&my[k * kWarp], &ring_in[(int64_t)k * kWarp]);
-                cp_async_commit();
+        auto copy_block = [&](int blk) {  // block blk's entries into slot blk % kPreBlocks
+            if (4 * blk < xm4) {
+                uint4* d = my + (blk % kPreBlocks) * 2 * kWarp;
+                cp_async16(d, row_in + (2 * blk) * kWarp);
+                cp_async16(d + kWarp, row_in + (2 * blk + 1) * kWarp);
             }
+            cp_async_commit();
+        };
+        if (BND && has_up) {
+#pragma unroll
+            for (int k = 0; k < kPreBlocks - 1; ++k) copy_block(k);
         }
         for (int x4 = 0; x4 < xm4; x4 += 4) {
             if (!need_cols(min(x4 + kChainNeed, xm4))) {
@@ -465,51 +424,37 @@ __device__ __forceinline__ bool sweep16_chain(const uint8_t* qc, int lq4, const 
                 return false;
             }
             const uint32_t cw = cw_next, cw2 = cw2_next;
-            if (x4 + 4 < xm4) {
-                cw_next = code_word(x4 + 4);
-                if constexpr (DL) cw2_next = code_word2(x4 + 4);
+            cw_next = code_word(x4 + 4);
+            if constexpr (DL) cw2_next = code_word2(x4 + 4);
+            uint4 in0 = make_uint4(kNeg16x2, 0u, kNeg16x2, 0u), in1 = in0;
+            if (BND && has_up) {
+                copy_block(x4 / 4 + kPreBlocks - 1);  // its slot held the block before this one
+                cp_async_wait<kPreBlocks - 1>();      // this block's copies have landed
+                const uint4* d = my + ((x4 / 4) % kPreBlocks) * 2 * kWarp;
+                in0 = d[0];
+                in1 = d[kWarp];
             }
+            uint4 out0, out1;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const int x = x4 + j;
-                const int a = (cw >> (8 * j)) & 0xff;
-                const int a2 = DL ? (cw2 >> (8 * j)) & 0xff : 0;
-                uint4 v = make_uint4(ge2, kNeg16x2, 0u, 0u);
-                if (has_up) {
-                    const int xn = x + kPre - 1;  // its slot held column x - 1, already read
-                    if (xn < xm4) cp_async16(&my[(xn % kPre) * kWarp], &ring_in[(int64_t)xn * kWarp]);
-                    cp_async_commit();
-                    cp_async_wait<kPre - 1>();  // column x's copy has landed
-                    v = my[(x % kPre) * kWarp];
-                }
-                uint32_t mgup = v.x, yup = v.y, bup = v.z;
-                uint32_t bdiag = bb_prev;
-                bb_prev = bup;
-#pragma unroll
-                for (int g = 0; g < S / 4; ++g) {
-                    uint32_t sc[4];
-                    fetch16<DL>(prof, g * alpha1 + a, g * alpha1 + a2, sc);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int r = 4 * g + k;
-                        const uint32_t mg = __viaddmax_s16x2(bdiag, sc[k], ge2);
-                        const uint32_t y = __viaddmax_s16x2(yup, e2, mgup);
-                        const uint32_t xg = Zl[r];
-                        const uint32_t bst = __vimax3_s16x2(__viaddmax_s16x2(mg, nge2, kNeg16x2), y, xg);
-                        Zl[r] = __viaddmax_s16x2(xg, e2, mg);
-                        bdiag = Bl[r];
-                        Bl[r] = bst;
-                        mgup = mg;
-                        yup = y;
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < S; r += 2) mx = __vimax3_s16x2(mx, Bl[r], Bl[r + 1]);
-                if (has_down) __stcg(&ring_out[(int64_t)x * kWarp], make_uint4(mgup, yup, Bl[S - 1], 0u));
+                const void* pa = prof + ((cw >> (8 * j)) & 0xff) * kResidue;
+                const void* pb = DL ? prof + ((cw2 >> (8 * j)) & 0xff) * kResidue : pa;
+                uint32_t y = j == 0 ? in0.x : j == 1 ? in0.z : j == 2 ? in1.x : in1.z;
+                column16_affine<S, FORM>(Zl, Bl, prev, y, pa, pb, e2, ge2, mx);
+                prev = j == 0 ? in0.y : j == 1 ? in0.w : j == 2 ? in1.y : in1.w;
+                if (j == 0) out0.x = y, out0.y = Bl[S - 1];
+                if (j == 1) out0.z = y, out0.w = Bl[S - 1];
+                if (j == 2) out1.x = y, out1.y = Bl[S - 1];
+                if (j == 3) out1.z = y, out1.w = Bl[S - 1];
             }
-            if (has_down && (((x4 + 4) % kChainPublish) == 0 || x4 + 4 >= xm4)) chain_publish(prog_out, x4 + 4);
+            if (BND && has_down) {
+                uint4* d = row_out + (x4 / 2) * kWarp;
+                __stcg(d, out0);
+                __stcg(d + kWarp, out1);
+                if (prog_out && (((x4 + 4) % kChainPublish) == 0 || x4 + 4 >= xm4)) chain_publish(prog_out, x4 + 4);
+            }
         }
-        cp_async_wait<0>();
+        if constexpr (BND) cp_async_wait<0>();
     }
     return true;
 }
@@ -575,75 +520,97 @@ __device__ __forceinline__ void store_max16(const Score16Args& A, const WorkItem
     if (ma >= kOvf16 || (s_hi >= 0 && mb >= kOvf16)) atomicAdd(A.ovf_count, 1);
 }
 
-template <int S, bool DL>
-__device__ __forceinline__ void build_item_profile(void* prof, const Score16Args& A, const uint8_t* ra,
-                                                   const uint8_t* rb, int y0, int la, int lb, int shift, int lane) {
-    if constexpr (DL)
-        build_profile16_dual<S>((uint2*)prof, A.cmat, ra, y0, la, A.alpha1, A.dim, shift, lane);
-    else
-        build_profile16<S>((uint4*)prof, A.cmat, ra, rb, y0, la, lb, A.alpha1, A.dim, shift, lane);
+// A block's shared memory: its four warps' profiles, then (affine, with
+// boundary rows) their prefetch rings.
+template <int S, bool AFFINE, int FORM, bool BND>
+__host__ __device__ constexpr int score16_smem(int alpha1) {
+    return block_profile_bytes<S, FORM>(alpha1) + (AFFINE && BND ? 4 * kPreBytes : 0);
 }
 
-template <int S, bool AFFINE, bool DL>
-__global__ void __launch_bounds__(128, 3) score16_chain_kernel(Score16Args A) {
+// Every strip of an item on this warp, its boundary rows in the warp's slot of
+// bnd_pool.
+template <int S, bool AFFINE, int FORM, bool MULTI>
+__device__ __forceinline__ uint32_t whole_item16(const Score16Args& A, const WorkItem& W, const Lanes16& L,
+                                                 unsigned char* prof, uint4* pre, uint4* bnd, int lane) {
+    const int sa = W.target, sb = FORM == kDual ? -1 : W.index;
+    const int la = A.strip_len[sa];
+    const int lb = sb >= 0 ? A.strip_len[sb] : 0;
+    const uint8_t* ra = A.strip_res + A.strip_off[sa];
+    const uint8_t* rb = A.strip_res + A.strip_off[sb >= 0 ? sb : sa];
+    const int nstrips = MULTI ? (max(la, lb) + S - 1) / S : 1;
+    const int xm4 = (W.xmax + 3) & ~3;
+    const int64_t row = ring_row<AFFINE>(xm4);
+    const uint32_t pad4 = (uint32_t)A.pad_code * 0x01010101u;
+    uint32_t mx = 0;
+    for (int st = 0; st < nstrips; ++st) {
+        if (MULTI && st > 0) fence_acq_rel_gpu();  // the row above is stored before it is copied back
+        __syncwarp();
+        build_profile16<S, FORM>(prof, A.cmat, ra, rb, st * S, la, lb, A.alpha1, A.dim, lane);
+        __syncwarp();
+        const uint4* row_in = MULTI ? bnd + ((st + 1) & 1) * row : nullptr;
+        uint4* row_out = MULTI ? bnd + (st & 1) * row : nullptr;
+        sweep16<S, AFFINE, FORM, MULTI>(L.qc, L.lq4, L.qc2, L.lq42, xm4, pad4, prof, A.gap, A.ext, st > 0,
+                                        st + 1 < nstrips, row_in, row_out, nullptr, nullptr, nullptr, 0ull, pre, mx);
+    }
+    return mx;
+}
+
+template <int S, bool AFFINE, int FORM>
+__global__ void __launch_bounds__(128, AFFINE ? 3 : 4) score16_chain_kernel(Score16Args A) {
+    constexpr bool DL = FORM == kDual;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    void* prof = warp_profile<S, DL>(smem, wib, A.alpha1);
-    // after the four warps' profiles: each warp's prefetch ring (affine)
-    uint4* pre = (uint4*)(smem + chain_profile_bytes<S, DL>(A.alpha1)) + wib * kPre * kWarp;
-    const int shift = AFFINE ? A.ge : 0;
+    unsigned char* prof = smem + wib * warp_profile_bytes<S, FORM>(A.alpha1);
+    uint4* pre = (uint4*)(smem + block_profile_bytes<S, FORM>(A.alpha1) + wib * kPreBytes);
     const uint32_t pad4 = (uint32_t)A.pad_code * 0x01010101u;
     const int64_t warp_global = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
-    uint4* bnd = A.bnd_pool + warp_global * A.bnd_slot + lane;
     for (;;) {
         int it = 0;
         if (lane == 0) it = A.item_base + atomicAdd(A.counter, 1);
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= A.n_items) break;
-        const WorkItem W = A.items[it];
         const int4 ci = A.chain[it];
-        const int c = ci.x, s = ci.y, pred = ci.z;
+        const WorkItem W = A.items[ci.w];
+        const int c = ci.x, pred = ci.z;
+        const bool whole = ci.y < 0;
         const int sa = W.target, sb = DL ? -1 : W.index;
         const int la = A.strip_len[sa];
         const int lb = sb >= 0 ? A.strip_len[sb] : 0;
-        const int ls = la > lb ? la : lb;
-        const int nstrips = (ls + S - 1) / S;
+        const int nstrips = (max(la, lb) + S - 1) / S;
         const Lanes16 L = item_lanes<DL>(A, W, lane);
         const uint8_t* ra = A.strip_res + A.strip_off[sa];
         const uint8_t* rb = A.strip_res + A.strip_off[sb >= 0 ? sb : sa];
+        const int xm4 = (W.xmax + 3) & ~3;
+        const int64_t row = ring_row<AFFINE>(xm4);
+        uint4* rows = (whole ? A.bnd_pool + warp_global * A.bnd_slot : A.ring + A.ring_off[c]) + lane;
+        // a chain entry is one strip; a whole item runs its strips one after
+        // another here, without progress flags
         uint32_t mx = 0;
-        bool finished = true;
-        if (s < 0) {
-            // a whole item on this warp, strip after strip
-            for (int st = 0; st < nstrips; ++st) {
-                __syncwarp();
-                build_item_profile<S, DL>(prof, A, ra, rb, st * S, la, lb, shift, lane);
-                __syncwarp();
-                if (L.active)
-                    sweep16<S, AFFINE, DL>(L.qc, L.lq4, L.qc2, L.lq42, pad4, prof, A.alpha1, A.gap, A.ext, A.ge,
-                                           st > 0, st + 1 < nstrips, bnd, mx);
-            }
-        } else {
-            const int xm4 = (W.xmax + 3) & ~3;
-            const int64_t row = (int64_t)xm4 * kWarp;
-            const uint4* ring_in = A.ring + A.ring_off[c] + ((s + 1) & 1) * row + lane;
-            uint4* ring_out = A.ring + A.ring_off[c] + (s & 1) * row + lane;
+        bool ok = true;
+        int s = whole ? 0 : ci.y;
+        const int s_end = whole ? nstrips : s + 1;
+        for (; s < s_end && ok; ++s) {
+            if (whole && s > 0) fence_acq_rel_gpu();  // the row above is stored before it is copied back
             __syncwarp();
-            build_item_profile<S, DL>(prof, A, ra, rb, s * S, la, lb, shift, lane);
+            build_profile16<S, FORM>(prof, A.cmat, ra, rb, s * S, la, lb, A.alpha1, A.dim, lane);
             __syncwarp();
             const bool has_down = s + 1 < nstrips;
-            if (!sweep16_chain<S, AFFINE, DL>(L.qc, L.lq4, L.qc2, L.lq42, xm4, pad4, prof, A.alpha1, A.gap, A.ext,
-                                              A.ge, s > 0, has_down, ring_in, ring_out,
-                                              s > 0 ? A.progress + pred : nullptr, A.progress + it, A.abort_flag,
-                                              A.wait_ns, pre, mx))
-                break;
-            if (s > 0) {
+            ok = sweep16<S, AFFINE, FORM, true>(L.qc, L.lq4, L.qc2, L.lq42, xm4, pad4, prof, A.gap, A.ext, s > 0,
+                                                has_down, rows + ((s + 1) & 1) * row, rows + (s & 1) * row,
+                                                !whole && s > 0 ? A.progress + pred : nullptr,
+                                                !whole && has_down ? A.progress + it : nullptr, A.abort_flag,
+                                                A.wait_ns, pre, mx);
+        }
+        if (!ok) break;
+        bool finished = true;
+        if (!whole) {
+            if (ci.y > 0) {
                 // the predecessor's running maximum is final once it has finished
                 if (chain_wait(A.progress + pred, kChainDone, A.abort_flag, A.wait_ns) < 0) break;
                 mx = __vmaxs2(mx, __ldcg(&A.run_max[(int64_t)pred * kWarp + lane]));
             }
-            if (has_down) {
+            if (ci.y + 1 < nstrips) {
                 __stcg(&A.run_max[(int64_t)it * kWarp + lane], mx);
                 chain_publish(A.progress + it, kChainDone);
                 finished = false;
@@ -653,40 +620,24 @@ __global__ void __launch_bounds__(128, 3) score16_chain_kernel(Score16Args A) {
     }
 }
 
-template <int S, bool AFFINE, bool MULTI, bool DL>
+template <int S, bool AFFINE, bool MULTI, int FORM>
 __global__ void __launch_bounds__(128) score16_kernel(Score16Args A) {
+    constexpr bool DL = FORM == kDual;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    void* prof = warp_profile<S, DL>(smem, wib, A.alpha1);
+    unsigned char* prof = smem + wib * warp_profile_bytes<S, FORM>(A.alpha1);
+    uint4* pre = (uint4*)(smem + block_profile_bytes<S, FORM>(A.alpha1) + wib * kPreBytes);
     const int64_t warp_global = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
     uint4* bnd = MULTI ? A.bnd_pool + warp_global * A.bnd_slot + lane : nullptr;
-    const int shift = AFFINE ? A.ge : 0;
-    const uint32_t pad4 = (uint32_t)A.pad_code * 0x01010101u;
     for (;;) {
         int it = 0;
         if (lane == 0) it = atomicAdd(A.counter, 1);
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= A.n_items) break;
         const WorkItem W = A.grid_strips ? grid_item<S, DL>(A, it) : A.items[it];
-        const int sa = W.target, sb = DL ? -1 : W.index;
-        const int la = A.strip_len[sa];
-        const int lb = sb >= 0 ? A.strip_len[sb] : 0;
         const Lanes16 L = item_lanes<DL>(A, W, lane);
-        const uint8_t* ra = A.strip_res + A.strip_off[sa];
-        const uint8_t* rb = A.strip_res + A.strip_off[sb >= 0 ? sb : sa];
-        const int ls = la > lb ? la : lb;
-        const int nstrips = MULTI ? (ls + S - 1) / S : 1;
-        uint32_t mx = 0;
-        for (int s = 0; s < nstrips; ++s) {
-            const int y0 = s * S;
-            __syncwarp();
-            build_item_profile<S, DL>(prof, A, ra, rb, y0, la, lb, shift, lane);
-            __syncwarp();
-            if (L.active)
-                sweep16<S, AFFINE, DL>(L.qc, L.lq4, L.qc2, L.lq42, pad4, prof, A.alpha1, A.gap, A.ext, A.ge, s > 0,
-                                       s + 1 < nstrips, bnd, mx);
-        }
+        const uint32_t mx = whole_item16<S, AFFINE, FORM, MULTI>(A, W, L, prof, MULTI ? pre : nullptr, bnd, lane);
         if (L.active) store_max16<DL>(A, W, L, mx);
     }
 }
