@@ -23,7 +23,16 @@ struct ChainPlan {
 // Items (already ordered longest first) have nstr[k] strips of xm4[k]
 // columns.  Items whose cost nstr * xm4 reaches permille/1000 of the mean
 // per-warp load become chains of one-strip entries; the rest stay whole.
-// The queue comes from a list-scheduling simulation of `warps` equally fast
+//
+// With at least half as many chains as warps the queue goes by levels, the
+// chains aligned at their ends: level l holds strip l - (max strips - strips)
+// of every chain that has one, longest chains first, and the whole items
+// follow.  A strip's predecessor was then handed out about a level earlier and
+// is well ahead, so no simulation is needed to keep the warps busy (92,000
+// entries: 0.3 ms against 3.4 ms; the sweep takes the same time).
+//
+// With fewer chains their pipelining decides: the queue comes from a
+// list-scheduling simulation of `warps` equally fast
 // warps, time counted in columns of one strip: a warp that frees up takes the
 // next strip of the chain that became ready first (its predecessor started at
 // least `lead` columns ago; ties go to the longer chain), else the next whole
@@ -54,6 +63,24 @@ inline void plan_chain_queue(const std::vector<int>& nstr, const std::vector<int
         n_sub += (size_t)nstr[chain_item[c]];
     }
     out.queue.reserve(n_sub);
+    if (nc > 0 && 2 * (int64_t)nc >= warps) {
+        std::vector<int32_t> by_len(nc);
+        for (int c = 0; c < nc; ++c) by_len[c] = c;
+        std::stable_sort(by_len.begin(), by_len.end(),
+                         [&](int32_t a, int32_t b) { return nstr[chain_item[a]] > nstr[chain_item[b]]; });
+        const int top = nstr[chain_item[by_len[0]]];
+        int active = 0;
+        for (int level = 0; level < top; ++level) {
+            while (active < nc && nstr[chain_item[by_len[active]]] >= top - level) ++active;
+            for (int k = 0; k < active; ++k) {
+                const int c = by_len[k];
+                out.queue.push_back(PlanEntry{chain_item[c], c, next[c]++, last_q[c]});
+                last_q[c] = (int32_t)out.queue.size() - 1;
+            }
+        }
+        for (int32_t k : whole) out.queue.push_back(PlanEntry{k, -1, -1, -1});
+        return;
+    }
     // min-heaps on int64 keys: warps by free time; ready chains by
     // (ready time << 24 | chain), chain < 2^24
     std::vector<int64_t> freew((size_t)warps, 0);
