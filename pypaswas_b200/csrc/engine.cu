@@ -33,8 +33,8 @@
 #include "pw_kernels.cuh"
 #include "score16_variants.h"
 #include "pw_band.cuh"
+#include "pw_band_ck.cuh"
 #include "pw_tiles.cuh"
-#include "pw_band16.cuh"
 #include "pw_plan.h"
 #include "pw_finish.cuh"
 #include "pw_host.h"
@@ -242,13 +242,17 @@ struct pw_engine {
     DevBuf band_pairs, band_entries, band_prog, band_max, band_ring, band_out;  // band sweep (pw_band.cuh)
     DevBuf tile_ck, tile_marks, tile_pairs, slot_tile;                        // tile form (pw_tiles.cuh)
     DevBuf tile_pairs_alt, tile_sel, tile_cnt, tile_acc, tile_scratch, tile_ops;
-    DevBuf band_over;                                                         // band16_kernel: pairs past 16 bits
-    // explicit pairs: the score sweep's tile-form checkpoints (band_kernel<false, 4>)
+    DevBuf band_over;                                                         // band_ck_kernel: pairs past 16 bits
+    // explicit pairs: the score sweep's tile-form checkpoints (band_ck_kernel)
     DevBuf p1_ck;
     bool p1_tiles = false;
     int64_t p1_free = 0;
     double p1_free_t = -1.0;
-    std::vector<int64_t> p1_ck_off, p1_tm_off;           // per listed pair
+    struct P1Ck {                                        // per listed pair: its checkpoints (TilePair)
+        int64_t rows = 0, cols = 0, tm = 0;
+        int fmt = 0;
+    };
+    std::vector<P1Ck> p1_pairs;
     std::unordered_map<int64_t, int32_t> p1_index;        // query * nt + target -> listed pair
     DevBuf scan_tmp;  // CUB scan / select scratch
     DevBuf prune_flags, prune_cnt, prune_sel, t_skip, q_count;  // phase-2 pruning on the device
@@ -1565,7 +1569,8 @@ static cudaError_t finish_hits(pw_engine* e, int64_t n, int64_t* str_bytes) {
 
 // Queue entries (pair, band, queue index of the band above) of band chains:
 // pair k has nbands[k] bands of steps[k] steps, pairs in priority order.
-static std::vector<int4> band_queue(const std::vector<int>& nbands, const std::vector<int64_t>& steps, int warps) {
+static std::vector<int4> band_queue(const std::vector<int>& nbands, const std::vector<int64_t>& steps, int warps,
+                                    int lead) {
     std::vector<int4> entries;
     if ((int64_t)nbands.size() * 2 >= warps) {
         // many pairs: band-major order (every band 0, then every band 1, ...,
@@ -1583,7 +1588,7 @@ static std::vector<int4> band_queue(const std::vector<int>& nbands, const std::v
     } else {
         // few (long) pairs: a list-scheduling plan pipelines each pair's bands
         ChainPlan plan;
-        plan_chain_queue(nbands, steps, warps, 1, kBandLead, plan);
+        plan_chain_queue(nbands, steps, warps, 1, lead, plan);
         entries.resize(plan.queue.size());
         for (size_t k = 0; k < plan.queue.size(); ++k) {
             const PlanEntry& p = plan.queue[k];
@@ -1597,7 +1602,7 @@ static std::vector<int4> band_queue(const std::vector<int>& nbands, const std::v
 // chained across warps, pw_band.cuh).  DIRS 1: the direction sweep of traced
 // pairs (cell codes), 2: the same storing H (linear gap), 3: the checkpoint
 // sweep of the tile form (linear gap, checkpoints into tile_ck); 0: pair
-// maxima into band_max (indexed by BandPair.slot).
+// maxima into band_out (indexed by BandPair.slot).
 template <int DIRS>
 static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pairs, double* kernel_ms,
                           int* n_launch) {
@@ -1635,12 +1640,12 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
         sorted[k] = pairs[order[k]];
         nstr[k] = sorted[k].nbands;
         xm[k] = steps[order[k]];
-        if constexpr (DIRS < 3) {  // DIRS 4 keeps its tile-maxima offset there
+        if constexpr (DIRS < 3) {
             sorted[k].ring_off = ring_elems;
             if (sorted[k].nbands > 1) ring_elems += 2 * (int64_t)e->pr.qlen[sorted[k].q];
         }
     }
-    std::vector<int4> entries = band_queue(nstr, xm, warps);
+    std::vector<int4> entries = band_queue(nstr, xm, warps, kBandLead);
     const size_t n = entries.size();
     if (e->tune[PW_TUNE_STALL_TEST]) {
         // one band below another waits on the spare flag (index n) instead
@@ -1673,7 +1678,7 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
     B.run_max = e->band_max.as<int>();
     B.abort_flag = e->chain_abort.as<int>();
     B.max_out = e->band_out.as<float>();
-    B.ck = DIRS == 3 ? e->tile_ck.as<int>() : DIRS == 4 ? e->p1_ck.as<int>() : nullptr;
+    B.ck = DIRS == 3 ? e->tile_ck.as<int>() : nullptr;
     B.wait_ns = wait_limit(e);
     const int grid = std::max(1, std::min(grid_cap(e, per_sm), (int)((n + 3) / 4)));
     cudaEvent_t a, b;
@@ -1698,30 +1703,34 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
     return PW_OK;
 }
 
-// Launches band16_kernel over `pairs` (two explicit pairs a chain, 16x2;
-// pw_band16.cuh): maxima into band_out by pair-list index, the pairs past the
-// 16-bit limit flagged in band_over, checkpoints and tile maxima into p1_ck.
-static int run_band16_phase(pw_engine* e, KernelArgs A, const std::vector<BandPair2>& pairs, int limit,
-                            double* kernel_ms, int* n_launch) {
+// Launches band_ck_kernel over `pairs` (listed pairs, PAIR: two a chain in
+// 16-bit halves): maxima into band_out by pair-list index, the pairs past the
+// 16-bit limit flagged in band_over, checkpoints and tile maxima into p1_ck
+// (whose rows are zero before).
+template <bool PAIR>
+static int run_band_ck_phase(pw_engine* e, KernelArgs A, const std::vector<BandCk>& pairs, int limit,
+                             double* kernel_ms, int* n_launch) {
     if (pairs.empty()) return PW_OK;
-    const int smem = 4 * kWarp * (A.P.alpha + 1) * kWarpRows * 4;
+    auto kern = band_ck_kernel<PAIR>;
+    const int smem = 4 * band_ck_warp_smem(A.P.alpha + 1);
     cudaError_t c;
     if (smem > 48 * 1024 &&
-        (c = cudaFuncSetAttribute(band16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
+        (c = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
         return cuda_fail(e, c, "band sweep smem");
     int per_sm = 0;
-    if ((c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, band16_kernel, 128, smem)) != cudaSuccess)
+    if ((c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem)) != cudaSuccess)
         return cuda_fail(e, c, "occupancy");
     per_sm = std::max(1, std::min(per_sm, 16));
     const int warps = grid_cap(e, per_sm) * 4;
     std::vector<int> order(pairs.size());
     std::iota(order.begin(), order.end(), 0);
     std::vector<int64_t> steps(pairs.size());
-    for (size_t k = 0; k < pairs.size(); ++k) steps[k] = (int64_t)e->pr.qlen[pairs[k].q] + kWarp - 1;
+    for (size_t k = 0; k < pairs.size(); ++k)
+        steps[k] = ((int64_t)e->pr.qlen[pairs[k].q] + kBlkCols - 1) / kBlkCols + kWarp - 1;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
         return steps[x] * pairs[x].nbands > steps[y] * pairs[y].nbands;
     });
-    std::vector<BandPair2> sorted(pairs.size());
+    std::vector<BandCk> sorted(pairs.size());
     std::vector<int> nstr(pairs.size());
     std::vector<int64_t> xm(pairs.size());
     for (size_t k = 0; k < order.size(); ++k) {
@@ -1729,8 +1738,17 @@ static int run_band16_phase(pw_engine* e, KernelArgs A, const std::vector<BandPa
         nstr[k] = std::max(1, sorted[k].nbands);
         xm[k] = steps[order[k]];
     }
-    const std::vector<int4> entries = band_queue(nstr, xm, warps);
+    std::vector<int4> entries = band_queue(nstr, xm, warps, kBandCkLead);
     const size_t n = entries.size();
+    if (e->tune[PW_TUNE_STALL_TEST]) {
+        // one band below another waits on the spare flag (index n) instead
+        for (int4& v : entries)
+            if (v.y > 0) {
+                e->tune[PW_TUNE_STALL_TEST] = 0;
+                v.z = (int)n;
+                break;
+            }
+    }
     if ((c = upload(e, e->band_pairs, sorted)) != cudaSuccess) return cuda_fail(e, c, "upload band pairs");
     if ((c = upload(e, e->band_entries, entries)) != cudaSuccess) return cuda_fail(e, c, "upload band queue");
     if ((c = e->band_prog.reserve(e->stream, (n + 1) * sizeof(int))) != cudaSuccess ||
@@ -1741,10 +1759,10 @@ static int run_band16_phase(pw_engine* e, KernelArgs A, const std::vector<BandPa
         (c = cudaMemsetAsync(e->chain_abort.p, 0, sizeof(int), e->stream)) != cudaSuccess ||
         (c = cudaMemsetAsync(e->counter.as<int>() + kNumClasses, 0, sizeof(int), e->stream)) != cudaSuccess)
         return cuda_fail(e, c, "reset band state");
-    BandArgs2 B;
+    BandCkArgs B;
     memset(&B, 0, sizeof(B));
     B.entries = e->band_entries.as<int4>();
-    B.pairs = e->band_pairs.as<BandPair2>();
+    B.pairs = e->band_pairs.as<BandCk>();
     B.n_entries = (int)n;
     B.counter = e->counter.as<int>() + kNumClasses;
     B.progress = e->band_prog.as<int>();
@@ -1760,7 +1778,7 @@ static int run_band16_phase(pw_engine* e, KernelArgs A, const std::vector<BandPa
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     cudaEventRecord(a, e->stream);
-    PW_LAUNCH(band16_kernel, grid, 128, smem, e->stream, A, B);
+    PW_LAUNCH(kern, grid, 128, smem, e->stream, A, B);
     e->launches++;
     cudaEventRecord(b, e->stream);
     if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "band sweep launch");
@@ -1779,7 +1797,7 @@ static int run_band16_phase(pw_engine* e, KernelArgs A, const std::vector<BandPa
 }
 
 // Candidates of tile-form pairs whose checkpoints the score sweep kept
-// (band_kernel<false, 4>): the pairs' records and the tiles that reach their
+// (band_ck_kernel): the pairs' records and the tiles that reach their
 // thresholds (tile_select_kernel), those tiles recomputed with the
 // candidate test (tile_cand_kernel), the counts into the records.
 static int run_tile_cands(pw_engine* e, KernelArgs A, TileArgs T, const TilePair* dev_list,
@@ -1940,56 +1958,26 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         if ((c = e->band_out.reserve(e->stream, np * sizeof(float))) != cudaSuccess)
             return cuda_fail(e, c, "alloc band maxima");
         // linear integer scoring: the sweep also keeps the tile form's
-        // checkpoints and tile maxima (band_kernel<false, 4>), so that the
-        // traced pairs need no second sweep -- when they take at most 35% of
-        // the free device memory
+        // checkpoints and tile maxima (band_ck_kernel), so that the traced
+        // pairs need no second sweep -- when they take at most 35% of the free
+        // device memory
         bool p1ck = !e->affine && e->tune[PW_TUNE_TILE_TRACE] != 1;
+        std::vector<BandCk> bp2, bp1;  // two pairs a chain in 16-bit halves, one on 32-bit lanes
+        int64_t ck_ints = 0;           // used ints of p1_ck
+        auto ck_of = [&](size_t j) {   // a single pair on 32-bit lanes
+            BandCk p;
+            memset(&p, 0, sizeof(p));
+            p.q = bp[j].q;
+            p.t[0] = p.t[1] = bp[j].t;
+            p.nbands = bp[j].nbands;
+            p.slot[0] = p.slot[1] = (int64_t)j;
+            return p;
+        };
+        const int limit = 32767 - (int)std::ceil(A.P.highest);
         if (p1ck) {
-            e->p1_ck_off.assign(np, 0);
-            e->p1_tm_off.assign(np, 0);
-            int64_t ck = 0, tm = 0;
-            for (size_t k = 0; k < np; ++k) {
-                const int lq = qlen[bp[k].q], lt = tlen[bp[k].t];
-                e->p1_ck_off[k] = ck;
-                ck += tile_checkpoint_ints(lq, lt);
-                e->p1_tm_off[k] = tm;
-                tm += (int64_t)bp[k].nbands * tile_count(lq);
-            }
-            // the driver's free-memory query can be held for tens of
-            // milliseconds by tools polling the GPU: read at most every 10 s
-            const double now = wall_ms();
-            if (e->p1_free_t < 0 || now - e->p1_free_t > 10000.0) {
-                size_t free_b = 0, total_b = 0;
-                cudaMemGetInfo(&free_b, &total_b);
-                e->p1_free = (int64_t)free_b + (int64_t)e->p1_ck.bytes;
-                e->p1_free_t = now;
-            }
-            const int64_t bytes = (ck + tm) * (int64_t)sizeof(int);
-            p1ck = (double)bytes <= 0.35 * (double)e->p1_free;
-            if (p1ck && e->p1_ck.reserve(e->stream, (size_t)bytes) != cudaSuccess) {
-                cudaGetLastError();  // no room after all: the traced pairs get the checkpoint sweep
-                p1ck = false;
-            }
-            if (p1ck) {
-                if ((c = cudaMemsetAsync(e->p1_ck.as<int>() + ck, 0, (size_t)tm * sizeof(int), e->stream)) != cudaSuccess)
-                    return cuda_fail(e, c, "reset tile maxima");
-                e->p1_index.clear();
-                for (size_t k = 0; k < np; ++k) {
-                    e->p1_tm_off[k] += ck;
-                    bp[k].dir_base = e->p1_ck_off[k];
-                    bp[k].ring_off = e->p1_tm_off[k];
-                    e->p1_index.emplace((int64_t)bp[k].q * nt + bp[k].t, (int32_t)k);
-                }
-            }
-        }
-        cudaEventRecord(e->ev[0], e->stream);
-        if (p1ck) {
-            // pairs that share their query and their target's length go two to
-            // a 16x2 sweep (pw_band16.cuh); the others, and pairs whose maximum
-            // passes the 16-bit limit, run on 32-bit lanes
-            const int limit = 32767 - (int)std::ceil(A.P.highest);
-            std::vector<BandPair2> bp2;
-            std::vector<BandPair> bp1;
+            // pairs that share their query and their target's length go two
+            // to a 16x2 sweep and share their checkpoint words; the others,
+            // and pairs whose maximum passes the 16-bit limit, run on 32-bit lanes
             if (!(flags & PW_FLAG_INT32) && limit > 0) {
                 std::map<std::pair<int32_t, int32_t>, size_t> open;
                 std::vector<char> paired(np, 0);
@@ -2002,47 +1990,115 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
                     }
                     const size_t j = f->second;
                     open.erase(f);
-                    BandPair2 p2;
-                    memset(&p2, 0, sizeof(p2));
-                    p2.q = bp[j].q;
-                    p2.t[0] = bp[j].t;
+                    BandCk p2 = ck_of(j);
                     p2.t[1] = bp[k].t;
-                    p2.nbands = bp[j].nbands;
-                    p2.slot[0] = (int64_t)j;
                     p2.slot[1] = (int64_t)k;
-                    p2.ck[0] = bp[j].dir_base;
-                    p2.ck[1] = bp[k].dir_base;
-                    p2.tm[0] = bp[j].ring_off;
-                    p2.tm[1] = bp[k].ring_off;
                     bp2.push_back(p2);
                     paired[j] = paired[k] = 1;
                     inf.paired_cells += 2 * (int64_t)qlen[bp[j].q] * tlen[bp[j].t];
                 }
                 for (size_t k = 0; k < np; ++k)
-                    if (!paired[k]) bp1.push_back(bp[k]);
+                    if (!paired[k]) bp1.push_back(ck_of(k));
             } else {
-                bp1 = bp;
+                for (size_t k = 0; k < np; ++k) bp1.push_back(ck_of(k));
             }
+            // the rows (zeroed before the sweep), the columns, the tile maxima
+            int64_t rows = 0, cols = 0, tm = 0;
+            for (auto* v : {&bp2, &bp1})
+                for (BandCk& p : *v) {
+                    const int lq = qlen[p.q], lt = tlen[p.t[0]];
+                    p.rows = rows;
+                    rows += tile_row_ints(lq, lt);
+                    p.cols = cols;
+                    cols += tile_col_ints(lq, lt);
+                    for (int h = 0; h < (v == &bp2 ? 2 : 1); ++h) {
+                        p.tm[h] = tm;
+                        tm += (int64_t)p.nbands * tile_count(lq);
+                    }
+                }
+            ck_ints = align_up(rows + cols + tm, 4);
+            // the driver's free-memory query can be held for tens of
+            // milliseconds by tools polling the GPU: read at most every 10 s
+            const double now = wall_ms();
+            if (e->p1_free_t < 0 || now - e->p1_free_t > 10000.0) {
+                size_t free_b = 0, total_b = 0;
+                cudaMemGetInfo(&free_b, &total_b);
+                e->p1_free = (int64_t)free_b + (int64_t)e->p1_ck.bytes;
+                e->p1_free_t = now;
+            }
+            const int64_t bytes = ck_ints * (int64_t)sizeof(int);
+            p1ck = (double)bytes <= 0.35 * (double)e->p1_free;
+            if (p1ck && e->p1_ck.reserve(e->stream, (size_t)std::max<int64_t>(bytes, 16)) != cudaSuccess) {
+                cudaGetLastError();  // no room after all: the traced pairs get the checkpoint sweep
+                p1ck = false;
+            }
+            if (p1ck) {
+                int* base = e->p1_ck.as<int>();
+                if ((c = cudaMemsetAsync(base, 0, (size_t)rows * sizeof(int), e->stream)) != cudaSuccess ||
+                    (c = cudaMemsetAsync(base + rows + cols, 0, (size_t)tm * sizeof(int), e->stream)) != cudaSuccess)
+                    return cuda_fail(e, c, "reset checkpoints");
+                e->p1_pairs.assign(np, pw_engine::P1Ck());
+                for (auto* v : {&bp2, &bp1})
+                    for (BandCk& p : *v) {
+                        p.cols += rows;
+                        p.tm[0] += rows + cols;
+                        p.tm[1] += rows + cols;
+                        for (int h = 0; h < (v == &bp2 ? 2 : 1); ++h) {
+                            pw_engine::P1Ck& o = e->p1_pairs[(size_t)p.slot[h]];
+                            o.rows = p.rows;
+                            o.cols = p.cols;
+                            o.tm = p.tm[h];
+                            o.fmt = v == &bp2 ? 1 + h : 0;
+                        }
+                    }
+                e->p1_index.clear();
+                for (size_t k = 0; k < np; ++k) e->p1_index.emplace((int64_t)bp[k].q * nt + bp[k].t, (int32_t)k);
+            } else {
+                inf.paired_cells = 0;
+            }
+        }
+        cudaEventRecord(e->ev[0], e->stream);
+        if (p1ck) {
             if (!bp2.empty()) {
                 if ((c = e->band_over.reserve(e->stream, np * sizeof(int))) != cudaSuccess ||
                     (c = cudaMemsetAsync(e->band_over.p, 0, np * sizeof(int), e->stream)) != cudaSuccess)
                     return cuda_fail(e, c, "alloc band flags");
-                rc = run_band16_phase(e, A, bp2, limit, &inf.score_kernel_ms, &inf.score_launches);
+                rc = run_band_ck_phase<true>(e, A, bp2, limit, &inf.score_kernel_ms, &inf.score_launches);
                 if (rc != PW_OK) return rc;
                 std::vector<int32_t> over;
                 if ((c = download(e, over, e->band_over.p, np)) != cudaSuccess) return cuda_fail(e, c, "copy band flags");
+                // pairs past the limit: 32-bit lanes, their checkpoints behind the others
+                std::vector<BandCk> again;
+                int64_t end = ck_ints;
                 for (size_t k = 0; k < np; ++k) {
                     if (!over[k]) continue;
-                    const int lq = qlen[bp[k].q];
-                    if ((c = cudaMemsetAsync(e->p1_ck.as<int>() + bp[k].ring_off, 0,
-                                             (size_t)bp[k].nbands * tile_count(lq) * sizeof(int), e->stream)) != cudaSuccess)
-                        return cuda_fail(e, c, "reset tile maxima");
-                    bp1.push_back(bp[k]);
+                    BandCk p = ck_of(k);
+                    const int lq = qlen[p.q], lt = tlen[p.t[0]];
+                    p.rows = end;
+                    p.cols = p.rows + tile_row_ints(lq, lt);
+                    p.tm[0] = p.tm[1] = p.cols + tile_col_ints(lq, lt);
+                    end = align_up(p.tm[0] + (int64_t)p.nbands * tile_count(lq), 4);
+                    again.push_back(p);
                     inf.overflow_pairs++;
-                    inf.paired_cells -= (int64_t)qlen[bp[k].q] * tlen[bp[k].t];
+                    inf.paired_cells -= (int64_t)lq * lt;
+                }
+                if (!again.empty()) {
+                    if ((c = e->p1_ck.grow_keep(e->stream, (size_t)ck_ints * sizeof(int), (size_t)end * sizeof(int))) !=
+                            cudaSuccess ||
+                        (c = cudaMemsetAsync(e->p1_ck.as<int>() + ck_ints, 0, (size_t)(end - ck_ints) * sizeof(int),
+                                             e->stream)) != cudaSuccess)
+                        return cuda_fail(e, c, "alloc checkpoints");
+                    for (BandCk& p : again) {
+                        pw_engine::P1Ck& o = e->p1_pairs[(size_t)p.slot[0]];
+                        o.rows = p.rows;
+                        o.cols = p.cols;
+                        o.tm = p.tm[0];
+                        o.fmt = 0;
+                        bp1.push_back(p);
+                    }
                 }
             }
-            rc = run_band_phase<4>(e, A, bp1, &inf.score_kernel_ms, &inf.score_launches);
+            rc = run_band_ck_phase<false>(e, A, bp1, limit, &inf.score_kernel_ms, &inf.score_launches);
         } else {
             rc = run_band_phase<0>(e, A, bp, &inf.score_kernel_ms, &inf.score_launches);
         }
@@ -2510,10 +2566,14 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
                 if (p1ck) {
                     const auto f = e->p1_index.find((int64_t)tp.q * nt + tp.t);
                     if (f == e->p1_index.end()) return fail(e, PW_ERR_STATE, "traced pair without checkpoints");
-                    tp.ck = e->p1_ck_off[f->second];
-                    tp.tm = e->p1_tm_off[f->second];
+                    const pw_engine::P1Ck& o = e->p1_pairs[(size_t)f->second];
+                    tp.rows = o.rows;
+                    tp.cols = o.cols;
+                    tp.tm = o.tm;
+                    tp.fmt = o.fmt;
                 } else {
-                    tp.ck = ck_ints;
+                    tp.rows = ck_ints;
+                    tp.cols = ck_ints + tile_row_ints(lq_, lt_);
                     wi[k].dir_base = ck_ints;  // band_kernel<false, 3>: the pair's checkpoints
                     ck_ints += tile_checkpoint_ints(lq_, lt_);
                 }

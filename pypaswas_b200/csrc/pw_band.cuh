@@ -34,10 +34,8 @@
 // bottom row is kept (in place of the two-row ring) and every lane stores its
 // 8 rows' H at the last column of each kTileW-column tile, from which any
 // 256 x kTileW tile's codes are recomputed later.
-// DIRS = 4 (linear gap): the score sweep of DIRS 0 that also keeps the tile
-// form's checkpoints (as DIRS 3) and each tile's maximum H, so that traced
-// pairs need no second sweep: only the tiles that reach a pair's threshold
-// are recomputed for its candidates (pw_tiles.cuh).
+// The score sweep of listed pairs (linear gap) keeps the tile form's
+// checkpoints and tile maxima itself, in a kernel of its own (pw_band_ck.cuh).
 #pragma once
 #include "pw_kernels.cuh"
 #include "pw_score16.cuh"
@@ -59,17 +57,21 @@ __host__ __device__ __forceinline__ int64_t warp_code_bytes(int lq, int lt, bool
     return hstore ? cells * 2 : cells / 2;
 }
 
-// Tile form: ints of a pair's checkpoints -- the bottom rows of its bands but
-// the last ((nbands - 1) x lq), then per band and tile the 256 H values of the
-// tile's last column (nbands x ntiles x 256; tile ntiles - 1's are not read).
+// Tile form: a pair's checkpoints are the bottom rows of its bands but the
+// last (tile_row_ints: (nbands - 1) rows of tile_row_stride) and, per band and
+// tile, the 256 H values of the tile's last column (tile_col_ints: nbands x
+// ntiles x 256; tile j's left boundary is at index j, index 0 is not used).
 __host__ __device__ __forceinline__ int tile_count(int lq) { return lq > 0 ? (lq + kTileW - 1) / kTileW : 1; }
-__host__ __device__ __forceinline__ int64_t tile_col_offset(int lq, int lt) {  // 4-int aligned
-    const int64_t bands = lt > 0 ? (lt + kBandRows - 1) / kBandRows : 1;
-    return ((bands - 1) * (int64_t)lq + 3) & ~(int64_t)3;
+__host__ __device__ __forceinline__ int64_t tile_bands(int lt) { return lt > 0 ? (lt + kBandRows - 1) / kBandRows : 1; }
+__host__ __device__ __forceinline__ int64_t tile_row_stride(int lq) { return ((int64_t)lq + 3) & ~(int64_t)3; }
+__host__ __device__ __forceinline__ int64_t tile_row_ints(int lq, int lt) {  // a multiple of 4
+    return (tile_bands(lt) - 1) * tile_row_stride(lq);
 }
-__host__ __device__ __forceinline__ int64_t tile_checkpoint_ints(int lq, int lt) {  // a multiple of 4
-    const int64_t bands = lt > 0 ? (lt + kBandRows - 1) / kBandRows : 1;
-    return tile_col_offset(lq, lt) + bands * tile_count(lq) * (int64_t)kBandRows;
+__host__ __device__ __forceinline__ int64_t tile_col_ints(int lq, int lt) {  // a multiple of 4
+    return tile_bands(lt) * tile_count(lq) * (int64_t)kBandRows;
+}
+__host__ __device__ __forceinline__ int64_t tile_checkpoint_ints(int lq, int lt) {
+    return tile_row_ints(lq, lt) + tile_col_ints(lq, lt);
 }
 
 struct BandPair {
@@ -78,6 +80,7 @@ struct BandPair {
     int32_t meta_item;   // DIRS: value for PairMeta.item (the pair's work item in the wave)
     int64_t ring_off;    // int4 offset of the pair's two boundary rows (2 x lq)
     int64_t dir_base;    // DIRS 1, 2: byte offset of the pair's cell codes; 3: int offset of its checkpoints
+                         // (rows, then columns)
     int64_t slot;        // DIRS: pair slot (metas, candidates); score sweep: pair_max index
 };
 
@@ -91,8 +94,7 @@ struct BandArgs {
     int* run_max;         // per entry: running maximum of the pair's bands so far
     int* abort_flag;
     float* max_out;       // score sweep: pair maxima, indexed by BandPair.slot
-    int* ck;              // DIRS 3, 4: checkpoints (tile_checkpoint_ints per pair, at BandPair.dir_base);
-                          // DIRS 4: tile maxima (bands x tiles per pair, at BandPair.ring_off)
+    int* ck;              // DIRS 3: checkpoints (tile_checkpoint_ints per pair, at BandPair.dir_base)
     unsigned long long wait_ns;  // bound of one wait for the band above
 };
 
@@ -125,8 +127,8 @@ __device__ __forceinline__ int prof_score(uint2 pw, int r) {
 template <bool AFFINE, int DIRS>
 __global__ void __launch_bounds__(128, AFFINE ? 5 : 8) band_kernel(KernelArgs A, BandArgs B) {
     static_assert(DIRS < 2 || !AFFINE, "H store and tile form: linear gap only");
-    constexpr bool MAXIMA = DIRS == 0 || DIRS == 4;  // pair maxima, no trace
-    constexpr bool CKPT = DIRS == 3 || DIRS == 4;    // tile-form checkpoints
+    constexpr bool MAXIMA = DIRS == 0;  // pair maxima, no trace
+    constexpr bool CKPT = DIRS == 3;    // tile-form checkpoints
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -198,16 +200,14 @@ __global__ void __launch_bounds__(128, AFFINE ? 5 : 8) band_kernel(KernelArgs A,
         const bool store_bnd = band + 1 < nbands;
         const int4* ring_in = nullptr;
         int4* ring_out = nullptr;
-        const int* ck_in = nullptr;  // DIRS 3, 4: the bottom row of the band above, this band's, its tile columns
+        const int* ck_in = nullptr;  // DIRS 3: the bottom row of the band above, this band's, its tile columns
         int* ck_out = nullptr;
         int* ck_col = nullptr;
-        int* tmax = nullptr;  // DIRS 4: this band's tile maxima
         if constexpr (CKPT) {
             int* ckp = B.ck + BP.dir_base;
-            if constexpr (DIRS == 4) tmax = B.ck + BP.ring_off + (int64_t)band * tile_count(lq);
-            if (has_up) ck_in = ckp + (int64_t)(band - 1) * lq;
-            if (store_bnd) ck_out = ckp + (int64_t)band * lq;
-            ck_col = ckp + tile_col_offset(lq, lt) + ((int64_t)band * tile_count(lq)) * kBandRows + lane * kWarpRows;
+            if (has_up) ck_in = ckp + (int64_t)(band - 1) * tile_row_stride(lq);
+            if (store_bnd) ck_out = ckp + (int64_t)band * tile_row_stride(lq);
+            ck_col = ckp + tile_row_ints(lq, lt) + ((int64_t)band * tile_count(lq)) * kBandRows + lane * kWarpRows;
         } else {
             ring_in = B.ring + BP.ring_off + (int64_t)((band + 1) & 1) * lq;
             ring_out = B.ring + BP.ring_off + (int64_t)(band & 1) * lq;
@@ -229,7 +229,6 @@ __global__ void __launch_bounds__(128, AFFINE ? 5 : 8) band_kernel(KernelArgs A,
         int dg_h = 0, dg_m = 0, dg_b = 0;
         int bt_h = 0, bt_m = 0, bt_i = neg, bt_b = 0;
         int mx = 0;
-        int tm = 0;  // DIRS 4: the lane's maximum in its current tile
         int avail = 0;
         bool ok = true;
         // the row above, 32 columns at a time: lane k holds column 32j + k of
@@ -328,9 +327,7 @@ __global__ void __launch_bounds__(128, AFFINE ? 5 : 8) band_kernel(KernelArgs A,
                         Hl[r] = h;
                         up = h;
                     }
-                    if constexpr (DIRS == 4)
-                        tm = max3(tm, max3(Hl[0], Hl[1], Hl[2]), max3(Hl[3], Hl[4], max3(Hl[5], Hl[6], Hl[7])));
-                    else if constexpr (DIRS == 0)
+                    if constexpr (DIRS == 0)
                         mx = max3(mx, max3(Hl[0], Hl[1], Hl[2]), max3(Hl[3], Hl[4], max3(Hl[5], Hl[6], Hl[7])));
                     if constexpr (!MAXIMA) {
                         // candidates: UL cells inside the matrix at or above the
@@ -356,14 +353,6 @@ __global__ void __launch_bounds__(128, AFFINE ? 5 : 8) band_kernel(KernelArgs A,
                         }
                     }
                     bt_h = up;
-                    if constexpr (DIRS == 4) {
-                        // the lane's maximum over a tile's columns, into the tile's maximum
-                        if (((x + 1) & (kTileW - 1)) == 0 || x + 1 == lq) {
-                            atomicMax(tmax + x / kTileW, tm);
-                            mx = max(mx, tm);
-                            tm = 0;
-                        }
-                    }
                     if constexpr (CKPT) {
                         // the lane's rows at the last column of a tile: the next tile's left boundary
                         if (((x + 1) & (kTileW - 1)) == 0 && x + 1 < lq) {

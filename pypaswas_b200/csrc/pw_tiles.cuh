@@ -25,10 +25,11 @@ namespace pw {
 struct TilePair {
     int32_t q, t;     // query / target index (reference orientation)
     int32_t slot;     // pair slot of the wave (metas, candidates, starting points)
-    int32_t pad;
-    int64_t ck;       // int offset of the pair's checkpoints (tile_checkpoint_ints)
+    int32_t fmt;      // checkpoint words: 0 one H each, 1 / 2 the low / high 16-bit half (pw_band_ck.cuh)
+    int64_t rows;     // int offset of the pair's checkpoint rows (tile_row_ints)
+    int64_t cols;     // int offset of its checkpoint columns (tile_col_ints)
     int64_t marks;    // uint32 offset of the pair's mark plane
-    int64_t tm;       // checkpoints of the score sweep (band_kernel<false, 4>): int offset of the tile maxima
+    int64_t tm;       // checkpoints of the score sweep (pw_band_ck.cuh): int offset of the tile maxima
     int64_t scratch;  // byte offset of the pair's walk scratch (lq + lt bytes)
 };
 
@@ -66,8 +67,9 @@ __host__ __device__ __forceinline__ int tile_smem_bytes(int alpha1) {
 
 // One warp's view of a pair in the tile form, with its one cached tile.
 struct TileView {
-    const int* ckp;         // the pair's checkpoints
-    int64_t col_off;        // tile columns' offset in ckp
+    const int* rows;        // the pair's checkpoint rows and columns
+    const int* cols;
+    int fmt;                // their words (TilePair::fmt)
     int ntiles, lq, lt, thr, gap, alpha1, dim;
     const uint8_t* qg;      // query codes (compact)
     const uint8_t* tres;    // target residues (matrix index)
@@ -79,6 +81,10 @@ struct TileView {
     int xmax_c, ymax_c;     // the cached tile's computed extent (its cells up to these coordinates)
     uint32_t* mark_plane;   // the pair's mark bits
 
+    // H of a checkpoint word: its half, without the row words' tag (pw_band_ck.cuh)
+    __device__ __forceinline__ int h_of(int w) const {
+        return fmt == 0 ? w & 0x7fffffff : fmt == 1 ? w & 0xffff : (w >> 16) & 0x7fff;
+    }
     __device__ __forceinline__ uint32_t* mark_word(int x, int y) const {
         return mark_plane + (((int64_t)y * lq + x) >> 5);
     }
@@ -127,16 +133,16 @@ struct TileView {
         // border row (r = 0): the row above, columns x0 - 1 .. x0 + ncol - 1; 0 above band 0 and left of column 0
         for (int k = lane; k <= ncol; k += kWarp) {
             const int xx = x0 - 1 + k;
-            hs[k * kTileRows] = (b > 0 && xx >= 0) ? __ldcg(ckp + (int64_t)(b - 1) * lq + xx) : 0;
+            hs[k * kTileRows] = (b > 0 && xx >= 0) ? h_of(__ldcg(rows + (int64_t)(b - 1) * tile_row_stride(lq) + xx)) : 0;
         }
         for (int k = lane; k < ncol; k += kWarp) qc[k] = qg[x0 + k];
         // border column (c = 0): the checkpointed last column of tile j - 1
         int Hl[kWarpRows];
         if (j > 0) {
-            const int4* src = (const int4*)(ckp + col_off + ((int64_t)b * ntiles + j) * kBandRows + lane * kWarpRows);
+            const int4* src = (const int4*)(cols + ((int64_t)b * ntiles + j) * kBandRows + lane * kWarpRows);
             const int4 v0 = __ldcg(src), v1 = __ldcg(src + 1);
-            Hl[0] = v0.x; Hl[1] = v0.y; Hl[2] = v0.z; Hl[3] = v0.w;
-            Hl[4] = v1.x; Hl[5] = v1.y; Hl[6] = v1.z; Hl[7] = v1.w;
+            Hl[0] = h_of(v0.x); Hl[1] = h_of(v0.y); Hl[2] = h_of(v0.z); Hl[3] = h_of(v0.w);
+            Hl[4] = h_of(v1.x); Hl[5] = h_of(v1.y); Hl[6] = h_of(v1.z); Hl[7] = h_of(v1.w);
         } else {
 #pragma unroll
             for (int r = 0; r < kWarpRows; ++r) Hl[r] = 0;
@@ -254,8 +260,9 @@ __device__ __forceinline__ TileView tile_view(const KernelArgs& A, const TileArg
     TileView v;
     v.lq = A.q.len[tp.q];
     v.lt = A.t.len[tp.t];
-    v.ckp = T.ck + tp.ck;
-    v.col_off = tile_col_offset(v.lq, v.lt);
+    v.rows = T.ck + tp.rows;
+    v.cols = T.ck + tp.cols;
+    v.fmt = tp.fmt;
     v.ntiles = tile_count(v.lq);
     v.thr = thr;
     v.gap = A.P.gap_i;
@@ -513,7 +520,7 @@ __global__ void __launch_bounds__(32) tile_ops_kernel(KernelArgs A, TraceArgs TA
     }
 }
 
-// ---- candidates from the score sweep's checkpoints (band_kernel<false, 4>)
+// ---- candidates from the score sweep's checkpoints (pw_band_ck.cuh)
 
 // The candidate threshold of a pair (default_main.cu:609,
 // SmithWatermanCuda.py:269-275), as band_kernel computes it.
