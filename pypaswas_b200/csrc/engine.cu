@@ -242,6 +242,7 @@ struct pw_engine {
     DevBuf band_pairs, band_entries, band_prog, band_max, band_ring, band_out;  // band sweep (pw_band.cuh)
     DevBuf tile_ck, tile_marks, tile_pairs, slot_tile;                        // tile form (pw_tiles.cuh)
     DevBuf tile_pairs_alt, tile_sel, tile_cnt, tile_acc, tile_scratch, tile_ops;
+    DevBuf tile_slot_base, tile_slot, tile_list, tile_codes;                  // codes of the walks' tiles, computed ahead
     DevBuf band_over;                                                         // band_ck_kernel: pairs past 16 bits
     // explicit pairs: the score sweep's tile-form checkpoints (band_ck_kernel)
     DevBuf p1_ck;
@@ -1825,7 +1826,10 @@ static int run_tile_cands(pw_engine* e, KernelArgs A, TileArgs T, const TilePair
     cudaEventRecord(a, e->stream);
     const int n = (int)list.size();
     PW_LAUNCH(tile_select_kernel, n, 256, 0, e->stream, A, T, dev_list, e->tile_sel.as<int2>(), cnt, (int)tiles);
-    PW_LAUNCH(tile_cand_kernel, e->sm_count, kWarp, tsmem, e->stream, A, T, dev_list,
+    int per_sm = 0;
+    if ((c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tile_cand_kernel, kWarp, tsmem)) != cudaSuccess)
+        return cuda_fail(e, c, "occupancy");
+    PW_LAUNCH(tile_cand_kernel, e->sm_count * std::max(1, per_sm), kWarp, tsmem, e->stream, A, T, dev_list,
               (const int2*)e->tile_sel.as<int2>(), (const int*)cnt, cnt + 1);
     PW_LAUNCH(tile_cand_count_kernel, (n + 127) / 128, 128, 0, e->stream, A, dev_list, n);
     e->launches += 3;
@@ -1840,6 +1844,9 @@ static int run_tile_cands(pw_engine* e, KernelArgs A, TileArgs T, const TilePair
     cudaEventDestroy(b);
     return PW_OK;
 }
+
+// Tiles whose codes a wave computes ahead of its walks (16 KB each).
+constexpr int64_t kMaxTileSlots = 1 << 14;
 
 // The phase-2 warp items as band pairs.
 static std::vector<BandPair> band_pairs_of(pw_engine* e, const std::vector<WorkItem>& items) {
@@ -2638,7 +2645,8 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         TT.ops_total = n_tile > 0 ? e->tile_acc.as<unsigned long long>() + 1 : nullptr;
         const int tsmem = tile_smem_bytes(Aref.P.alpha + 1);
         if (n_tile > 0 && tsmem > 48 * 1024) {
-            if ((c = cudaFuncSetAttribute(tile_collect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem)) != cudaSuccess ||
+            if ((c = cudaFuncSetAttribute(tile_codes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem)) != cudaSuccess ||
+                (c = cudaFuncSetAttribute(tile_collect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem)) != cudaSuccess ||
                 (c = cudaFuncSetAttribute(tile_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem)) != cudaSuccess ||
                 (c = cudaFuncSetAttribute(tile_ops_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem)) != cudaSuccess)
                 return cuda_fail(e, c, "tile kernels smem");
@@ -2806,6 +2814,47 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         TA.slot_tile = TT.slot_tile;
         const int tb = 128;
         const int gb = (int)((n_pairs + tb - 1) / tb);
+        // the tile form's walks: the tiles along the candidates' diagonals
+        // computed at once on the whole GPU when pairs have more than a few
+        // tiles (one or two a pair are computed as fast by the walk itself)
+        int64_t tiles_all = 0;
+        std::vector<int64_t> slot_base((size_t)n_tile);
+        for (int k = 0; k < n_tile; ++k) {
+            slot_base[k] = tiles_all;
+            tiles_all += tile_bands(tlen[tps[k].t]) * tile_count(qlen[tps[k].q]);
+        }
+        int64_t max_slots = std::min<int64_t>(tiles_all, kMaxTileSlots);
+        if (e->wave_limit > 0)  // within the caller's bound, beside the wave's marks
+            max_slots = std::min<int64_t>(max_slots, e->wave_limit / 4 / (kTileWords * 4));
+        if (tiles_all > 4 * (int64_t)n_tile && max_slots > 0 &&
+            e->tile_codes.reserve(e->stream, (size_t)max_slots * kTileWords * 4) != cudaSuccess) {
+            cudaGetLastError();  // no room: the walks compute their tiles
+            max_slots = 0;
+        }
+        if (tiles_all > 4 * (int64_t)n_tile && max_slots > 0) {
+            if ((c = upload(e, e->tile_slot_base, slot_base)) != cudaSuccess ||
+                (c = e->tile_slot.reserve(e->stream, (size_t)tiles_all * sizeof(int32_t))) != cudaSuccess ||
+                (c = cudaMemsetAsync(e->tile_slot.p, 0xff, (size_t)tiles_all * sizeof(int32_t), e->stream)) != cudaSuccess ||
+                (c = e->tile_list.reserve(e->stream, (size_t)max_slots * sizeof(int2))) != cudaSuccess ||
+                (c = e->tile_cnt.reserve(e->stream, 4 * sizeof(int))) != cudaSuccess ||
+                (c = cudaMemsetAsync(e->tile_cnt.p, 0, 4 * sizeof(int), e->stream)) != cudaSuccess)
+                return cuda_fail(e, c, "alloc tile slots");
+            TT.slot_base = e->tile_slot_base.as<int64_t>();
+            TT.tile_slot = e->tile_slot.as<int32_t>();
+            TT.tile_codes = e->tile_codes.as<uint32_t>();
+            TT.tile_list = e->tile_list.as<int2>();
+            TT.tile_count = e->tile_cnt.as<int>();
+            TT.max_slots = (int)max_slots;
+            TT.use_tm = p1ck ? 1 : 0;
+            int per_sm = 0;
+            if ((c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tile_codes_kernel, kWarp, tsmem)) != cudaSuccess)
+                return cuda_fail(e, c, "occupancy");
+            const int grid = (int)std::min<int64_t>(tiles_all, (int64_t)e->sm_count * std::max(1, per_sm));
+            PW_LAUNCH(tile_corridor_kernel, n_tile, 128, 0, e->stream, Aw, TA, TT);
+            PW_LAUNCH(tile_codes_kernel, grid, kWarp, tsmem, e->stream, Aw, TA, TT, e->tile_cnt.as<int>() + 1);
+            e->launches += 2;
+            if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "tile codes launch");
+        }
         if (e->affine)
             PW_LAUNCH(collect_kernel<true>, gb, tb, 0, e->stream, TA);
         else

@@ -3,19 +3,26 @@
 // The band direction sweep of a long pair stores a 4-bit code for every cell
 // (a 30 kb x 30 kb pair: 450 MB), and the walks then follow their paths one
 // dependent global load a step.  The tile form stores no cell codes: the
-// checkpoint sweep (band_kernel<false, 3>) finds the candidates and keeps
-// every band's bottom row and, per band, the H column at every kTileW-th
-// column.  From those, one warp recomputes the codes of any 256 x kTileW tile
-// into shared memory -- the same codes, bit for bit, as the direction sweep
-// (same recurrence, same boundary values, same classification) -- and the
-// covering chains, the walks and the column operations read them there.
+// checkpoint sweep (band_kernel<false, 3>, or the score sweep of listed pairs
+// itself, pw_band_ck.cuh) keeps every band's bottom row and, per band, the H
+// column at every kTileW-th column.  From those, one warp recomputes the codes
+// of any 256 x kTileW tile -- the same codes, bit for bit, as the direction
+// sweep (same recurrence, same boundary values, same classification): 16 KB,
+// one word (8 rows) a lane and column.
 //
-// One warp per pair (collect, walk) or per hit (operations); every lane runs
-// the same path in step, so a tile miss is recomputed by the whole warp.  The
-// walk follows up to 32 steps by the codes alone and then checks the cells'
-// marks (one load per lane): a walk never revisits its own cells, so the
-// first marked cell of the batch is where the reference's walk stops.  Marks
-// are one bit per cell, bit y * lq + x of the pair's plane.
+// Tiles do not depend on one another, and a path runs close to a diagonal.  So
+// when pairs have many tiles, tile_corridor_kernel lists the tiles along the
+// diagonals of the candidates and tile_codes_kernel computes them all at once
+// on the whole GPU; the covering chains and the walks, one warp a pair, then
+// copy the tiles they pass into shared memory (1 us) and compute only those
+// that the list missed (20 us).  Computing every tile where the walk met it
+// took 11 ms for a 25 kb path.
+//
+// A walk reads 32 cells of its diagonal at a time, one a lane, and takes the
+// run of plain diagonal steps and the step after it together.  Marks (one bit
+// per cell, bit y * lq + x of the pair's plane) are checked with one load per
+// lane for these cells: a walk never revisits its own cells, so the first
+// marked cell of the batch is where the reference's walk stops.
 #pragma once
 #include "pw_band.cuh"
 
@@ -43,6 +50,16 @@ struct CandSink {
 struct TileArgs {
     const TilePair* pairs;
     int n_pairs;
+    // codes computed ahead (null: none): per pair its tiles' slots, at
+    // slot_base[pair index] + band * ntiles + tile, -1 where there is none;
+    // slot s holds kTileWords words
+    const int64_t* slot_base;
+    int32_t* tile_slot;
+    uint32_t* tile_codes;
+    int2* tile_list;           // per slot: (pair index, band * ntiles + tile)
+    int* tile_count;           // slots asked for (may exceed max_slots)
+    int max_slots;
+    int use_tm;                // the pairs have tile maxima (TilePair::tm)
     const int* ck;
     uint32_t* marks;
     const int32_t* slot_tile;  // per pair slot: index into pairs, -1 for the other pairs
@@ -55,14 +72,12 @@ struct TileArgs {
     unsigned long long* ops_bound;  // tile_collect_kernel: sum of starts x (lq + lt) over the pairs
 };
 
-// The cached tile holds H, int32, column-major with a one-cell border:
-// column c = x - x0 + 1 (c = 0: the left boundary, column x0 - 1), row
-// r = y - yb + 1 (r = 0: the row above the band); kTileRows values a column.
-constexpr int kTileRows = kBandRows + 1;
-constexpr int kTileCells = (kTileW + 1) * kTileRows;
+// A tile's codes: word (x - x0) * 32 + (y - yb) / 8 holds the nibbles of 8 rows.
+constexpr int kTileWords = kTileW * kWarp;
 
 __host__ __device__ __forceinline__ int tile_smem_bytes(int alpha1) {
-    return ((kTileCells * 4 + 15) & ~15) + ((kWarp * alpha1 * kWarpRows + 15) & ~15) + kTileW;
+    // codes, profile, the row above with its corner, query codes
+    return kTileWords * 4 + ((kWarp * alpha1 * kWarpRows + 15) & ~15) + (kTileW + 4) * 4 + kTileW;
 }
 
 // One warp's view of a pair in the tile form, with its one cached tile.
@@ -74,11 +89,14 @@ struct TileView {
     const uint8_t* qg;      // query codes (compact)
     const uint8_t* tres;    // target residues (matrix index)
     const int8_t* cmat;
-    int* hs;                // shared: the cached tile's H with its border
+    uint32_t* codes;        // shared: the cached tile's codes
     uint2* prof;            // shared: [lane][alpha1] scores of the lane's 8 rows in the cached band
+    int* top;               // shared: the row above the tile, columns x0 - 1 ..
     uint8_t* qc;            // shared: the query codes of the tile's columns
+    const int32_t* slots;   // the pair's tile slots (null: none)
+    const uint32_t* slot_codes;
     int band, tile, prof_band, x0, yb;
-    int xmax_c, ymax_c;     // the cached tile's computed extent (its cells up to these coordinates)
+    int xmax_c, ymax_c;     // the cached tile's extent (its cells up to these coordinates)
     uint32_t* mark_plane;   // the pair's mark bits
 
     // H of a checkpoint word: its half, without the row words' tag (pw_band_ck.cuh)
@@ -95,18 +113,40 @@ struct TileView {
     __device__ __forceinline__ void mark(int x, int y) const { atomicOr(mark_word(x, y), mark_bit(x, y)); }
     __device__ __forceinline__ void unmark(int x, int y) const { atomicAnd(mark_word(x, y), ~mark_bit(x, y)); }
 
+    // Makes tile (band b, tile j) the cached one, as far as cell (xneed,
+    // yneed); every lane of the warp calls it.
     __device__ void load(int b, int j, int xneed, int yneed) {
-        load_h<false>(b, j, CandSink{nullptr, 0, nullptr}, xneed, yneed);
+        const int slot = slots ? slots[(int64_t)b * ntiles + j] : -1;
+        if (slot < 0) {
+            compute<false>(b, j, CandSink{nullptr, 0, nullptr}, xneed, yneed);
+            return;
+        }
+        const int lane = threadIdx.x & 31;
+        __syncwarp();
+        x0 = j * kTileW;
+        yb = b * kBandRows;
+        const uint4* src = (const uint4*)(slot_codes + (int64_t)slot * kTileWords);
+        const int n = (xneed - x0 + 1) * (kWarp / 4);
+#pragma unroll 8
+        for (int i = lane; i < n; i += kWarp) ((uint4*)codes)[i] = __ldcg(src + i);
+        band = b;
+        tile = j;
+        xmax_c = xneed;
+        ymax_c = yb + kBandRows - 1;
+        __syncwarp();
     }
 
-    // Recomputes the H values of tile (band b, tile j) and its border, as far
-    // as cell (xneed, yneed): the columns up to xneed and the lanes up to
-    // yneed's (a walk only moves up and left, so it needs no more of the
-    // tile); every lane of the warp calls it.  CANDS: the whole tile, and its
-    // candidates into the sink, with the band sweep's test (UL cells inside
-    // the matrix at or above the threshold).
+    // Computes the codes of tile (band b, tile j) into `codes`, as far as cell
+    // (xneed, yneed): the columns up to xneed and the lanes up to yneed's (a
+    // walk only moves up and left, so it needs no more of the tile).  The
+    // code: LEFT when the left neighbour plus the gap reaches H, else UP when
+    // the upper one does, else UL; NO where H is 0; the stop flag on a UL cell
+    // inside the matrix with a zero diagonal neighbour, the candidate flag on
+    // a UL cell at or above the pair's threshold.  CANDS: its candidates into
+    // the sink, with the band sweep's test (UL cells inside the matrix at or
+    // above the threshold).
     template <bool CANDS>
-    __device__ void load_h(int b, int j, CandSink sink, int xneed, int yneed) {
+    __device__ void compute(int b, int j, CandSink sink, int xneed, int yneed) {
         const int lane = threadIdx.x & 31;
         __syncwarp();
         yb = b * kBandRows;
@@ -130,13 +170,13 @@ struct TileView {
         }
         const int ncol = min(min(kTileW, lq - x0), xneed - x0 + 1);
         const int lanes_need = min(kWarp - 1, (yneed - yb) >> 3);
-        // border row (r = 0): the row above, columns x0 - 1 .. x0 + ncol - 1; 0 above band 0 and left of column 0
+        // the row above, columns x0 - 1 .. x0 + ncol - 1; 0 above band 0 and left of column 0
         for (int k = lane; k <= ncol; k += kWarp) {
             const int xx = x0 - 1 + k;
-            hs[k * kTileRows] = (b > 0 && xx >= 0) ? h_of(__ldcg(rows + (int64_t)(b - 1) * tile_row_stride(lq) + xx)) : 0;
+            top[k] = (b > 0 && xx >= 0) ? h_of(__ldcg(rows + (int64_t)(b - 1) * tile_row_stride(lq) + xx)) : 0;
         }
         for (int k = lane; k < ncol; k += kWarp) qc[k] = qg[x0 + k];
-        // border column (c = 0): the checkpointed last column of tile j - 1
+        // the left boundary: the checkpointed last column of tile j - 1
         int Hl[kWarpRows];
         if (j > 0) {
             const int4* src = (const int4*)(cols + ((int64_t)b * ntiles + j) * kBandRows + lane * kWarpRows);
@@ -147,34 +187,32 @@ struct TileView {
 #pragma unroll
             for (int r = 0; r < kWarpRows; ++r) Hl[r] = 0;
         }
-#pragma unroll
-        for (int r = 0; r < kWarpRows; ++r) hs[1 + lane * kWarpRows + r] = Hl[r];
         __syncwarp();
         // the skewed wavefront of band_kernel over the tile's columns; a lane
         // that has not started hands down its left boundary's bottom value
         const int ymine = yb + lane * kWarpRows;
         const int rows_left = lt - ymine;
         int bt_h = Hl[kWarpRows - 1];
-        int up_h = lane == 0 ? hs[0] : 0;  // lane 0: the corner, its first cell's diagonal
+        int up_h = lane == 0 ? top[0] : 0;  // lane 0: the corner, its first cell's diagonal
         const int nsteps = ncol + lanes_need;
         // the shared-memory reads of a step (its scores; lane 0: the row
         // above) are issued one step ahead, off the recurrence's path
         auto fetch_pw = [&](int c) -> uint2 {
             return (c >= 0 && c < ncol) ? prof[lane * alpha1 + qc[c]] : make_uint2(0u, 0u);
         };
-        auto fetch_top = [&](int c) -> int { return (b > 0 && c >= 0 && c < ncol) ? hs[(c + 1) * kTileRows] : 0; };
+        auto fetch_top = [&](int c) -> int { return c < ncol ? top[c + 1] : 0; };
         uint2 pw_n = fetch_pw(-lane);
-        int top_n = lane == 0 ? fetch_top(0) : 0;
+        int top_n = fetch_top(0);
         for (int s = 0; s < nsteps; ++s) {
             const int xl = s - lane;
             const int x = x0 + xl;
             const bool active = xl >= 0 && xl < ncol;
             const uint2 pw = pw_n;
-            const int top = top_n;
+            const int top_h = top_n;
             pw_n = fetch_pw(xl + 1);
-            if (lane == 0) top_n = fetch_top(xl + 1);
+            if (lane == 0) top_n = fetch_top(s + 1);
             int rh = __shfl_up_sync(0xffffffffu, bt_h, 1);
-            if (lane == 0) rh = top;
+            if (lane == 0) rh = top_h;
             const int dg_h = x == 0 ? 0 : up_h;
             up_h = rh;
             if (active) {
@@ -184,23 +222,33 @@ struct TileView {
 #pragma unroll
                     for (int r = 0; r < kWarpRows; ++r) Hold[r] = Hl[r];
                 }
+                // the stop flag needs a cell inside the matrix: x > 0 and y > 0
+                const uint32_t stop = x > 0 ? kUL | kStopFlag : kUL;
+                const uint32_t stop0 = ymine > 0 ? stop : (uint32_t)kUL;
+                uint32_t w = 0;
 #pragma unroll
                 for (int r = 0; r < kWarpRows; ++r) {
-                    const int sc = prof_score(pw, r);
                     const int left = Hl[r];
-                    int h = addmax(left, gap, diag + sc);
-                    h = addmax_relu(up, gap, h);
+                    const int ls = left + gap, us = up + gap;
+                    const int m = max3(ls, us, diag + prof_score(pw, r));
+                    uint32_t cd = diag == 0 ? (r > 0 ? stop : stop0) : (uint32_t)kUL;
+                    cd = us == m ? (uint32_t)kUp : cd;
+                    cd = ls == m ? (uint32_t)kLeft : cd;
+                    cd = m > 0 ? cd : 0u;
+                    w += cd << (4 * r);
                     diag = left;
-                    Hl[r] = h;
-                    up = h;
+                    up = max(m, 0);
+                    Hl[r] = up;
                 }
-                if constexpr (CANDS) {
-                    const int smax = max(max3(Hl[0], Hl[1], Hl[2]), max3(Hl[3], Hl[4], max3(Hl[5], Hl[6], Hl[7])));
-                    if (smax >= thr) {
+                const int smax = max(max3(Hl[0], Hl[1], Hl[2]), max3(Hl[3], Hl[4], max3(Hl[5], Hl[6], Hl[7])));
+                if (smax >= thr) {
 #pragma unroll
-                        for (int r = 0; r < kWarpRows; ++r) {
-                            const int h = Hl[r], upv = r > 0 ? Hl[r - 1] : up_h;
-                            if (h < thr || h <= 0 || r >= rows_left || h == Hold[r] + gap || h == upv + gap) continue;
+                    for (int r = 0; r < kWarpRows; ++r) {
+                        const int h = Hl[r];
+                        if (h < thr || ((w >> (4 * r)) & 3u) != kUL) continue;
+                        w |= (uint32_t)kCand << (4 * r);
+                        if constexpr (CANDS) {
+                            if (r >= rows_left) continue;
                             const int k = atomicAdd(sink.n, 1);
                             if (k < sink.cap) {
                                 Cand cc;
@@ -214,9 +262,7 @@ struct TileView {
                     }
                 }
                 bt_h = up;
-                int* dst = hs + (xl + 1) * kTileRows + 1 + lane * kWarpRows;
-#pragma unroll
-                for (int r = 0; r < kWarpRows; ++r) dst[r] = Hl[r];
+                codes[xl * kWarp + lane] = w;
             } else if (xl < 0) {
                 bt_h = Hl[kWarpRows - 1];
             }
@@ -228,35 +274,38 @@ struct TileView {
         __syncwarp();
     }
 
-    // The 4-bit code of cell (x, y), derived from the cached H values exactly
-    // as the direction sweep classifies it (LEFT when the left neighbour plus
-    // the gap reaches H, else UP, else UL; NO where H is 0; the stop flag on a
-    // UL cell inside the matrix with a zero diagonal neighbour, the candidate
-    // flag on a UL cell at or above the pair's threshold); kNo outside the
-    // matrix.  Uniform across the warp.
+    // Cell (x, y) of the matrix and those of its tile above and left of it in
+    // the cache.  A miss, or a cell past the cached extent (the covering chains
+    // of several candidates reuse a tile): far enough for both.
+    __device__ __forceinline__ void ensure(int x, int y) {
+        const int b = y >> 8, j = x / kTileW;
+        if (b == band && j == tile && x <= xmax_c && y <= ymax_c) return;
+        const bool same = b == band && j == tile;
+        load(b, j, same ? max(x, xmax_c) : x, same ? max(y, ymax_c) : y);
+    }
+    // The 4-bit code of a cell in the cache.
+    __device__ __forceinline__ uint32_t cached(int x, int y) const {
+        return (codes[(x - x0) * kWarp + ((y - yb) >> 3)] >> (4 * (y & 7))) & 15u;
+    }
+    // The code of any cell (kNo outside the matrix); uniform across the warp.
     __device__ __forceinline__ uint32_t code(int x, int y) {
         if (x < 0 || y < 0 || x >= lq || y >= lt) return kNo;
-        const int b = y >> 8, j = x / kTileW;
-        if (b != band || j != tile || x > xmax_c || y > ymax_c) {
-            // a miss, or a cell past the cached extent (the covering chains of
-            // several candidates reuse a tile): recompute far enough for both
-            const bool same = b == band && j == tile;
-            load(b, j, same ? max(x, xmax_c) : x, same ? max(y, ymax_c) : y);
-        }
-        const int* c = hs + (x - x0 + 1) * kTileRows + (y - yb + 1);
-        const int h = c[0], l = c[-kTileRows], u = c[-1], d = c[-kTileRows - 1];
-        if (h <= 0) return kNo;
-        if (h == l + gap) return kLeft;
-        if (h == u + gap) return kUp;
-        uint32_t cd = kUL;
-        if (x > 0 && y > 0 && d == 0) cd |= kStopFlag;
-        if (h >= thr) cd |= kCand;
-        return cd;
+        ensure(x, y);
+        return cached(x, y);
+    }
+    // Lane i's cell of the diagonal up from (x, y), a cell of the matrix: its
+    // code when it lies in the cached tile.
+    __device__ __forceinline__ bool diagonal(int x, int y, int lane, uint32_t* cd) {
+        ensure(x, y);
+        const int cx = x - lane, cy = y - lane;
+        const bool in = cx >= x0 && cy >= yb;
+        *cd = in ? cached(cx, cy) : (uint32_t)kNo;
+        return in;
     }
 };
 
-__device__ __forceinline__ TileView tile_view(const KernelArgs& A, const TileArgs& T, const TilePair& tp, int thr,
-                                              unsigned char* smem) {
+__device__ __forceinline__ TileView tile_view(const KernelArgs& A, const TileArgs& T, const TilePair& tp, int index,
+                                              int thr, unsigned char* smem) {
     TileView v;
     v.lq = A.q.len[tp.q];
     v.lt = A.t.len[tp.t];
@@ -271,9 +320,12 @@ __device__ __forceinline__ TileView tile_view(const KernelArgs& A, const TileArg
     v.qg = A.q.codes + A.q.code_off[tp.q];
     v.tres = A.t.codes + A.t.code_off[tp.t];
     v.cmat = A.cmat_i8;
-    v.hs = (int*)smem;
-    v.prof = (uint2*)(smem + ((kTileCells * 4 + 15) & ~15));
-    v.qc = (uint8_t*)v.prof + ((kWarp * v.alpha1 * kWarpRows + 15) & ~15);
+    v.codes = (uint32_t*)smem;
+    v.prof = (uint2*)(v.codes + kTileWords);
+    v.top = (int*)((uint8_t*)v.prof + ((kWarp * v.alpha1 * kWarpRows + 15) & ~15));
+    v.qc = (uint8_t*)(v.top + kTileW + 4);
+    v.slots = T.slot_base && index >= 0 ? T.tile_slot + T.slot_base[index] : nullptr;
+    v.slot_codes = T.tile_codes;
     v.x0 = 0;
     v.yb = 0;
     v.band = -1;
@@ -283,6 +335,70 @@ __device__ __forceinline__ TileView tile_view(const KernelArgs& A, const TileArg
     v.prof_band = -1;
     v.mark_plane = T.marks + tp.marks;
     return v;
+}
+
+// Columns and rows that a corridor extends beyond a diagonal (indels move the
+// path off it).
+constexpr int kCorridor = 32;
+// Tiles whose maximum is below this fraction of the pair's are not listed: the
+// diagonal has left the alignment (its first few tiles are then computed where
+// the walk meets them).
+constexpr int kCorridorFade = 32;
+
+// Lists the tiles along the diagonals of each pair's candidates, one block a
+// pair: a lane per tile column of a diagonal, the bands that the diagonal
+// crosses there within kCorridor rows.
+__global__ void tile_corridor_kernel(KernelArgs A, TraceArgs TA, TileArgs T) {
+    const TilePair tp = T.pairs[blockIdx.x];
+    const PairMeta pm = TA.metas[tp.slot];
+    const Cand* cl = TA.cands + TA.cand_base[tp.slot];
+    const int lq = A.q.len[tp.q], lt = A.t.len[tp.t];
+    const int ntiles = tile_count(lq), nb = (int)tile_bands(lt);
+    int32_t* slot = T.tile_slot + T.slot_base[blockIdx.x];
+    const int* tm = T.use_tm ? T.ck + tp.tm : nullptr;
+    const int fade = (int)fminf(pm.max_f, 1.0e9f) / kCorridorFade;
+    for (int k = 0; k < pm.n_cand; ++k) {
+        const int x = cl[k].x, y = cl[k].y;
+        for (int j = x / kTileW - (int)threadIdx.x; j >= 0; j -= blockDim.x) {
+            // rows of the diagonal (and the corridor around it) in this tile column
+            const int xl = j * kTileW, xr = min(x, xl + kTileW - 1);
+            const int ylo = y - (x - xl) - kCorridor, yhi = min(y - (x - xr) + kCorridor, y);
+            if (yhi < 0) continue;
+            for (int b = max(ylo, 0) >> 8; b <= min(yhi >> 8, nb - 1); ++b) {
+                const int64_t i = (int64_t)b * ntiles + j;
+                if (tm && tm[i] < fade) continue;
+                if (atomicCAS(&slot[i], -1, -2) != -1) continue;
+                const int s = atomicAdd(T.tile_count, 1);
+                if (s < T.max_slots) {
+                    T.tile_list[s] = make_int2((int)blockIdx.x, (int)i);
+                    slot[i] = s;
+                }
+            }
+        }
+    }
+}
+
+// Computes the codes of the listed tiles into their slots; one warp a block,
+// persistent.
+__global__ void __launch_bounds__(32) tile_codes_kernel(KernelArgs A, TraceArgs TA, TileArgs T, int* counter) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x;
+    const int total = min(*T.tile_count, T.max_slots);
+    for (;;) {
+        int it = 0;
+        if (lane == 0) it = atomicAdd(counter, 1);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= total) break;
+        const int2 en = T.tile_list[it];
+        const TilePair tp = T.pairs[en.x];
+        TileView v = tile_view(A, T, tp, -1, TA.metas[tp.slot].thr_i, smem);
+        const int b = en.y / v.ntiles, j = en.y % v.ntiles;
+        v.compute<false>(b, j, CandSink{nullptr, 0, nullptr}, v.lq - 1, b * kBandRows + kBandRows - 1);
+        uint4* dst = (uint4*)(T.tile_codes + (int64_t)it * kTileWords);
+        const int n = min(kTileW, v.lq - v.x0) * (kWarp / 4);
+#pragma unroll 8
+        for (int i = lane; i < n; i += kWarp) __stcg(dst + i, ((const uint4*)v.codes)[i]);
+    }
 }
 
 // collect_kernel for the pairs of the tile form: the covering chains, the
@@ -295,27 +411,32 @@ __global__ void __launch_bounds__(32) tile_collect_kernel(KernelArgs A, TraceArg
     const PairMeta pm = TA.metas[p];
     Cand* cl = TA.cands + TA.cand_base[p];
     const int n = pm.n_cand;
-    TileView v = tile_view(A, T, tp, pm.thr_i, smem);
+    TileView v = tile_view(A, T, tp, (int)blockIdx.x, pm.thr_i, smem);
     // marking chains: the nearest candidate up a candidate's chain is covered
     // (a lone candidate has no other candidate to cover)
     for (int k = 0; k < n && n > 1; ++k) {
         int x = cl[k].x - 1, y = cl[k].y - 1;
         while (x >= 0 && y >= 0) {
-            const uint32_t cd = v.code(x, y);
+            // the run of plain UL cells up the diagonal, then the cell after it
+            uint32_t cd;
+            const bool in = v.diagonal(x, y, lane, &cd);
+            const unsigned ul = __ballot_sync(0xffffffffu, in && (cd & 3) == kUL && !(cd & kCand));
+            const unsigned ins = __ballot_sync(0xffffffffu, in);
+            const int run = ul == 0xffffffffu ? kWarp : __ffs(~ul) - 1;
+            x -= run;
+            y -= run;
+            if (run == kWarp || !((ins >> run) & 1u)) continue;  // into the next tile
+            cd = __shfl_sync(0xffffffffu, cd, run);
             const int d = cd & 3;
             if (cd & kCand) {
                 if (lane == 0) v.mark(x, y);  // covered
                 break;
             }
             if (d == kNo) break;
-            if (d == kUL) {
-                --x;
+            if (d == kUp)
                 --y;
-            } else if (d == kUp) {
-                --y;
-            } else {
+            else
                 --x;
-            }
         }
     }
     __syncwarp();
@@ -357,7 +478,7 @@ __global__ void __launch_bounds__(32) tile_walk_kernel(KernelArgs A, TraceArgs T
     const PairMeta pm = TA.metas[p];
     const Cand* cl = TA.cands + TA.cand_base[p];
     const int m = TA.n_starts[p];
-    TileView v = tile_view(A, T, tp, pm.thr_i, smem);
+    TileView v = tile_view(A, T, tp, (int)blockIdx.x, pm.thr_i, smem);
     const uint8_t* qs = TA.q.raw + TA.q.raw_off[pm.query];
     const uint8_t* ts = TA.t.raw + TA.t.raw_off[pm.target];
     const bool same_id = TA.q.key[pm.query] == TA.t.key[pm.target];
@@ -383,37 +504,21 @@ __global__ void __launch_bounds__(32) tile_walk_kernel(KernelArgs A, TraceArgs T
         int s_start = x + 1, t_start = y + 1, ncols = 0, mt = 0, mm = 0;
         bool go = show && x >= 0 && y >= 0 && dir != kStopDir && dir != 32;  // :761
         while (go) {
-            // up to 32 steps by the codes alone; lane i keeps step i
-            int sx = 0, sy = 0, sd = kNo, n = 0;
-            bool end = false;
-            int cx = x, cy = y;
-            for (int i = 0; i < kWarp; ++i) {
-                if (cx < 0 || cy < 0) {
-                    end = true;
-                    break;
-                }
-                const uint32_t cd = v.code(cx, cy);
-                const int d = cd & 3;
-                const int dd = (d == kUL && (cd & kStopFlag)) ? kStopDir : d;
-                if (lane == i) {
-                    sx = cx;
-                    sy = cy;
-                    sd = dd;
-                }
-                ++n;
-                if (dd == kStopDir || dd == kNo) {  // the walk ends at this cell
-                    end = true;
-                    break;
-                }
-                if (dd == kUL) {
-                    --cx;
-                    --cy;
-                } else if (dd == kLeft) {
-                    --cx;
-                } else {
-                    --cy;
-                }
-            }
+            if (x < 0 || y < 0) break;
+            // the run of plain diagonal steps from here, a lane a step, and the
+            // step after it, by the codes alone
+            uint32_t cd;
+            const bool in = v.diagonal(x, y, lane, &cd);
+            const int sx = x - lane, sy = y - lane;
+            const int sd = (cd & 3) == kUL && (cd & kStopFlag) ? kStopDir : (int)(cd & 3);
+            const unsigned ul = __ballot_sync(0xffffffffu, in && sd == kUL);
+            const unsigned ins = __ballot_sync(0xffffffffu, in);
+            const int run = ul == 0xffffffffu ? kWarp : __ffs(~ul) - 1;
+            const bool more = run < kWarp && ((ins >> run) & 1u);
+            const int n = run + (more ? 1 : 0);  // at least 1: lane 0's cell is in the tile
+            const int last = more ? __shfl_sync(0xffffffffu, sd, run) : (int)kUL;
+            const bool end = last == kStopDir || last == kNo;  // the walk ends at that cell
+            const int cx = x - run - (last == kLeft ? 1 : 0), cy = y - run - (last == kUp ? 1 : 0);
             // the first marked cell of the batch ends the walk there (IN_ALIGNMENT)
             const unsigned hit_mark = __ballot_sync(0xffffffffu, lane < n && v.marked(sx, sy));
             const int f = hit_mark ? __ffs(hit_mark) - 1 : n;
@@ -493,7 +598,7 @@ __global__ void __launch_bounds__(32) tile_ops_kernel(KernelArgs A, TraceArgs TA
     const int ti = T.slot_tile[H.pair];
     if (ti < 0) return;
     const TilePair tp = T.pairs[ti];
-    TileView v = tile_view(A, T, tp, TA.metas[H.pair].thr_i, smem);
+    TileView v = tile_view(A, T, tp, ti, TA.metas[H.pair].thr_i, smem);
     int x = H.end_x, y = H.end_y;
     char* o = TA.ops + H.ops_offset;
     char mine = 0;
@@ -577,9 +682,9 @@ __global__ void __launch_bounds__(32) tile_cand_kernel(KernelArgs A, TileArgs T,
         if (it >= total) break;
         const int2 en = sel[it];
         const TilePair tp = list[en.x];
-        TileView v = tile_view(A, T, tp, A.metas[tp.slot].thr_i, smem);
+        TileView v = tile_view(A, T, tp, -1, A.metas[tp.slot].thr_i, smem);
         const int b = en.y / v.ntiles, j = en.y % v.ntiles;
-        v.load_h<true>(b, j, CandSink{A.cands + A.cand_base[tp.slot], A.cand_cap[tp.slot], A.n_cand + tp.slot},
+        v.compute<true>(b, j, CandSink{A.cands + A.cand_base[tp.slot], A.cand_cap[tp.slot], A.n_cand + tp.slot},
                        v.lq - 1, b * kBandRows + kBandRows - 1);
     }
 }
