@@ -193,10 +193,18 @@ struct DevBuf {
     T* as() const { return (T*)p; }
 };
 
+// An array inside another buffer.
+struct DevView {
+    void* p = nullptr;
+    template <typename T>
+    T* as() const { return (T*)p; }
+};
+
+// A sequence set on the host, page-locked: the device copies are taken from here.
 struct HostSeqs {
-    std::vector<uint8_t> raw;
-    std::vector<int64_t> off;
-    std::vector<int32_t> key;
+    HostBuf<uint8_t> raw;
+    HostBuf<int64_t> off;
+    HostBuf<int32_t> key;
     int32_t n = 0;
     bool set = false;
 };
@@ -235,10 +243,14 @@ struct pw_engine {
     // sequences
     HostSeqs Q, T;
     // device buffers
-    DevBuf q_codes, q_code_off, q_raw, q_raw_off, q_len, q_key, q_order;
-    DevBuf t_codes, t_code_off, t_raw, t_raw_off, t_len, t_key;
-    DevBuf q_res, t_ccodes, t_order, cmat_t8, cmat_tf;  // the other orientation's encodings
-    DevBuf cmat_i8, cmat_f, pair_max, items, items_alt, counter, bnd_pool, q_order2;
+    // per sequence set: residues and encodings, the small arrays in one block
+    // (one copy a set), the alphabet's tables in another
+    DevBuf q_block, q_tables, q_raw_buf, q_codes, q_res;
+    DevBuf t_block, t_tables, t_raw_buf, t_codes, t_ccodes;
+    DevView q_code_off, q_raw, q_raw_off, q_len, q_key, q_order, cmat_i8, cmat_f;
+    DevView t_code_off, t_raw, t_raw_off, t_len, t_key, t_order, cmat_t8, cmat_tf;
+    DevBuf seen_flags;  // residue values present in a set
+    DevBuf pair_max, items, items_alt, counter, bnd_pool, q_order2;
     DevBuf band_pairs, band_entries, band_prog, band_max, band_ring, band_out;  // band sweep (pw_band.cuh)
     DevBuf tile_ck, tile_marks, tile_pairs, slot_tile;                        // tile form (pw_tiles.cuh)
     DevBuf tile_pairs_alt, tile_sel, tile_cnt, tile_acc, tile_scratch, tile_ops;
@@ -261,8 +273,8 @@ struct pw_engine {
     DevBuf acc_hits, acc_ops, fk_a, fk_b, fk_c, fk_t, fk_g, fi_a, fi_b, f_len, f_soff, f_out, f_str;
     HostBuf<int64_t> h_sel;
     HostBuf<int32_t> h_ptq, h_p2order;  // phase-2 pair lists (kept across calls: no page faults, no zero fill)
-    HostBuf<uint8_t> h_qc, h_qres;      // query encodings staged for upload (page-locked, kept across calls)
-    HostBuf<uint8_t> h_stage;           // page-locked staging of the other per-set uploads (Staged)
+    HostBuf<uint8_t> h_stage[4];        // page-locked staging of the sets' blocks and tables (Staged)
+    HostBuf<uint8_t> h_seen;
     int64_t free_mem = 0;    // free device memory plus this engine's kept wave buffers, as last queried
     double free_mem_t = -1;  // wall_ms() of that query
     DevBuf chain_info, chain_prog, chain_max, chain_ring_off, chain_ring, chain_abort, p1_items, p1_grid;
@@ -428,10 +440,11 @@ extern "C" int pw_set_scoring(pw_engine* e, const float* matrix, int dim, int ch
 // The residues as the engine keeps them: ASCII letters upper-cased (the
 // reference upper-cases every sequence before its kernels see it), on host
 // threads.  Returns whether dst already held exactly that.
-static bool copy_upper(std::vector<uint8_t>& dst, const uint8_t* src, int64_t n) {
+static bool copy_upper(HostBuf<uint8_t>& dst, const uint8_t* src, int64_t n, bool* ok) {
     const bool same_size = (int64_t)dst.size() == n;
     std::atomic<bool> differ{!same_size};
-    if (!same_size) dst.resize((size_t)n);
+    *ok = same_size || dst.resize((size_t)n);
+    if (!*ok) return false;
     parallel_for(n, [&](int64_t i0, int64_t i1) {
         uint8_t* d = dst.data();
         bool diff = false;
@@ -460,14 +473,22 @@ static int set_seqs(pw_engine* e, HostSeqs& S, const uint8_t* residues, const in
     if (total > 0 && !residues) return fail(e, PW_ERR_ARG, "residues missing");
     // the same set again (a resident database handed in once more): keep the
     // device copy
-    const bool same_raw = copy_upper(S.raw, residues, total);
+    bool ok = true;
+    const bool same_raw = copy_upper(S.raw, residues, total, &ok);
+    if (!ok) {
+        S.set = false;
+        return fail(e, PW_ERR_NOMEM, "host memory for the sequences");
+    }
     if (S.set && S.n == n && same_raw && S.off.size() == (size_t)(n > 0 ? n + 1 : 1) &&
         (n == 0 || (std::memcmp(S.off.data(), offsets, (size_t)(n + 1) * sizeof(int64_t)) == 0 &&
                     std::memcmp(S.key.data(), id_keys, (size_t)n * sizeof(int32_t)) == 0)))
         return PW_OK;
-    S.off.assign(offsets, offsets + (n > 0 ? n + 1 : 0));
-    if (n == 0) S.off.assign(1, 0);
-    S.key.assign(id_keys, id_keys + n);
+    S.set = false;
+    if (!S.off.resize((size_t)n + 1) || !S.key.resize((size_t)n))
+        return fail(e, PW_ERR_NOMEM, "host memory for the sequences");
+    S.off[0] = 0;
+    if (n > 0) std::memcpy(S.off.data(), offsets, (size_t)(n + 1) * sizeof(int64_t));
+    if (n > 0) std::memcpy(S.key.data(), id_keys, (size_t)n * sizeof(int32_t));
     S.n = n;
     S.set = true;
     (&S == &e->Q ? e->q_gen : e->t_gen)++;
@@ -628,154 +649,206 @@ static cudaError_t download(pw_engine* e, std::vector<HT>& v, const void* src, s
     return cudaStreamSynchronize(e->stream);
 }
 
-// The uploads of one sequence set, gathered into the engine's page-locked
-// staging buffer and copied asynchronously (a pageable source makes every
-// cudaMemcpyAsync a synchronous staged copy of its own); the caller
-// synchronises the stream before the staging buffer is reused.
+// Small arrays gathered into a page-locked staging buffer and copied with one
+// call into one device block; each gets its place in the block.  The staging
+// buffer is not reused before the stream has been synchronised (every pw_align
+// ends so, and a set is prepared at most once in it).
 struct Staged {
     struct Item {
-        DevBuf* dst;
+        DevView* dst;
         const void* src;
         size_t bytes;
     };
     std::vector<Item> items;
+    void add(DevView& v, const void* src, size_t bytes) { items.push_back({&v, src, bytes}); }
     template <typename V>
-    void add(DevBuf& b, const V& v) {
-        items.push_back({&b, v.data(), v.size() * sizeof(v[0])});
-    }
-    cudaError_t run(pw_engine* e) {
+    void add(DevView& v, const V& src) { add(v, src.data(), src.size() * sizeof(src[0])); }
+    cudaError_t run(pw_engine* e, DevBuf& block, HostBuf<uint8_t>& stage) {
         size_t total = 0;
         for (const Item& it : items) total += (it.bytes + 15) & ~(size_t)15;
-        if (!e->h_stage.resize(std::max<size_t>(total, 16))) return cudaErrorMemoryAllocation;
+        total = std::max<size_t>(total, 16);
+        if (!stage.resize(total)) return cudaErrorMemoryAllocation;
+        cudaError_t c = block.reserve(e->stream, total);
+        if (c != cudaSuccess) return c;
         size_t off = 0;
         for (const Item& it : items) {
-            cudaError_t c = it.dst->reserve(e->stream, std::max<size_t>(it.bytes, 16));
-            if (c != cudaSuccess) return c;
-            if (it.bytes) {
-                std::memcpy(e->h_stage.data() + off, it.src, it.bytes);
-                if ((c = copy_h2d(e, it.dst->p, e->h_stage.data() + off, it.bytes)) != cudaSuccess) return c;
-            }
+            if (it.bytes) std::memcpy(stage.data() + off, it.src, it.bytes);
+            it.dst->p = (uint8_t*)block.p + off;
             off += (it.bytes + 15) & ~(size_t)15;
         }
-        return cudaSuccess;
+        return copy_h2d(e, block.p, stage.data(), total);
     }
 };
 
-// The byte values present in data[0, n), ascending (chunks marked on host
-// threads, without branches).  The compact alphabets number them in this
-// order; any numbering gives the same scores.
-static std::vector<int> present_bytes(const uint8_t* data, int64_t n) {
-    std::vector<std::vector<uint8_t>> marks;
-    std::mutex mu;
-    parallel_for(n, [&](int64_t b0, int64_t b1) {
-        std::vector<uint8_t> m(256, 0);
-        for (int64_t k = b0; k < b1; ++k) m[data[k]] = 1;
-        std::lock_guard<std::mutex> g(mu);
-        marks.push_back(std::move(m));
-    }, (int64_t)1 << 20);
+// Residue sets larger than this go to the device straight from their own
+// page-locked array (smaller ones with the set's block, in one copy), and the
+// residue values present are found there.
+constexpr size_t kDirectBytes = (size_t)1 << 18;
+
+// The byte values present in data[0, n), ascending.  The compact alphabets
+// number them in this order; any numbering gives the same scores.
+static std::vector<int> listed_bytes(const uint8_t* seen) {
     std::vector<int> out;
-    for (int c = 0; c < 256; ++c) {
-        bool any = false;
-        for (auto& m : marks) any = any || m[c];
-        if (any) out.push_back(c);
-    }
+    for (int c = 0; c < 256; ++c)
+        if (seen[c]) out.push_back(c);
     return out;
 }
 
-// Builds the device copies of the sequences, the compact query alphabet and the
-// compact substitution matrices.  Targets and queries are prepared separately
-// and cached: a target database stays resident on the device while query sets
-// come and go, and nothing is uploaded again while the sequences and the
-// scoring model are unchanged.
+// One sequence set on the device: residues as given, and the two encodings (the
+// host loops that wrote them, with two copies of the padded set over PCIe, took
+// 18 ms for 500,000 reads and 9 ms for 5.8 Mb of long DNA; 1.9 and 0.4 ms now) --
+// compact codes (codes: the distinct residues numbered, padding coded as one
+// more) and matrix indices (res) -- written by encode_kernel, each sequence
+// 16-byte aligned and padded.  Queries and targets are prepared separately and
+// cached: a target database stays resident on the device while query sets come
+// and go, and nothing is uploaded again while the sequences and the scoring
+// model are unchanged.
+struct SetBuffers {
+    DevBuf *block, *tables, *raw_buf, *codes, *res;
+    DevView *raw, *raw_off, *code_off, *len, *key, *order, *m8, *mf;
+    HostBuf<uint8_t>*stage, *stage_tables;
+    std::vector<int32_t>*host_len, *host_order;
+    int64_t* longest;
+    int* alpha;
+    bool* int8;
+    bool transposed;  // the matrix rows are target residues (its columns query residues)
+    const char* what;
+};
+
+static int prepare_set(pw_engine* e, const HostSeqs& S, const SetBuffers& B, float* maxabs) {
+    const int off = e->char_offset, dim = e->dim, n = S.n;
+    cudaError_t c;
+    const size_t raw_bytes = S.raw.size();
+    const bool direct = raw_bytes > kDirectBytes;
+    // lengths, aligned offsets, whether the records come longest first already
+    std::vector<int32_t>& len = *B.host_len;
+    len.resize((size_t)n);
+    std::vector<int64_t> code_off((size_t)n + 1);
+    int64_t pos = 0, longest = 0;
+    bool sorted = true;
+    for (int32_t i = 0; i < n; ++i) {
+        const int32_t L = (int32_t)(S.off[i + 1] - S.off[i]);
+        sorted = sorted && (i == 0 || L <= len[i - 1]);
+        len[i] = L;
+        longest = std::max<int64_t>(longest, L);
+        code_off[i] = pos;
+        pos += align_up(std::max<int64_t>(L, 1), 16);
+    }
+    code_off[n] = pos;
+    *B.longest = longest;
+    // a stable order by length, longest first
+    std::vector<int32_t>& order = *B.host_order;
+    if (sorted) {
+        order.resize((size_t)n);
+        std::iota(order.begin(), order.end(), 0);
+    } else {
+        std::vector<uint64_t> key((size_t)n);
+        for (int32_t i = 0; i < n; ++i) key[i] = (uint64_t)(longest - len[i]);
+        const std::vector<uint32_t> o = radix_order(std::move(key));
+        order.assign(o.begin(), o.end());
+    }
+    Staged st;
+    st.add(*B.raw_off, S.off);
+    st.add(*B.code_off, code_off);
+    st.add(*B.len, len);
+    st.add(*B.key, S.key);
+    st.add(*B.order, order);
+    if (!direct) st.add(*B.raw, S.raw);
+    if ((c = st.run(e, *B.block, *B.stage)) != cudaSuccess) return cuda_fail(e, c, "upload sequences");
+    // the residue values present
+    uint8_t seen[256] = {};
+    if (direct) {
+        if ((c = B.raw_buf->reserve(e->stream, raw_bytes)) != cudaSuccess ||
+            (c = copy_h2d(e, B.raw_buf->p, S.raw.data(), raw_bytes)) != cudaSuccess ||
+            (c = e->seen_flags.reserve(e->stream, 256)) != cudaSuccess ||
+            (c = cudaMemsetAsync(e->seen_flags.p, 0, 256, e->stream)) != cudaSuccess)
+            return cuda_fail(e, c, "upload sequences");
+        B.raw->p = B.raw_buf->p;
+        const int grid = (int)std::min<int64_t>((int64_t)(raw_bytes + 4095) / 4096, (int64_t)e->sm_count * 8);
+        PW_LAUNCH(present_kernel, grid, 256, 0, e->stream, (const uint8_t*)B.raw_buf->as<uint8_t>(), (int64_t)raw_bytes,
+                  e->seen_flags.as<uint8_t>());
+        e->launches++;
+        if (!e->h_seen.resize(256)) return fail(e, PW_ERR_NOMEM, "host memory for the sequences");
+        if ((c = cudaGetLastError()) != cudaSuccess ||
+            (c = copy_d2h(e, e->h_seen.data(), e->seen_flags.p, 256)) != cudaSuccess ||
+            (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
+            return cuda_fail(e, c, "residues present");
+        std::memcpy(seen, e->h_seen.data(), 256);
+    } else {
+        for (size_t k = 0; k < raw_bytes; ++k) seen[S.raw[k]] = 1;
+    }
+    const std::vector<int> alphabet = listed_bytes(seen);
+    // residues must index the matrix (default_main.cu:234 reads matrix[c - offset]);
+    // the first invalid one of the input is reported
+    {
+        int64_t bad_at = INT64_MAX;
+        int bad = -1;
+        for (int v : alphabet)
+            if (v == 0 || v < off || v >= off + dim) {
+                const int64_t at =
+                    (int64_t)(std::find(S.raw.data(), S.raw.data() + raw_bytes, (uint8_t)v) - S.raw.data());
+                if (at < bad_at) {
+                    bad_at = at;
+                    bad = v;
+                }
+            }
+        if (bad >= 0)
+            return fail(e, PW_ERR_ARG,
+                        std::string(B.what) + " residue outside the scoring matrix: code " + std::to_string(bad));
+    }
+    const int alpha = (int)alphabet.size();
+    if (!B.transposed && alpha > 250) return fail(e, PW_ERR_ARG, "too many distinct query residues");
+    *B.alpha = alpha;
+    // the matrix compacted to the residues present: rows of this set's
+    // residues, the padding row last
+    std::vector<uint8_t> map(256, (uint8_t)alpha);
+    for (int a = 0; a < alpha; ++a) map[alphabet[a]] = (uint8_t)a;
+    std::vector<int8_t> m8((size_t)(alpha + 1) * dim, (int8_t)-128);
+    std::vector<float> mf((size_t)(alpha + 1) * dim, -1.0e30f);
+    bool int8 = alpha <= 250;
+    for (int a = 0; a < alpha; ++a)
+        for (int j = 0; j < dim; ++j) {
+            const int r = alphabet[a] - off;
+            const float v = B.transposed ? e->matrix[(size_t)j * dim + r] : e->matrix[(size_t)r * dim + j];
+            if (std::floor(v) != v || v < -127.0f || v > 127.0f) int8 = false;
+            if (maxabs) *maxabs = std::max(*maxabs, std::fabs(v));
+            mf[(size_t)a * dim + j] = v;
+        }
+    for (int a = 0; a < alpha; ++a)
+        for (int j = 0; j < dim; ++j) m8[(size_t)a * dim + j] = int8 ? (int8_t)mf[(size_t)a * dim + j] : 0;
+    *B.int8 = int8;
+    DevView d_map;
+    Staged tb;
+    tb.add(d_map, map);
+    tb.add(*B.m8, m8);
+    tb.add(*B.mf, mf);
+    const int64_t chunks = std::max<int64_t>(pos / 16, 1);
+    if ((c = tb.run(e, *B.tables, *B.stage_tables)) != cudaSuccess ||
+        (c = B.codes->reserve(e->stream, (size_t)chunks * 16)) != cudaSuccess ||
+        (c = B.res->reserve(e->stream, (size_t)chunks * 16)) != cudaSuccess)
+        return cuda_fail(e, c, "upload residue tables");
+    PW_LAUNCH(encode_kernel, (int)((chunks + 255) / 256), 256, 0, e->stream, (const uint8_t*)B.raw->as<uint8_t>(),
+              (const int64_t*)B.raw_off->as<int64_t>(), (const int64_t*)B.code_off->as<int64_t>(), n,
+              (const uint8_t*)d_map.as<uint8_t>(), alpha, off, chunks, B.codes->as<uint4>(), B.res->as<uint4>());
+    e->launches++;
+    if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "encode sequences");
+    return PW_OK;
+}
+
 static int prepare_targets(pw_engine* e) {
     if (e->prep_t[0] == e->t_gen && e->prep_t[1] == e->s_gen) {
         e->reuse |= PW_REUSE_TARGETS;
         return PW_OK;
     }
-    const HostSeqs& T = e->T;
-    const int off = e->char_offset, dim = e->dim;
     Prepared& pr = e->pr;
-    // the byte values present (host threads)
-    const std::vector<int> present = present_bytes(T.raw.data(), (int64_t)T.raw.size());
-    {
-        // the first invalid residue of the input is reported
-        int64_t bad_at = INT64_MAX;
-        int bad = -1;
-        for (int c : present)
-            if (c == 0 || c < off || c >= off + dim) {
-                const int64_t at = (int64_t)(std::find(T.raw.begin(), T.raw.end(), (uint8_t)c) - T.raw.begin());
-                if (at < bad_at) {
-                    bad_at = at;
-                    bad = c;
-                }
-            }
-        if (bad >= 0)
-            return fail(e, PW_ERR_ARG, "target residue outside the scoring matrix: code " + std::to_string(bad));
-    }
-    pr.tlen.assign(T.n, 0);
-    pr.maxlt = 0;
-    for (int32_t i = 0; i < T.n; ++i)
-        pr.maxlt = std::max<int64_t>(pr.maxlt, pr.tlen[i] = (int32_t)(T.off[i + 1] - T.off[i]));
-    // targets: matrix residue index, each sequence 16-byte aligned
-    std::vector<int64_t> tco(T.n + 1, 0);
-    int64_t pos = 0;
-    for (int32_t i = 0; i < T.n; ++i) {
-        tco[i] = pos;
-        pos += align_up(std::max<int64_t>(pr.tlen[i], 1), 16);
-    }
-    tco[T.n] = pos;
-    // the transposed orientation: targets on the lanes in a compact target
-    // alphabet, with the matrix transposed to [target residue][query residue]
-    int tmap[256];
-    for (int i = 0; i < 256; ++i) tmap[i] = -1;
-    std::vector<int> talpha;
-    for (int c : present) {
-        tmap[c] = (int)talpha.size();
-        talpha.push_back(c);
-    }
-    pr.alpha_t = (int)talpha.size();
-    std::vector<uint8_t> tc((size_t)std::max<int64_t>(pos, 16), 0);
-    std::vector<uint8_t> tcc(tc.size(), (uint8_t)pr.alpha_t);
-    parallel_for(T.n, [&](int64_t i0, int64_t i1) {
-        for (int64_t i = i0; i < i1; ++i) {
-            const uint8_t* r = T.raw.data() + T.off[i];
-            for (int32_t k = 0; k < pr.tlen[i]; ++k) {
-                tc[tco[i] + k] = (uint8_t)(r[k] - off);
-                tcc[tco[i] + k] = (uint8_t)tmap[r[k]];
-            }
-        }
-    }, (int64_t)64);
-    {
-        std::vector<uint64_t> key((size_t)T.n);
-        for (int32_t i = 0; i < T.n; ++i) key[i] = (uint64_t)(pr.maxlt - pr.tlen[i]);
-        const std::vector<uint32_t> o = radix_order(std::move(key));
-        pr.order_t.assign(o.begin(), o.end());
-    }
-    std::vector<int8_t> cmt8((size_t)(pr.alpha_t + 1) * dim, (int8_t)-128);
-    std::vector<float> cmtf((size_t)(pr.alpha_t + 1) * dim, -1.0e30f);
-    bool t_int8 = pr.alpha_t <= 250;
-    for (int b = 0; b < pr.alpha_t; ++b)
-        for (int j = 0; j < dim; ++j) {
-            const float v = e->matrix[(size_t)j * dim + (talpha[b] - off)];
-            if (std::floor(v) != v || v < -127.0f || v > 127.0f) t_int8 = false;
-            cmt8[(size_t)b * dim + j] = (int8_t)(t_int8 ? v : 0);
-            cmtf[(size_t)b * dim + j] = v;
-        }
-    pr.t_int8 = t_int8;
-    cudaError_t c;
-    Staged st;
-    st.add(e->t_codes, tc);
-    st.add(e->t_code_off, tco);
-    st.add(e->t_raw, T.raw);
-    st.add(e->t_raw_off, T.off);
-    st.add(e->t_len, pr.tlen);
-    st.add(e->t_key, T.key);
-    st.add(e->t_ccodes, tcc);
-    st.add(e->t_order, pr.order_t);
-    st.add(e->cmat_t8, cmt8);
-    st.add(e->cmat_tf, cmtf);
-    if ((c = st.run(e)) != cudaSuccess || (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
-        return cuda_fail(e, c, "upload targets");
+    e->prep_t[0] = 0;
+    // t_codes: matrix indices (targets as strips); t_ccodes: compact codes (on
+    // the lanes), with the matrix transposed to [target residue][query residue]
+    const SetBuffers B{&e->t_block, &e->t_tables, &e->t_raw_buf, &e->t_ccodes, &e->t_codes, &e->t_raw, &e->t_raw_off,
+                       &e->t_code_off, &e->t_len, &e->t_key, &e->t_order, &e->cmat_t8, &e->cmat_tf, &e->h_stage[0],
+                       &e->h_stage[1], &pr.tlen, &pr.order_t, &pr.maxlt, &pr.alpha_t, &pr.t_int8, true, "target"};
+    const int rc = prepare_set(e, e->T, B, nullptr);
+    if (rc != PW_OK) return rc;
     e->prep_t[0] = e->t_gen;
     e->prep_t[1] = e->s_gen;
     return PW_OK;
@@ -786,116 +859,15 @@ static int prepare_queries(pw_engine* e) {
         e->reuse |= PW_REUSE_QUERIES;
         return PW_OK;
     }
-    const HostSeqs& Q = e->Q;
-    const int off = e->char_offset, dim = e->dim;
     Prepared& pr = e->pr;
-    // residues must index the matrix (default_main.cu:234 reads matrix[c - offset];
-    // the first invalid one of the input is reported); the compact alphabet
-    // numbers the residues present in byte order
-    int map[256];
-    for (int i = 0; i < 256; ++i) map[i] = -1;
-    std::vector<int> alphabet;
-    const std::vector<int> present = present_bytes(Q.raw.data(), (int64_t)Q.raw.size());
-    {
-        int64_t bad_at = INT64_MAX;
-        int bad = -1;
-        for (int c : present)
-            if (c == 0 || c < off || c >= off + dim) {
-                const int64_t at = (int64_t)(std::find(Q.raw.begin(), Q.raw.end(), (uint8_t)c) - Q.raw.begin());
-                if (at < bad_at) {
-                    bad_at = at;
-                    bad = c;
-                }
-            }
-        if (bad >= 0)
-            return fail(e, PW_ERR_ARG, "query residue outside the scoring matrix: code " + std::to_string(bad));
-    }
-    for (int c : present) {
-        map[c] = (int)alphabet.size();
-        alphabet.push_back(c);
-    }
-    if (alphabet.size() > 250) return fail(e, PW_ERR_ARG, "too many distinct query residues");
-    pr.alpha = (int)alphabet.size();
-    const int alpha1 = pr.alpha + 1;
-    // scores of the used rows: all integers in the int8 range?
-    bool q_int8 = true;
-    float maxabs = 0.0f;
-    for (int a = 0; a < pr.alpha; ++a)
-        for (int j = 0; j < dim; ++j) {
-            const float v = e->matrix[(size_t)(alphabet[a] - off) * dim + j];
-            if (std::floor(v) != v || v < -127.0f || v > 127.0f) q_int8 = false;
-            maxabs = std::max(maxabs, std::fabs(v));
-        }
-    pr.q_int8 = q_int8;
-    pr.maxabs = maxabs;
-    pr.qlen.assign(Q.n, 0);
-    pr.maxlq = 0;
-    for (int32_t i = 0; i < Q.n; ++i)
-        pr.maxlq = std::max<int64_t>(pr.maxlq, pr.qlen[i] = (int32_t)(Q.off[i + 1] - Q.off[i]));
-    std::vector<int8_t> cm8((size_t)alpha1 * dim, (int8_t)-128);
-    std::vector<float> cmf((size_t)alpha1 * dim, -1.0e30f);
-    for (int a = 0; a < pr.alpha; ++a)
-        for (int j = 0; j < dim; ++j) {
-            const float v = e->matrix[(size_t)(alphabet[a] - off) * dim + j];
-            cmf[(size_t)a * dim + j] = v;
-            cm8[(size_t)a * dim + j] = q_int8 ? (int8_t)v : 0;
-        }
-    // queries: compact codes, each sequence 16-byte aligned and padded to a
-    // multiple of 4 with the pad code
-    std::vector<int64_t> qco(Q.n + 1, 0);
-    int64_t pos = 0;
-    for (int32_t i = 0; i < Q.n; ++i) {
-        qco[i] = pos;
-        pos += align_up(std::max<int64_t>(pr.qlen[i], 1), 16);
-    }
-    qco[Q.n] = pos;
-    // the transposed orientation: queries as strips (matrix residue indices)
-    HostBuf<uint8_t>& qc = e->h_qc;
-    HostBuf<uint8_t>& qres = e->h_qres;
-    if (!qc.resize((size_t)std::max<int64_t>(pos, 16)) || !qres.resize((size_t)std::max<int64_t>(pos, 16)))
-        return fail(e, PW_ERR_NOMEM, "host memory for the query encodings");
-    parallel_for(Q.n, [&](int64_t i0, int64_t i1) {
-        for (int64_t i = i0; i < i1; ++i) {
-            const uint8_t* r = Q.raw.data() + Q.off[i];
-            uint8_t* d = qc.data() + qco[i];
-            uint8_t* d2 = qres.data() + qco[i];
-            const int64_t L = pr.qlen[i], end = qco[i + 1] - qco[i];
-            for (int64_t k = 0; k < L; ++k) {
-                d[k] = (uint8_t)map[r[k]];
-                d2[k] = (uint8_t)(r[k] - off);
-            }
-            for (int64_t k = L; k < end; ++k) {
-                d[k] = (uint8_t)pr.alpha;
-                d2[k] = 0;
-            }
-        }
-    }, (int64_t)1 << 14);
-    for (size_t k = (size_t)pos; k < qc.size(); ++k) {
-        qc.data()[k] = (uint8_t)pr.alpha;
-        qres.data()[k] = 0;
-    }
-    // a stable sort by length, longest first
-    {
-        std::vector<uint64_t> key((size_t)Q.n);
-        for (int32_t i = 0; i < Q.n; ++i) key[i] = (uint64_t)(pr.maxlq - pr.qlen[i]);
-        const std::vector<uint32_t> o = radix_order(std::move(key));
-        pr.order.assign(o.begin(), o.end());
-    }
-    cudaError_t c;
-    // the encodings are page-locked already; the rest goes through the staging buffer
-    if ((c = upload(e, e->q_codes, qc)) != cudaSuccess || (c = upload(e, e->q_res, qres)) != cudaSuccess)
-        return cuda_fail(e, c, "upload query encodings");
-    Staged st;
-    st.add(e->q_code_off, qco);
-    st.add(e->q_raw, Q.raw);
-    st.add(e->q_raw_off, Q.off);
-    st.add(e->q_len, pr.qlen);
-    st.add(e->q_key, Q.key);
-    st.add(e->q_order, pr.order);
-    st.add(e->cmat_i8, cm8);
-    st.add(e->cmat_f, cmf);
-    if ((c = st.run(e)) != cudaSuccess || (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
-        return cuda_fail(e, c, "upload queries");
+    e->prep_q[0] = 0;
+    pr.maxabs = 0.0f;
+    // q_codes: compact codes (on the lanes); q_res: matrix indices (queries as strips)
+    const SetBuffers B{&e->q_block, &e->q_tables, &e->q_raw_buf, &e->q_codes, &e->q_res, &e->q_raw, &e->q_raw_off,
+                       &e->q_code_off, &e->q_len, &e->q_key, &e->q_order, &e->cmat_i8, &e->cmat_f, &e->h_stage[2],
+                       &e->h_stage[3], &pr.qlen, &pr.order, &pr.maxlq, &pr.alpha, &pr.q_int8, false, "query"};
+    const int rc = prepare_set(e, e->Q, B, &pr.maxabs);
+    if (rc != PW_OK) return rc;
     e->prep_q[0] = e->q_gen;
     e->prep_q[1] = e->s_gen;
     return PW_OK;

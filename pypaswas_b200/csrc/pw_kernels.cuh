@@ -1041,6 +1041,58 @@ __global__ void int_peak16_kernel(int iters, int seed, int* sink) {
     if (r == 0x7fffffffu) sink[0] = (int)r;
 }
 
+// Byte values present in data[0, n): flags[value] = 1 (flags start at 0).
+__global__ void present_kernel(const uint8_t* data, int64_t n, uint8_t* flags) {
+    __shared__ uint8_t seen[256];
+    seen[threadIdx.x] = 0;  // 256 threads
+    __syncthreads();
+    const int64_t words = n / 16, stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t i = t; i < words; i += stride) {
+        const uint4 v = __ldg((const uint4*)data + i);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 16; ++k) seen[(w[k / 4] >> (8 * (k % 4))) & 0xff] = 1;
+    }
+    for (int64_t i = words * 16 + t; i < n; i += stride) seen[data[i]] = 1;
+    __syncthreads();
+    if (seen[threadIdx.x]) flags[threadIdx.x] = 1;
+}
+
+// The two encodings of a sequence set: compact codes (map; pad past a
+// sequence's end) and matrix indices (residue - char_off; 0 past its end).  One
+// thread per 16 bytes of the aligned layout, whose sequence it finds by
+// bisection of the n aligned offsets.
+__global__ void encode_kernel(const uint8_t* raw, const int64_t* raw_off, const int64_t* code_off, int n,
+                              const uint8_t* map, int pad, int char_off, int64_t chunks, uint4* codes, uint4* res) {
+    __shared__ uint8_t m[256];
+    m[threadIdx.x] = map[threadIdx.x];  // 256 threads
+    __syncthreads();
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= chunks) return;
+    const int64_t at = c * 16;
+    int lo = 0, hi = n;  // code_off[lo] <= at < code_off[hi]
+    while (hi - lo > 1) {
+        const int mid = lo + (hi - lo) / 2;
+        if (code_off[mid] <= at)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    const int64_t k0 = at - code_off[lo], len = raw_off[lo + 1] - raw_off[lo];
+    const uint8_t* r = raw + raw_off[lo] + k0;
+    const int left = (int)(len - k0 < 16 ? len - k0 : 16);  // residues in this chunk (<= 0: none)
+    uint32_t a[4] = {0u, 0u, 0u, 0u}, b[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const uint32_t v = k < left ? r[k] : 0u;
+        a[k / 4] |= (uint32_t)(k < left ? m[v] : (uint8_t)pad) << (8 * (k % 4));
+        b[k / 4] |= (k < left ? (v - (uint32_t)char_off) & 0xffu : 0u) << (8 * (k % 4));
+    }
+    codes[c] = make_uint4(a[0], a[1], a[2], a[3]);
+    res[c] = make_uint4(b[0], b[1], b[2], b[3]);
+}
+
 // Passing pairs per query (target-major pair indices k = t * nq + sp from the
 // pruning selection; pairs of targets marked in skip are left out).
 __global__ void query_count_kernel(const int64_t* sel, int64_t n, int nq, const int32_t* q_order,
