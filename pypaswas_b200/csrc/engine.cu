@@ -34,6 +34,7 @@
 #include "score16_variants.h"
 #include "pw_band.cuh"
 #include "pw_band_ck.cuh"
+#include "pw_band_affine.cuh"
 #include "pw_tiles.cuh"
 #include "pw_plan.h"
 #include "pw_finish.cuh"
@@ -85,11 +86,14 @@ struct HostBuf {
         p = nullptr;
         n = cap = 0;
     }
-    bool resize(size_t m) {  // contents are not kept
+    // Contents are not kept.  Room for a quarter more: page-locking anew (and
+    // unlocking the old pages) takes tens of milliseconds, so slightly larger
+    // calls reuse it.  Arrays under `lock_from` bytes stay in ordinary memory.
+    bool resize(size_t m, size_t lock_from = 0) {
         if (m > cap) {
             release();
-            const size_t want = std::max<size_t>(m, 1);
-            pinned = cudaMallocHost((void**)&p, want * sizeof(T)) == cudaSuccess;
+            const size_t want = std::max<size_t>(m + m / 4, 1);
+            pinned = want * sizeof(T) >= lock_from && cudaMallocHost((void**)&p, want * sizeof(T)) == cudaSuccess;
             if (!pinned) {
                 cudaGetLastError();
                 p = (T*)malloc(want * sizeof(T));
@@ -200,11 +204,16 @@ struct DevView {
     T* as() const { return (T*)p; }
 };
 
-// A sequence set on the host, page-locked: the device copies are taken from here.
+// Residue sets larger than this go to the device straight from their own
+// page-locked array (smaller ones with the set's block, in one copy), and the
+// residue values present are found there.
+constexpr size_t kDirectBytes = (size_t)1 << 18;
+
+// A sequence set on the host.
 struct HostSeqs {
     HostBuf<uint8_t> raw;
-    HostBuf<int64_t> off;
-    HostBuf<int32_t> key;
+    std::vector<int64_t> off;
+    std::vector<int32_t> key;
     int32_t n = 0;
     bool set = false;
 };
@@ -443,7 +452,7 @@ extern "C" int pw_set_scoring(pw_engine* e, const float* matrix, int dim, int ch
 static bool copy_upper(HostBuf<uint8_t>& dst, const uint8_t* src, int64_t n, bool* ok) {
     const bool same_size = (int64_t)dst.size() == n;
     std::atomic<bool> differ{!same_size};
-    *ok = same_size || dst.resize((size_t)n);
+    *ok = same_size || dst.resize((size_t)n, kDirectBytes);
     if (!*ok) return false;
     parallel_for(n, [&](int64_t i0, int64_t i1) {
         uint8_t* d = dst.data();
@@ -474,6 +483,7 @@ static int set_seqs(pw_engine* e, HostSeqs& S, const uint8_t* residues, const in
     // the same set again (a resident database handed in once more): keep the
     // device copy
     bool ok = true;
+    if (cudaSetDevice(e->device) != cudaSuccess) return fail(e, PW_ERR_DEVICE, "cudaSetDevice failed");
     const bool same_raw = copy_upper(S.raw, residues, total, &ok);
     if (!ok) {
         S.set = false;
@@ -483,12 +493,9 @@ static int set_seqs(pw_engine* e, HostSeqs& S, const uint8_t* residues, const in
         (n == 0 || (std::memcmp(S.off.data(), offsets, (size_t)(n + 1) * sizeof(int64_t)) == 0 &&
                     std::memcmp(S.key.data(), id_keys, (size_t)n * sizeof(int32_t)) == 0)))
         return PW_OK;
-    S.set = false;
-    if (!S.off.resize((size_t)n + 1) || !S.key.resize((size_t)n))
-        return fail(e, PW_ERR_NOMEM, "host memory for the sequences");
-    S.off[0] = 0;
-    if (n > 0) std::memcpy(S.off.data(), offsets, (size_t)(n + 1) * sizeof(int64_t));
-    if (n > 0) std::memcpy(S.key.data(), id_keys, (size_t)n * sizeof(int32_t));
+    S.off.assign(offsets, offsets + (n > 0 ? n + 1 : 0));
+    if (n == 0) S.off.assign(1, 0);
+    S.key.assign(id_keys, id_keys + n);
     S.n = n;
     S.set = true;
     (&S == &e->Q ? e->q_gen : e->t_gen)++;
@@ -679,11 +686,6 @@ struct Staged {
         return copy_h2d(e, block.p, stage.data(), total);
     }
 };
-
-// Residue sets larger than this go to the device straight from their own
-// page-locked array (smaller ones with the set's block, in one copy), and the
-// residue values present are found there.
-constexpr size_t kDirectBytes = (size_t)1 << 18;
 
 // The byte values present in data[0, n), ascending.  The compact alphabets
 // number them in this order; any numbering gives the same scores.
@@ -1581,10 +1583,10 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
                           int* n_launch) {
     if (pairs.empty()) return PW_OK;
     const int prof_bytes = (int)align_up((int64_t)kWarp * (A.P.alpha + 1) * kWarpRows, 16);
-    const int smem = 4 * prof_bytes;
-    auto kern = band_kernel<false, DIRS>;
+    const int smem = 4 * (e->affine ? band_affine_warp_smem(A.P.alpha + 1) : prof_bytes);
+    auto kern = band_kernel<DIRS>;
     if constexpr (DIRS < 2)
-        if (e->affine) kern = band_kernel<true, DIRS>;
+        if (e->affine) kern = band_affine_kernel<DIRS>;
     cudaError_t c;
     if (smem > 48 * 1024 &&
         (c = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
@@ -1600,7 +1602,8 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
     std::vector<int64_t> steps(pairs.size());
     for (size_t k = 0; k < pairs.size(); ++k) {
         pairs[k].nbands = std::max(1, pairs[k].nbands);
-        steps[k] = (int64_t)e->pr.qlen[pairs[k].q] + kWarp - 1;
+        const int lq = e->pr.qlen[pairs[k].q];
+        steps[k] = (int64_t)(e->affine ? affine_blocks(lq) : lq) + kWarp - 1;
     }
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
         return steps[x] * pairs[x].nbands > steps[y] * pairs[y].nbands;
@@ -1615,10 +1618,11 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
         xm[k] = steps[order[k]];
         if constexpr (DIRS < 3) {
             sorted[k].ring_off = ring_elems;
-            if (sorted[k].nbands > 1) ring_elems += 2 * (int64_t)e->pr.qlen[sorted[k].q];
+            const int lq = e->pr.qlen[sorted[k].q];
+            if (sorted[k].nbands > 1) ring_elems += 2 * (int64_t)(e->affine ? affine_blocks(lq) : lq);
         }
     }
-    std::vector<int4> entries = band_queue(nstr, xm, warps, kBandLead);
+    std::vector<int4> entries = band_queue(nstr, xm, warps, e->affine ? kAffLead : kBandLead);
     const size_t n = entries.size();
     if (e->tune[PW_TUNE_STALL_TEST]) {
         // one band below another waits on the spare flag (index n) instead
@@ -1638,7 +1642,9 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
         return cuda_fail(e, c, "alloc band state");
     if ((c = cudaMemsetAsync(e->band_prog.p, 0, (n + 1) * sizeof(int), e->stream)) != cudaSuccess ||
         (c = cudaMemsetAsync(e->chain_abort.p, 0, sizeof(int), e->stream)) != cudaSuccess ||
-        (c = cudaMemsetAsync(e->counter.as<int>() + kNumClasses, 0, sizeof(int), e->stream)) != cudaSuccess)
+        (c = cudaMemsetAsync(e->counter.as<int>() + kNumClasses, 0, sizeof(int), e->stream)) != cudaSuccess ||
+        (e->affine && ring_elems > 0 &&  // no word shows a band's epoch yet
+         (c = cudaMemsetAsync(e->band_ring.p, 0, (size_t)ring_elems * sizeof(int4), e->stream)) != cudaSuccess))
         return cuda_fail(e, c, "reset band state");
     BandArgs B;
     memset(&B, 0, sizeof(B));
@@ -2436,7 +2442,7 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         w.first = wp.first;
         w.lanes = 1;
         w.xmax = qlen[wp.first];
-        w.orient = 2;
+        w.orient = e->affine ? 3 : 2;  // PairView::layout
         w.S = kWarpRows;
         items2.push_back(w);
         cls2.push_back(kNumClasses);  // marks a warp item
@@ -2444,7 +2450,8 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         // (the score sweep's checkpoints, when it kept them, are not the wave's)
         bytes2.push_back(tile_form ? (p1ck ? 0 : tile_checkpoint_ints(qlen[wp.first], tlen[wp.second]) * 4) +
                                          align_up(((int64_t)qlen[wp.first] * tlen[wp.second] + 31) / 32 * 4, 16)
-                                   : align_up(warp_code_bytes(qlen[wp.first], tlen[wp.second], hstore), 16));
+                                   : align_up(e->affine ? affine_code_bytes(qlen[wp.first], tlen[wp.second])
+                                                         : warp_code_bytes(qlen[wp.first], tlen[wp.second], hstore), 16));
         qmax_warp = std::max(qmax_warp, qlen[wp.first]);
     }
     ht.mark("phase-2 work items");

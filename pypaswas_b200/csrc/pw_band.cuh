@@ -1,4 +1,5 @@
-// pw_band.cuh -- one pair per warp, its 256-row bands chained across warps.
+// pw_band.cuh -- one pair per warp, its 256-row bands chained across warps
+// (linear gap; pw_band_affine.cuh is the affine sweep).
 //
 // The 32 lanes of a warp share one (query, target) pair: lane l owns target
 // rows [y0 + 8l, y0 + 8l + 8) of a 256-row band and the warp walks the query
@@ -26,15 +27,15 @@
 // pair's candidate list, exactly as the strip sweep computes them; 4-bit cell
 // codes are stored [band][step][lane][8 rows] (warp_layout_offset), one 4-byte
 // word per lane and step: a warp stores 128 contiguous bytes.
-// DIRS = 2 (linear gap): the same sweep storing each cell's 16-bit H at the
+// DIRS = 2: the same sweep storing each cell's 16-bit H at the
 // same positions (16 bytes per lane and step, 512 contiguous bytes a warp) and
 // the candidate list; codes are derived from H on read (PairView::code).
-// DIRS = 3 (linear gap): the checkpoint sweep of the tile form (pw_tiles.cuh):
+// DIRS = 3: the checkpoint sweep of the tile form (pw_tiles.cuh):
 // the candidate list as DIRS 1 finds it, no cell codes; instead every band's
 // bottom row is kept (in place of the two-row ring) and every lane stores its
 // 8 rows' H at the last column of each kTileW-column tile, from which any
 // 256 x kTileW tile's codes are recomputed later.
-// The score sweep of listed pairs (linear gap) keeps the tile form's
+// The score sweep of listed pairs keeps the tile form's
 // checkpoints and tile maxima itself, in a kernel of its own (pw_band_ck.cuh).
 #pragma once
 #include "pw_kernels.cuh"
@@ -55,6 +56,11 @@ __host__ __device__ __forceinline__ int64_t warp_code_bytes(int lq, int lt, bool
     const int64_t bands = lt > 0 ? (lt + kBandRows - 1) / kBandRows : 1;
     const int64_t cells = bands * ((int64_t)lq + kWarp - 1) * kWarp * kWarpRows;
     return hstore ? cells * 2 : cells / 2;
+}
+// ... and of the codes of the affine sweep (affine_layout_offset).
+__host__ __device__ __forceinline__ int64_t affine_code_bytes(int lq, int lt) {
+    const int64_t bands = lt > 0 ? (lt + kBandRows - 1) / kBandRows : 1;
+    return bands * ((int64_t)((lq + 1) / 2) + kWarp - 1) * kWarp * kWarpRows;
 }
 
 // Tile form: a pair's checkpoints are the bottom rows of its bands but the
@@ -78,7 +84,7 @@ struct BandPair {
     int32_t q, t;        // query / target index (reference orientation)
     int32_t nbands;
     int32_t meta_item;   // DIRS: value for PairMeta.item (the pair's work item in the wave)
-    int64_t ring_off;    // int4 offset of the pair's two boundary rows (2 x lq)
+    int64_t ring_off;    // int4 offset of the pair's two boundary rows (2 x lq; affine: 2 x affine_blocks)
     int64_t dir_base;    // DIRS 1, 2: byte offset of the pair's cell codes; 3: int offset of its checkpoints
                          // (rows, then columns)
     int64_t slot;        // DIRS: pair slot (metas, candidates); score sweep: pair_max index
@@ -124,9 +130,8 @@ __device__ __forceinline__ int prof_score(uint2 pw, int r) {
     }
 }
 
-template <bool AFFINE, int DIRS>
-__global__ void __launch_bounds__(128, AFFINE ? 5 : 8) band_kernel(KernelArgs A, BandArgs B) {
-    static_assert(DIRS < 2 || !AFFINE, "H store and tile form: linear gap only");
+template <int DIRS>
+__global__ void __launch_bounds__(128, 8) band_kernel(KernelArgs A, BandArgs B) {
     constexpr bool MAXIMA = DIRS == 0;  // pair maxima, no trace
     constexpr bool CKPT = DIRS == 3;    // tile-form checkpoints
     extern __shared__ __align__(16) unsigned char smem[];
@@ -135,8 +140,7 @@ __global__ void __launch_bounds__(128, AFFINE ? 5 : 8) band_kernel(KernelArgs A,
     const int alpha1 = A.P.alpha + 1;
     const int prof_bytes = ((kWarp * alpha1 * kWarpRows) + 15) & ~15;
     uint2* prof = (uint2*)(smem + wib * prof_bytes);  // [lane][alpha1] -> 8 int8 scores of that lane's rows
-    const int gap = A.P.gap_i, ext = A.P.ext_i, ge = A.P.ge_i;
-    const int neg = kNeg;
+    const int gap = A.P.gap_i;
 
     for (;;) {
         int it = 0;
@@ -217,30 +221,21 @@ __global__ void __launch_bounds__(128, AFFINE ? 5 : 8) band_kernel(KernelArgs A,
         const int ymine = yb + lane * kWarpRows;
         const bool ypos = ymine > 0;       // this lane's first row is not row 0
         const int rows_left = lt - ymine;  // rows r < rows_left of this lane lie inside the target
-        int Hl[kWarpRows], Ml[kWarpRows], Jl[kWarpRows], Bl[kWarpRows];
+        int Hl[kWarpRows];
 #pragma unroll
-        for (int r = 0; r < kWarpRows; ++r) {
-            Hl[r] = 0;
-            Ml[r] = 0;
-            Jl[r] = neg;
-            Bl[r] = 0;
-        }
-        int up_h = 0, up_m = 0, up_i = neg, up_b = 0;
-        int dg_h = 0, dg_m = 0, dg_b = 0;
-        int bt_h = 0, bt_m = 0, bt_i = neg, bt_b = 0;
+        for (int r = 0; r < kWarpRows; ++r) Hl[r] = 0;
+        int up_h = 0, dg_h = 0, bt_h = 0;
         int mx = 0;
         int avail = 0;
         bool ok = true;
         // the row above, 32 columns at a time: lane k holds column 32j + k of
         // the current block (cur) and of the next one (nxt), loaded with one
         // coalesced read a block ahead; lane 0 takes column s by a shuffle
-        // (linear gap: the H values only)
-        int4 cur = make_int4(0, 0, 0, 0), nxt = make_int4(0, 0, 0, 0);
-        auto fetch = [&](int64_t c) -> int4 {
-            if (c >= lq) return make_int4(0, 0, 0, 0);
-            if constexpr (CKPT) return make_int4(__ldcg(ck_in + c), 0, 0, 0);
-            if constexpr (AFFINE) return __ldcg(&ring_in[c]);
-            return make_int4(__ldcg((const int*)&ring_in[c]), 0, 0, 0);
+        int cur = 0, nxt = 0;
+        auto fetch = [&](int64_t c) -> int {
+            if (c >= lq) return 0;
+            if constexpr (CKPT) return __ldcg(ck_in + c);
+            return __ldcg((const int*)&ring_in[c]);
         };
         for (int64_t s = 0; s < nsteps; ++s) {
             if (has_up && (s & 31) == 0) {
@@ -258,49 +253,17 @@ __global__ void __launch_bounds__(128, AFFINE ? 5 : 8) band_kernel(KernelArgs A,
             }
             const int x = (int)s - lane;
             const bool active = x >= 0 && x < lq;
-            int rh = 0, rm = 0, ri = neg, rb = 0;
-            int4 above = make_int4(0, 0, 0, 0);
-            if (has_up) {
-                above.x = __shfl_sync(0xffffffffu, cur.x, (int)(s & 31));
-                if constexpr (AFFINE) {
-                    above.y = __shfl_sync(0xffffffffu, cur.y, (int)(s & 31));
-                    above.z = __shfl_sync(0xffffffffu, cur.z, (int)(s & 31));
-                }
-            }
-            if constexpr (AFFINE) {
-                rm = __shfl_up_sync(0xffffffffu, bt_m, 1);
-                ri = __shfl_up_sync(0xffffffffu, bt_i, 1);
-                rb = __shfl_up_sync(0xffffffffu, bt_b, 1);
-            } else {
-                rh = __shfl_up_sync(0xffffffffu, bt_h, 1);
-            }
-            if (lane == 0) {
-                if (has_up && active) {
-                    const int4 v = above;
-                    rh = v.x;
-                    rm = v.x;
-                    ri = v.y;
-                    rb = v.z;
-                } else {
-                    rh = 0;
-                    rm = 0;
-                    ri = neg;
-                    rb = 0;
-                }
-            }
+            const int above = has_up ? __shfl_sync(0xffffffffu, cur, (int)(s & 31)) : 0;
+            int rh = __shfl_up_sync(0xffffffffu, bt_h, 1);
+            if (lane == 0) rh = has_up && active ? above : 0;
             dg_h = x == 0 ? 0 : up_h;
-            dg_m = x == 0 ? 0 : up_m;
-            dg_b = x == 0 ? 0 : up_b;
             up_h = rh;
-            up_m = rm;
-            up_i = ri;
-            up_b = rb;
             if (active) {
                 const int a = __ldg(qg + x);
                 const uint2 pw = prof[lane * alpha1 + a];
                 const bool xin = x > 0;
                 uint32_t w0 = 0;  // the lane's 8 rows as 4-bit codes
-                if constexpr (!AFFINE) {
+                {
                     int up = up_h, diag = dg_h;
                     int Hold[kWarpRows];  // the left neighbours (previous column), for the candidate test
 #pragma unroll
@@ -369,59 +332,6 @@ __global__ void __launch_bounds__(128, AFFINE ? 5 : 8) band_kernel(KernelArgs A,
                         hv.w = __byte_perm(Hl[6], Hl[7], 0x5410);
                         *(uint4*)(codes + ((band * nsteps + s) * kWarp + lane) * kWarpRows * 2) = hv;
                     }
-                } else {
-                    int mup = up_m, iup = up_i, bdiag = dg_b, mdiag = dg_m;
-#pragma unroll
-                    for (int r = 0; r < kWarpRows; ++r) {
-                        const int sc = prof_score(pw, r);
-                        const int m = addmax_relu(bdiag, sc, neg);
-                        const int i = addmax(iup, ext, mup + ge);
-                        const int jj = addmax(Jl[r], ext, Ml[r] + ge);
-                        const int b = max3(m, i, jj);
-                        if constexpr (!MAXIMA) {
-                            uint32_t code = b == m ? kUL : (b == i ? kUp : kLeft);
-                            code = b > 0 ? code : kNo;
-                            const bool main_src = code == kUL;
-                            const bool stop = main_src && xin && (r > 0 || ypos) && mdiag == 0;
-                            code |= stop ? kStopFlag : 0u;
-                            w0 |= code << (4 * r);
-                        } else {
-                            mx = max(mx, b);
-                        }
-                        bdiag = Bl[r];
-                        mdiag = Ml[r];
-                        Ml[r] = m;
-                        Jl[r] = jj;
-                        Bl[r] = b;
-                        mup = m;
-                        iup = i;
-                    }
-                    bt_m = mup;
-                    bt_i = iup;
-                    bt_b = Bl[kWarpRows - 1];
-                    if constexpr (!MAXIMA) {
-                        // candidates: MAIN-source cells (b == m > 0) inside the
-                        // matrix with m at or above the threshold -- rare, so one
-                        // test of the step's maximum of m
-                        const int smax = max(max3(Ml[0], Ml[1], Ml[2]), max3(Ml[3], Ml[4], max3(Ml[5], Ml[6], Ml[7])));
-                        if (smax >= thr) {
-#pragma unroll
-                            for (int r = 0; r < kWarpRows; ++r) {
-                                const int m = Ml[r];
-                                if (m < thr || Bl[r] != m || m <= 0 || r >= rows_left) continue;
-                                w0 |= kCand << (4 * r);
-                                const int k = atomicAdd(ncand, 1);
-                                if (k < cap) {
-                                    Cand cc;
-                                    cc.x = x;
-                                    cc.y = ymine + r;
-                                    cc.score_i = m;
-                                    cc.score_f = (float)m;
-                                    cand[k] = cc;
-                                }
-                            }
-                        }
-                    }
                 }
                 if constexpr (DIRS == 1)
                     *(uint32_t*)(codes + ((band * nsteps + s) * kWarp + lane) * kWarpRows / 2) = w0;
@@ -429,14 +339,11 @@ __global__ void __launch_bounds__(128, AFFINE ? 5 : 8) band_kernel(KernelArgs A,
                     if constexpr (CKPT)
                         __stcg(ck_out + x, bt_h);
                     else
-                        __stcg(&ring_out[x], make_int4(AFFINE ? bt_m : bt_h, bt_i, bt_b, 0));
+                        __stcg(&ring_out[x], make_int4(bt_h, 0, 0, 0));
                 }
             } else {
                 // not started (x < 0): hand the left-boundary values down
                 bt_h = 0;
-                bt_m = 0;
-                bt_i = neg;
-                bt_b = 0;
             }
             // lane 31 stored columns 0 .. s - 31 of the bottom row
             if (store_bnd && lane == kWarp - 1 && ((s + 1) & 31) == 0 && s >= kWarp - 1)

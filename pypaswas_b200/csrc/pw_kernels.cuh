@@ -631,6 +631,14 @@ __host__ __device__ __forceinline__ int64_t warp_layout_offset(int x, int y, int
     return ((band * nsteps + x + l) * 32 + l) * 8 + r;
 }
 
+// The same of the affine band sweep (pw_band_affine.cuh): [band][step][lane]
+// [2 columns][8 rows], step = x / 2 + lane.
+__host__ __device__ __forceinline__ int64_t affine_layout_offset(int x, int y, int lq) {
+    const int band = y >> 8, l = (y & 255) >> 3, r = y & 7;
+    const int64_t nsteps = (int64_t)((lq + 1) / 2) + 31;
+    return (((band * nsteps + (x >> 1) + l) * 32 + l) * 2 + (x & 1)) * 8 + r;
+}
+
 // A traced pair's cells.  Each cell has a 4-bit code (direction, stop flag,
 // candidate flag; two cells per byte, the even index in the low nibble) and a
 // 1-bit mark in a separate plane: collect_kernel marks covered candidates there
@@ -641,11 +649,12 @@ struct PairView {
     uint8_t* marks;     // the wave's mark plane
     int64_t cell0;      // the item's first cell in the wave
     int S, lane, xmax4, lq, lt;
-    int layout;  // 0: strip sweep, targets as strips; 1: strip sweep, queries as strips; 2: warp sweep
+    int layout;  // 0: strip sweep, targets as strips; 1: strip sweep, queries as strips; 2: band sweep, 3: affine
     bool hstore;        // base holds H; codes are derived on read
     int gap, thr;       // hstore: the linear gap and the pair's integer candidate threshold
     // cell (x, y) in the reference's coordinates (x: query, y: target)
     __device__ __forceinline__ int64_t index(int x, int y) const {
+        if (layout == 3) return affine_layout_offset(x, y, lq);
         if (layout == 2) return warp_layout_offset(x, y, lq);
         return layout == 1 ? cell_offset_rt(S, y, x, lane, xmax4) : cell_offset_rt(S, x, y, lane, xmax4);
     }

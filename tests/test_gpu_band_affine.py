@@ -1,0 +1,74 @@
+"""The affine band sweep (blocks of 2 columns, groups of 32, bands of 256 rows)
+at lengths around these edges and over many bands (the row words' epochs
+repeat after 126 bands), as listed pairs (maxima, then codes) and traced from
+an all-against-all call, against the oracle: maxima and hits."""
+import numpy as np
+import pytest
+
+import cases
+from engine_helpers import configure, decode_hits
+from pypaswas_b200 import _native, scores
+
+pytestmark = pytest.mark.gpu
+EDGES = [1, 2, 3, 31, 32, 33, 34, 63, 65, 255, 256, 257, 258, 511, 512, 513, 700, 769]
+
+
+def _check(engine_lib, oracle_mod, q, t, pairs, st, **align):
+    score = scores.make_score(st)
+    e = _native.Engine(0, lib=engine_lib)
+    try:
+        configure(e, score, st)
+        e.set_queries([s.encode() for s in q], np.arange(len(q)))
+        e.set_targets([s.encode() for s in t], np.arange(len(t)) + len(q))
+        if pairs:
+            e.set_pairs([a for a, _ in pairs], [b for _, b in pairs])
+        info = e.align(**align)
+        pm = e.pair_max()
+        hits = decode_hits(*e.hits())
+    finally:
+        e.close()
+    got = {}
+    for h in hits:
+        got.setdefault((h["query"], h["target"]), []).append(h)
+    for a, b in pairs or [(a, b) for a in range(len(q)) for b in range(len(t))]:
+        ref = oracle_mod.run(cases.oracle_params(oracle_mod, score), [q[a]], [t[b]],
+                             cases.pos_scores(score, st, [q[a]], [t[b]]), float(st.minimum_score))
+        assert pm[a, b] == ref["pair_max"][0, 0]
+        assert got.get((a, b), []) == [dict(h, query=a, target=b) for h in ref["hits"]]
+    return info
+
+
+def _case(rng, alphabet, lens_q, lens_t):
+    rs = lambda n: "".join(alphabet[i] for i in rng.integers(0, len(alphabet), n))
+    q, t = [], []
+    for n, m in zip(lens_q, lens_t):
+        q.append(rs(n))
+        k = min(n, m) // 2
+        frag = cases.mutate(rng, q[-1][n - k:], alphabet, 0.1, k // 40)[:m]
+        p = int(rng.integers(0, m - len(frag) + 1))
+        s = rs(m)
+        t.append(s[:p] + frag + s[p + len(frag):])
+    return q, t
+
+
+@pytest.mark.parametrize("alphabet,settings", [
+    ("ACGT", dict(gap_score="-2", gap_extension="-1", minimum_score="6", filter_factor="0.05")),
+    (cases.PROTEIN, dict(matrix_name="BLOSUM62", gap_score="-11", gap_extension="-1", minimum_score="25",
+                         filter_factor="0.01", lower_limit_score="0.95"))])
+@pytest.mark.parametrize("listed", [True, False])
+def test_edge_lengths(engine_lib, oracle_mod, alphabet, settings, listed):
+    rng = np.random.default_rng(len(alphabet) + listed)
+    n = len(EDGES)
+    q, t = _case(rng, alphabet, EDGES, [EDGES[(7 * i + 5) % n] for i in range(n)])
+    info = _check(engine_lib, oracle_mod, q, t, [(i, i) for i in range(n)] if listed else None,
+                  cases.Settings(**settings))
+    assert info.warp_pairs > 0 and info.score_path == 2  # (few long sequences go band by band unlisted too)
+
+
+def test_many_bands(engine_lib, oracle_mod):
+    # 141 bands: ring slots reused 70 times, past the epochs' period of 63
+    rng = np.random.default_rng(5)
+    q, t = _case(rng, "ACGT", [150, 90], [36000, 33000])
+    st = cases.Settings(gap_score="-3", gap_extension="-1", minimum_score="20", filter_factor="0.1")
+    info = _check(engine_lib, oracle_mod, q, t, [(0, 0), (1, 1)], st)
+    assert info.score_path == 2
