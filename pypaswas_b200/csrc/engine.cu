@@ -2791,6 +2791,10 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         TA.t = Aref.t;
         TA.P = Aref.P;
         TA.slot_tile = TT.slot_tile;
+        // the band sweep's pairs have the wave's last slots
+        TA.thread_pairs = ww.empty() ? (int)n_pairs : (int)ww.front().pair_base;
+        const int n_warp = n_tile > 0 ? 0 : (int)n_pairs - TA.thread_pairs;  // (all of them in the tile form, or none)
+        const int gt = (TA.thread_pairs + 127) / 128, gw = (n_warp + 3) / 4;
         const int tb = 128;
         const int gb = (int)((n_pairs + tb - 1) / tb);
         // the tile form's walks: the tiles along the candidates' diagonals
@@ -2834,11 +2838,20 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
             e->launches += 2;
             if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "tile codes launch");
         }
-        if (e->affine)
-            PW_LAUNCH(collect_kernel<true>, gb, tb, 0, e->stream, TA);
-        else
-            PW_LAUNCH(collect_kernel<false>, gb, tb, 0, e->stream, TA);
-        e->launches++;
+        if (gt > 0) {
+            if (e->affine)
+                PW_LAUNCH(collect_kernel<true>, gt, tb, 0, e->stream, TA);
+            else
+                PW_LAUNCH(collect_kernel<false>, gt, tb, 0, e->stream, TA);
+            e->launches++;
+        }
+        if (gw > 0) {
+            if (e->affine)
+                PW_LAUNCH(warp_collect_kernel<true>, gw, tb, 0, e->stream, TA);
+            else
+                PW_LAUNCH(warp_collect_kernel<false>, gw, tb, 0, e->stream, TA);
+            e->launches++;
+        }
         if (n_tile > 0) {
             PW_LAUNCH(tile_collect_kernel, n_tile, kWarp, tsmem, e->stream, Aw, TA, TT);
             e->launches++;
@@ -2925,11 +2938,20 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
             TA.hit_count = e->hit_count.as<int>();
             TA.ops_total = (unsigned long long*)(e->hit_count.as<char>() + 8);
             TA.max_hits = (int)wave_starts;
-            if (e->affine)
-                PW_LAUNCH(walk_kernel<true>, gb, tb, 0, e->stream, TA);
-            else
-                PW_LAUNCH(walk_kernel<false>, gb, tb, 0, e->stream, TA);
-            e->launches++;
+            if (gt > 0) {
+                if (e->affine)
+                    PW_LAUNCH(walk_kernel<true>, gt, tb, 0, e->stream, TA);
+                else
+                    PW_LAUNCH(walk_kernel<false>, gt, tb, 0, e->stream, TA);
+                e->launches++;
+            }
+            if (gw > 0) {
+                if (e->affine)
+                    PW_LAUNCH(warp_walk_kernel<true>, gw, tb, 0, e->stream, TA);
+                else
+                    PW_LAUNCH(warp_walk_kernel<false>, gw, tb, 0, e->stream, TA);
+                e->launches++;
+            }
             if (n_tile > 0) {
                 PW_LAUNCH(tile_walk_kernel, n_tile, kWarp, tsmem, e->stream, Aw, TA, TT);
                 e->launches++;
@@ -2950,8 +2972,14 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
                     cudaSuccess)
                     return cuda_fail(e, c, "alloc ops");
                 TA.ops = e->acc_ops.as<char>();
-                PW_LAUNCH(ops_kernel, (nh + 127) / 128, 128, 0, e->stream, TA, TA.hits, nh);
-                e->launches++;
+                if (gt > 0) {
+                    PW_LAUNCH(ops_kernel, (nh + 127) / 128, 128, 0, e->stream, TA, TA.hits, nh);
+                    e->launches++;
+                }
+                if (gw > 0) {
+                    PW_LAUNCH(warp_ops_kernel, (nh + 3) / 4, 128, 0, e->stream, TA, (const DevHit*)TA.hits, nh);
+                    e->launches++;
+                }
                 if (n_tile > 0 && TT.ops) {
                     // the tile walks' operations go after the others
                     PW_LAUNCH(tile_ops_rebase_kernel, (nh + 127) / 128, 128, 0, e->stream, TT, TA.hits, nh, strip_end);

@@ -621,6 +621,9 @@ struct TraceArgs {
     unsigned long long* ops_total;  // column operations reserved so far (walk_kernel assigns ops offsets)
     const int32_t* slot_tile;       // per pair slot: >= 0 for pairs of the tile form (pw_tiles.cuh), which
                                     // these kernels leave to the tile kernels; null: none
+    int thread_pairs;               // pair slots below are the strip sweep's short pairs (collect_kernel,
+                                    // walk_kernel, ops_kernel: a thread each); from it on the band
+                                    // sweep's, a warp each (the warp_ kernels)
 };
 
 // Offset of cell (x, y) in the layout of the band direction sweep
@@ -741,11 +744,29 @@ __host__ __device__ __forceinline__ uint64_t emission_key(int x, int y) {
            ((uint64_t)(15u - i) << 4) | ty;
 }
 
+// A pair's m kept candidates in walk order: ascending score, then emission
+// order (SmithWaterman.py:699 is a stable sort).
+__device__ __forceinline__ void order_starts(Cand* cl, int m) {
+    for (int k = 1; k < m; ++k) {
+        const Cand key = cl[k];
+        const uint64_t ek = emission_key(key.x, key.y);
+        int j = k - 1;
+        while (j >= 0) {
+            const Cand o = cl[j];
+            const bool after = o.score_f > key.score_f ||
+                               (o.score_f == key.score_f && emission_key(o.x, o.y) > ek);
+            if (!after) break;
+            cl[j + 1] = o;
+            --j;
+        }
+        cl[j + 1] = key;
+    }
+}
+
 template <bool AFFINE>
 __global__ void collect_kernel(TraceArgs A) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= A.n_pairs) return;
-    if (A.slot_tile && A.slot_tile[p] >= 0) return;
+    if (p >= A.thread_pairs) return;
     const PairMeta pm = A.metas[p];
     Cand* cl = A.cands + A.cand_base[p];
     const int n = pm.n_cand;
@@ -779,9 +800,7 @@ __global__ void collect_kernel(TraceArgs A) {
         }
     }
     // keep uncovered candidates (clearing the covered marks, so that the
-    // plane holds only the walk's marks afterwards), then order them for the
-    // walk: ascending score, then emission order (SmithWaterman.py:699 is a
-    // stable sort)
+    // plane holds only the walk's marks afterwards), then order them
     int m = 0;
     for (int k = 0; k < n; ++k) {
         const Cand cc = cl[k];
@@ -790,20 +809,7 @@ __global__ void collect_kernel(TraceArgs A) {
         else
             cl[m++] = cc;
     }
-    for (int k = 1; k < m; ++k) {
-        const Cand key = cl[k];
-        const uint64_t ek = emission_key(key.x, key.y);
-        int j = k - 1;
-        while (j >= 0) {
-            const Cand o = cl[j];
-            const bool after = o.score_f > key.score_f ||
-                               (o.score_f == key.score_f && emission_key(o.x, o.y) > ek);
-            if (!after) break;
-            cl[j + 1] = o;
-            --j;
-        }
-        cl[j + 1] = key;
-    }
+    order_starts(cl, m);
     A.n_starts[p] = m;
 }
 
@@ -843,8 +849,7 @@ __device__ __forceinline__ bool same_residue(uint8_t a, uint8_t b) {
 template <bool AFFINE>
 __global__ void walk_kernel(TraceArgs A) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= A.n_pairs) return;
-    if (A.slot_tile && A.slot_tile[p] >= 0) return;
+    if (p >= A.thread_pairs) return;
     const PairMeta pm = A.metas[p];
     const Cand* cl = A.cands + A.cand_base[p];
     const int m = A.n_starts[p];
@@ -934,6 +939,190 @@ __global__ void walk_kernel(TraceArgs A) {
     }
 }
 
+// ---- the same, one warp a pair, for the pairs of the band sweep.  A path runs
+// along a diagonal most of the time, and one thread following it waits for a
+// dependent load a step; a warp reads 32 cells of the diagonal at once, one a
+// lane, and takes the run of plain diagonal steps and the step after it
+// together (12 protein pairs of 2-8 kaa: 4.9 ms a thread each, 0.4 ms a warp
+// each).  The cells of a batch lie in different columns, so their marks lie in
+// different bytes.
+
+// Lane i's cell of the diagonal up from (x, y): its code, kNo outside the matrix.
+__device__ __forceinline__ bool diagonal_code(const PairView& v, int x, int y, int lane, uint32_t* cd) {
+    const int cx = x - lane, cy = y - lane;
+    const bool in = cx >= 0 && cy >= 0;
+    *cd = in ? v.code(cx, cy) : (uint32_t)kNo;
+    v.prefetch(cx - kWarp, cy - kWarp);
+    return in;
+}
+
+template <bool AFFINE>
+__global__ void __launch_bounds__(128) warp_collect_kernel(TraceArgs A) {
+    const int lane = threadIdx.x & 31;
+    const int p = A.thread_pairs + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (p >= A.n_pairs || (A.slot_tile && A.slot_tile[p] >= 0)) return;
+    const PairMeta pm = A.metas[p];
+    Cand* cl = A.cands + A.cand_base[p];
+    const int n = pm.n_cand;
+    const PairView v = pair_view(A, pm);
+    // marking chains: the nearest candidate up a candidate's chain is covered
+    // (a lone candidate has no other candidate to cover)
+    for (int k = 0; k < n && n > 1; ++k) {
+        int x = cl[k].x - 1, y = cl[k].y - 1;
+        while (x >= 0 && y >= 0) {
+            uint32_t cd;
+            const bool in = diagonal_code(v, x, y, lane, &cd);
+            const unsigned ul = __ballot_sync(0xffffffffu, in && (cd & 3) == kUL && !(cd & kCand));
+            const int run = ul == 0xffffffffu ? kWarp : __ffs(~ul) - 1;
+            x -= run;
+            y -= run;
+            if (run == kWarp) continue;
+            cd = __shfl_sync(0xffffffffu, cd, run);  // kNo past the matrix
+            const int d = cd & 3;
+            if (cd & kCand) {
+                if (lane == 0) v.mark(x, y);  // covered
+                break;
+            }
+            if (d == kNo || AFFINE) break;
+            if (d == kUp)
+                --y;
+            else
+                --x;
+        }
+        __syncwarp();
+    }
+    // keep the uncovered candidates, 32 at a time; covered marks are cleared again
+    int m = 0;
+    for (int k0 = 0; k0 < n; k0 += kWarp) {
+        const int k = k0 + lane;
+        Cand cc;
+        bool keep = false;
+        if (k < n) {
+            cc = cl[k];
+            keep = !v.marked(cc.x, cc.y);
+        }
+        const unsigned kept = __ballot_sync(0xffffffffu, keep);
+        if (keep) cl[m + __popc(kept & ((1u << lane) - 1u))] = cc;
+        unsigned gone = __ballot_sync(0xffffffffu, k < n && !keep);
+        while (gone) {  // one at a time: marks of different cells may share a byte
+            const int i = __ffs(gone) - 1;
+            gone &= gone - 1;
+            if (lane == i) v.unmark(cc.x, cc.y);
+            __syncwarp();
+        }
+        m += __popc(kept);
+    }
+    __syncwarp();
+    if (lane != 0) return;
+    order_starts(cl, m);
+    A.n_starts[p] = m;
+}
+
+template <bool AFFINE>
+__global__ void __launch_bounds__(128) warp_walk_kernel(TraceArgs A) {
+    const int lane = threadIdx.x & 31;
+    const int p = A.thread_pairs + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (p >= A.n_pairs || (A.slot_tile && A.slot_tile[p] >= 0)) return;
+    const PairMeta pm = A.metas[p];
+    const Cand* cl = A.cands + A.cand_base[p];
+    const int m = A.n_starts[p];
+    const PairView v = pair_view(A, pm);
+    const uint8_t* qs = A.q.raw + A.q.raw_off[pm.query];
+    const uint8_t* ts = A.t.raw + A.t.raw_off[pm.target];
+    const bool same_id = A.q.key[pm.query] == A.t.key[pm.target];
+    for (int k = 0; k < m; ++k) {
+        if (A.allowed && !A.allowed[A.start_off[p] + k]) continue;
+        const Cand st = cl[k];
+        int x = st.x, y = st.y;
+        int dir = walk_direction<AFFINE>(v, x, y);
+        bool show = true;
+        if (same_id) {  // SmithWaterman.py:752-755
+            dir = kStopDir;
+            show = false;
+        }
+        if ((double)st.score_f < A.P.host_minimum) show = false;  // :758-759
+        int s_start = x + 1, t_start = y + 1, ncols = 0, mt = 0, mm = 0;
+        // affine stop rule: whether a candidate lies on the diagonal run of
+        // MAIN cells that the walk came along (-1: unknown, after a gap move)
+        int run_next = -1;
+        bool go = show && dir != kStopDir && dir != 32;  // :761
+        while (go && x >= 0 && y >= 0) {
+            uint32_t cd;
+            const bool in = diagonal_code(v, x, y, lane, &cd);
+            const int sx = x - lane, sy = y - lane;
+            const bool ul = in && (cd & 3) == kUL;
+            unsigned stops = __ballot_sync(0xffffffffu, ul && (cd & kStopFlag));
+            const unsigned uls = __ballot_sync(0xffffffffu, ul);
+            const int reach = uls == 0xffffffffu ? kWarp : __ffs(~uls) - 1;  // the run of MAIN cells
+            const unsigned in_run = reach == kWarp ? 0xffffffffu : (1u << reach) - 1u;
+            stops &= in_run;
+            int after = -1;  // run_next behind the run
+            if (AFFINE) {
+                // a stop cell ends the walk when a candidate lies on the run
+                // here or further down-right
+                const unsigned cands = __ballot_sync(0xffffffffu, ul && (cd & kCand)) & in_run;
+                const unsigned from = cands ? ~((cands & (0u - cands)) - 1u) : 0u;  // lanes from the first candidate on
+                if (run_next < 0 && (stops & ~from)) run_next = run_has_candidate(v, x + 1, y + 1) ? 1 : 0;
+                if (run_next != 1) stops &= from;
+                after = cands ? 1 : run_next;
+            }
+            const int run = stops ? __ffs(stops) - 1 : reach;
+            // the cell after the run: a stop cell, or one of another code
+            const bool more = run < kWarp && __shfl_sync(0xffffffffu, (int)in, run & 31) != 0;
+            const int d_end = stops ? kStopDir : (int)(__shfl_sync(0xffffffffu, cd, run & 31) & 3);
+            const int n = run + (more ? 1 : 0);
+            const int last = more ? d_end : (int)kUL;
+            const bool end = last == kStopDir || last == kNo || (!more && run < kWarp);
+            // the first marked cell of the batch ends the walk there (IN_ALIGNMENT)
+            const unsigned hit_mark = __ballot_sync(0xffffffffu, lane < n && v.marked(sx, sy));
+            const int f = hit_mark ? __ffs(hit_mark) - 1 : n;
+            if (lane < (hit_mark ? f + 1 : n)) v.mark(sx, sy);
+            const bool dg = lane < f && (lane < run || last == kStopDir);
+            const unsigned n_dg = __popc(__ballot_sync(0xffffffffu, dg));
+            const unsigned n_mt = __popc(__ballot_sync(0xffffffffu, dg && same_residue(ts[sy], qs[sx])));
+            const int n_l = more && f == n && last == kLeft, n_u = more && f == n && last == kUp;
+            mt += (int)n_mt;
+            mm += (int)(n_dg - n_mt);
+            ncols += (int)n_dg + n_l + n_u;
+            s_start -= (int)n_dg + n_l;
+            t_start -= (int)n_dg + n_u;
+            __syncwarp();
+            if (hit_mark) {
+                show = false;
+                go = false;
+            } else if (end) {
+                go = false;
+            } else {
+                x -= run + (last == kLeft ? 1 : 0);
+                y -= run + (last == kUp ? 1 : 0);
+                run_next = last == kUL ? after : -1;
+            }
+        }
+        if (show && lane == 0) {
+            const int h = atomicAdd(A.hit_count, 1);
+            if (h < A.max_hits) {
+                DevHit o;
+                o.pair = p;
+                o.query = pm.query;
+                o.target = pm.target;
+                o.s_start = s_start;
+                o.s_end = st.x;
+                o.t_start = t_start;
+                o.t_end = st.y;
+                o.score = st.score_f;
+                o.matches = mt;
+                o.mismatches = mm;
+                o.n_cols = ncols;
+                o.end_x = st.x;
+                o.end_y = st.y;
+                o.ops_offset = (int64_t)atomicAdd(A.ops_total, (unsigned long long)ncols);
+                A.hits[h] = o;
+            }
+        }
+        __syncwarp();
+    }
+}
+
 // Translation units that only need the score sweep define PW_SCORE_SWEEP_ONLY
 // so that these non-template kernels are emitted once, by engine.cu.
 #ifndef PW_SCORE_SWEEP_ONLY
@@ -943,7 +1132,7 @@ __global__ void ops_kernel(TraceArgs A, const DevHit* hits, int n_hits) {
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= n_hits) return;
     const DevHit H = hits[h];
-    if (A.slot_tile && A.slot_tile[H.pair] >= 0) return;
+    if (H.pair >= A.thread_pairs) return;
     const PairMeta pm = A.metas[H.pair];
     PairView v = pair_view(A, pm);
     int x = H.end_x, y = H.end_y;
@@ -964,6 +1153,37 @@ __global__ void ops_kernel(TraceArgs A, const DevHit* hits, int n_hits) {
             --y;
         }
         o[H.n_cols - 1 - k] = op;
+    }
+}
+
+// The same, one warp a hit, for the hits of the band sweep's pairs.
+__global__ void __launch_bounds__(128) warp_ops_kernel(TraceArgs A, const DevHit* hits, int n_hits) {
+    const int lane = threadIdx.x & 31;
+    const int h = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (h >= n_hits) return;
+    const DevHit H = hits[h];
+    if (H.pair < A.thread_pairs || (A.slot_tile && A.slot_tile[H.pair] >= 0)) return;
+    const PairView v = pair_view(A, A.metas[H.pair]);
+    int x = H.end_x, y = H.end_y;
+    char* o = A.ops + H.ops_offset + H.n_cols - 1;
+    for (int k = 0; k < H.n_cols;) {
+        uint32_t cd;
+        diagonal_code(v, x, y, lane, &cd);
+        const int d = cd & 3;
+        const unsigned uls = __ballot_sync(0xffffffffu, d == kUL);
+        const int reach = uls == 0xffffffffu ? kWarp : __ffs(~uls) - 1;
+        const int left = H.n_cols - k, run = min(reach, left);
+        const bool more = run < kWarp && run < left;  // a gap step behind the run
+        if (lane < run) o[-(k + lane)] = 'M';
+        const int d_end = __shfl_sync(0xffffffffu, d, run & 31);
+        if (more && lane == run) o[-(k + run)] = d == kLeft ? 'I' : d == kUp ? 'D' : 'M';
+        k += run + (more ? 1 : 0);
+        x -= run;
+        y -= run;
+        if (more) {
+            if (d_end != kUp) --x;
+            if (d_end != kLeft) --y;
+        }
     }
 }
 

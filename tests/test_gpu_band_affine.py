@@ -72,3 +72,34 @@ def test_many_bands(engine_lib, oracle_mod):
     st = cases.Settings(gap_score="-3", gap_extension="-1", minimum_score="20", filter_factor="0.1")
     info = _check(engine_lib, oracle_mod, q, t, [(0, 0), (1, 1)], st)
     assert info.score_path == 2
+
+
+@pytest.mark.parametrize("affine", [True, False])
+@pytest.mark.parametrize("limit", ["0.5", "0.9"])
+def test_walks_with_many_candidates(engine_lib, oracle_mod, affine, limit):
+    # repeats: candidates that cover one another, walks that meet, stop cells
+    # with and without a candidate on their run (a warp a pair; linear: stored codes)
+    rng = np.random.default_rng(9)
+    rs = lambda n: "".join("ACGT"[i] for i in rng.integers(0, 4, n))
+    unit = rs(45)
+    q, t = [], []
+    for n in (120, 330, 600):
+        q.append(rs(n) + unit + rs(20) + unit[:30] + rs(n // 3))
+        t.append(rs(n // 2) + cases.mutate(rng, unit, "ACGT", 0.08, 1) + rs(31) + unit + rs(n))
+    st = cases.Settings(match_score="5", mismatch_score="-3", gap_score="-4", gap_extension="-1" if affine else "0",
+                        minimum_score="40", lower_limit_score=limit, filter_factor="0.02")
+    score = scores.make_score(st)
+    ref = oracle_mod.run(cases.oracle_params(oracle_mod, score), q, t, cases.pos_scores(score, st, q, t),
+                         float(st.minimum_score))
+    e = _native.Engine(0, lib=engine_lib)
+    try:
+        configure(e, score, st)
+        e.set_queries([s.encode() for s in q], np.arange(len(q)))
+        e.set_targets([s.encode() for s in t], np.arange(len(t)) + len(q))
+        e.set_tuning(_native.PW_TUNE_TILE_TRACE, 1)
+        info = e.align()
+        hits = decode_hits(*e.hits())
+    finally:
+        e.close()
+    assert info.warp_pairs > 0 and info.starting_points > info.traced_pairs
+    assert hits == ref["hits"]
