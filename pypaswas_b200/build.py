@@ -13,7 +13,7 @@ CSRC = os.path.join(PACKAGE_DIR, "csrc")
 SOURCES = [os.path.join(CSRC, f) for f in (
     "engine.cu", "noalloc.cu", "score16_linear.cu", "score16_affine.cu", "score16_dual.cu",
     "server.cpp", "format.cpp", "reader.cpp")]
-DEPENDS = SOURCES + [os.path.join(CSRC, f) for f in ("score16_variants.h", "pw_device.cuh", "pw_kernels.cuh", "pw_score16.cuh", "pw_band.cuh", "pw_band_ck.cuh", "pw_band_affine.cuh", "pw_tiles.cuh", "pw_plan.h", "pw_finish.cuh", "pw_host.h", "server.cpp")] + [
+DEPENDS = SOURCES + [os.path.join(CSRC, f) for f in ("score16_variants.h", "pw_device.cuh", "pw_kernels.cuh", "pw_score16.cuh", "pw_band.cuh", "pw_band_ck.cuh", "pw_band_affine.cuh", "pw_band_float.cuh", "pw_tiles.cuh", "pw_plan.h", "pw_finish.cuh", "pw_host.h", "server.cpp")] + [
     os.path.join(REPO_DIR, "include", "paswas_b200.h")]
 LIBRARY = os.path.join(PACKAGE_DIR, "libpaswas_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")

@@ -35,6 +35,7 @@
 #include "pw_band.cuh"
 #include "pw_band_ck.cuh"
 #include "pw_band_affine.cuh"
+#include "pw_band_float.cuh"
 #include "pw_tiles.cuh"
 #include "pw_plan.h"
 #include "pw_finish.cuh"
@@ -540,8 +541,10 @@ int pick_class(int lt, bool affine) {
     return kS32Multi;
 }
 
-// The 16-bit score sweep's class of a strip pair whose longer strip has lt rows.
-int pick_class16(int lt, bool affine) {
+// The 16-bit score sweep's class of a strip pair whose longer strip has lt rows
+// (the profile of 64 rows and more than 220 residues leaves no room for four warps).
+int pick_class16(int lt, bool affine, int alpha1) {
+    if (lt > 48 && alpha1 > 220) return kS32Multi;
     if (lt > 16 && lt <= 24) return kS24;
     if (!affine && lt > 32 && lt <= 40) return kS40;
     return pick_class(lt, affine);
@@ -1189,6 +1192,7 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
         const std::vector<int32_t>& lane_len = trans ? pr.tlen : pr.qlen;
         const std::vector<int32_t>& lane_order = trans ? pr.order_t : pr.order;
         const int n_strip = trans ? nq : nt, n_lane = trans ? nt : nq;
+        const int alpha1 = (trans ? pr.alpha_t : pr.alpha) + 1;
         std::vector<WorkItem> items;
         std::vector<int> cls;
         std::vector<int64_t> cost;
@@ -1206,7 +1210,7 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
             const int sa = strip_order[i], sb = !dual && i + 1 < n_strip ? strip_order[i + 1] : -1;
             const int ls = std::max(strip_len[sa], sb >= 0 ? strip_len[sb] : 0);
             if (grid) {
-                const int k = pick_class16(ls, e->affine);
+                const int k = pick_class16(ls, e->affine, alpha1);
                 if (k != kS32Multi) {
                     gstrips[k].push_back(make_int2(sa, sb));
                     continue;
@@ -1221,7 +1225,7 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
                 w.lanes = std::min(kWarp, n_lane - g);
                 w.lanes_hi = dual ? std::max(0, std::min(kWarp, n_lane - g - kWarp)) : 0;
                 w.xmax = lane_len[lane_order[g]];
-                const int k = pick_class16(ls, e->affine);
+                const int k = pick_class16(ls, e->affine, alpha1);
                 w.S = class_S(k);
                 items.push_back(w);
                 cls.push_back(k);
@@ -1573,6 +1577,13 @@ static std::vector<int4> band_queue(const std::vector<int>& nbands, const std::v
     return entries;
 }
 
+// Warps of a block whose warps take `warp_smem` bytes of shared memory each:
+// four, fewer where large alphabets' profiles leave room for fewer.
+constexpr int kBlockSmem = 227 * 1024;
+static int block_warps(int warp_smem) {
+    return 4 * warp_smem <= kBlockSmem ? 4 : 2 * warp_smem <= kBlockSmem ? 2 : 1;
+}
+
 // Launches band_kernel over `pairs` (one warp per band, the bands of a pair
 // chained across warps, pw_band.cuh).  DIRS 1: the direction sweep of traced
 // pairs (cell codes), 2: the same storing H (linear gap), 3: the checkpoint
@@ -1582,20 +1593,25 @@ template <int DIRS>
 static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pairs, double* kernel_ms,
                           int* n_launch) {
     if (pairs.empty()) return PW_OK;
-    const int prof_bytes = (int)align_up((int64_t)kWarp * (A.P.alpha + 1) * kWarpRows, 16);
-    const int smem = 4 * (e->affine ? band_affine_warp_smem(A.P.alpha + 1) : prof_bytes);
+    const bool ints = e->pr.int_path, aff_ints = e->affine && ints;
+    const int warp_smem = !ints ? band_float_warp_smem(A.P.alpha + 1)
+                          : e->affine ? band_affine_warp_smem(A.P.alpha + 1)
+                                      : (int)align_up((int64_t)kWarp * (A.P.alpha + 1) * kWarpRows, 16);
+    const int bw = block_warps(warp_smem), smem = bw * warp_smem;
     auto kern = band_kernel<DIRS>;
     if constexpr (DIRS < 2)
-        if (e->affine) kern = band_affine_kernel<DIRS>;
+        if (aff_ints) kern = band_affine_kernel<DIRS>;
+    if constexpr (DIRS == 1)
+        if (!ints) kern = e->affine ? band_float_kernel<true> : band_float_kernel<false>;
     cudaError_t c;
     if (smem > 48 * 1024 &&
         (c = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
         return cuda_fail(e, c, "band sweep smem");
     int per_sm = 0;
-    if ((c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem)) != cudaSuccess)
+    if ((c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bw * kWarp, smem)) != cudaSuccess)
         return cuda_fail(e, c, "occupancy");
     per_sm = std::max(1, std::min(per_sm, 16));
-    const int warps = grid_cap(e, per_sm) * 4;
+    const int warps = grid_cap(e, per_sm) * bw;
     // queue: the bands of each pair form a chain (pw_plan.h), longest pairs first
     std::vector<int> order(pairs.size());
     std::iota(order.begin(), order.end(), 0);
@@ -1603,7 +1619,7 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
     for (size_t k = 0; k < pairs.size(); ++k) {
         pairs[k].nbands = std::max(1, pairs[k].nbands);
         const int lq = e->pr.qlen[pairs[k].q];
-        steps[k] = (int64_t)(e->affine ? affine_blocks(lq) : lq) + kWarp - 1;
+        steps[k] = (int64_t)(aff_ints ? affine_blocks(lq) : lq) + kWarp - 1;
     }
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
         return steps[x] * pairs[x].nbands > steps[y] * pairs[y].nbands;
@@ -1619,10 +1635,10 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
         if constexpr (DIRS < 3) {
             sorted[k].ring_off = ring_elems;
             const int lq = e->pr.qlen[sorted[k].q];
-            if (sorted[k].nbands > 1) ring_elems += 2 * (int64_t)(e->affine ? affine_blocks(lq) : lq);
+            if (sorted[k].nbands > 1) ring_elems += 2 * (int64_t)(aff_ints ? affine_blocks(lq) : lq);
         }
     }
-    std::vector<int4> entries = band_queue(nstr, xm, warps, e->affine ? kAffLead : kBandLead);
+    std::vector<int4> entries = band_queue(nstr, xm, warps, aff_ints ? kAffLead : kBandLead);
     const size_t n = entries.size();
     if (e->tune[PW_TUNE_STALL_TEST]) {
         // one band below another waits on the spare flag (index n) instead
@@ -1643,7 +1659,7 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
     if ((c = cudaMemsetAsync(e->band_prog.p, 0, (n + 1) * sizeof(int), e->stream)) != cudaSuccess ||
         (c = cudaMemsetAsync(e->chain_abort.p, 0, sizeof(int), e->stream)) != cudaSuccess ||
         (c = cudaMemsetAsync(e->counter.as<int>() + kNumClasses, 0, sizeof(int), e->stream)) != cudaSuccess ||
-        (e->affine && ring_elems > 0 &&  // no word shows a band's epoch yet
+        (aff_ints && ring_elems > 0 &&  // no word shows a band's epoch yet
          (c = cudaMemsetAsync(e->band_ring.p, 0, (size_t)ring_elems * sizeof(int4), e->stream)) != cudaSuccess))
         return cuda_fail(e, c, "reset band state");
     BandArgs B;
@@ -1659,12 +1675,12 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
     B.max_out = e->band_out.as<float>();
     B.ck = DIRS == 3 ? e->tile_ck.as<int>() : nullptr;
     B.wait_ns = wait_limit(e);
-    const int grid = std::max(1, std::min(grid_cap(e, per_sm), (int)((n + 3) / 4)));
+    const int grid = std::max(1, std::min(grid_cap(e, per_sm), (int)((n + bw - 1) / bw)));
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     cudaEventRecord(a, e->stream);
-    PW_LAUNCH(kern, grid, 128, smem, e->stream, A, B);
+    PW_LAUNCH(kern, grid, bw * kWarp, smem, e->stream, A, B);
     e->launches++;
     cudaEventRecord(b, e->stream);
     if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "band sweep launch");
@@ -1691,16 +1707,16 @@ static int run_band_ck_phase(pw_engine* e, KernelArgs A, const std::vector<BandC
                              double* kernel_ms, int* n_launch) {
     if (pairs.empty()) return PW_OK;
     auto kern = band_ck_kernel<PAIR>;
-    const int smem = 4 * band_ck_warp_smem(A.P.alpha + 1);
+    const int bw = block_warps(band_ck_warp_smem(A.P.alpha + 1)), smem = bw * band_ck_warp_smem(A.P.alpha + 1);
     cudaError_t c;
     if (smem > 48 * 1024 &&
         (c = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess)
         return cuda_fail(e, c, "band sweep smem");
     int per_sm = 0;
-    if ((c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem)) != cudaSuccess)
+    if ((c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bw * kWarp, smem)) != cudaSuccess)
         return cuda_fail(e, c, "occupancy");
     per_sm = std::max(1, std::min(per_sm, 16));
-    const int warps = grid_cap(e, per_sm) * 4;
+    const int warps = grid_cap(e, per_sm) * bw;
     std::vector<int> order(pairs.size());
     std::iota(order.begin(), order.end(), 0);
     std::vector<int64_t> steps(pairs.size());
@@ -1752,12 +1768,12 @@ static int run_band_ck_phase(pw_engine* e, KernelArgs A, const std::vector<BandC
     B.ck = e->p1_ck.as<int>();
     B.limit = limit;
     B.wait_ns = wait_limit(e);
-    const int grid = std::max(1, std::min(grid_cap(e, per_sm), (int)((n + 3) / 4)));
+    const int grid = std::max(1, std::min(grid_cap(e, per_sm), (int)((n + bw - 1) / bw)));
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     cudaEventRecord(a, e->stream);
-    PW_LAUNCH(kern, grid, 128, smem, e->stream, A, B);
+    PW_LAUNCH(kern, grid, bw * kWarp, smem, e->stream, A, B);
     e->launches++;
     cudaEventRecord(b, e->stream);
     if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "band sweep launch");
@@ -1946,7 +1962,7 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         // checkpoints and tile maxima (band_ck_kernel), so that the traced
         // pairs need no second sweep -- when they take at most 35% of the free
         // device memory
-        bool p1ck = !e->affine && e->tune[PW_TUNE_TILE_TRACE] != 1;
+        bool p1ck = !e->affine && e->tune[PW_TUNE_TILE_TRACE] != 1 && band_ck_warp_smem(A.P.alpha + 1) <= kBlockSmem;
         std::vector<BandCk> bp2, bp1;  // two pairs a chain in 16-bit halves, one on 32-bit lanes
         int64_t ck_ints = 0;           // used ints of p1_ck
         auto ck_of = [&](size_t j) {   // a single pair on 32-bit lanes
@@ -2299,10 +2315,9 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
     // one-warp-per-pair sweep (pw_band.cuh); the others are grouped 32 to
     // a warp, one pair per lane, in the orientation where they cluster
     // (slot cost = strip length x longest lane x 32 per item).
-    const bool warp_ok = pr.int_path;
     std::vector<std::pair<int32_t, int32_t>> warp_pairs;  // (query, target)
     std::vector<char> t_warp((size_t)nt, 0);              // targets whose pairs went to the warp sweep
-    if (warp_ok) {
+    if (pr.int_path || band_float_warp_smem(pr.alpha + 1) <= kBlockSmem) {
         // short targets stay on the strip sweep only when there are enough of
         // them to give every SM a full warp: a few strip items run one lane per
         // pair, latency bound, far longer than the same pairs one per warp
@@ -2442,7 +2457,7 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         w.first = wp.first;
         w.lanes = 1;
         w.xmax = qlen[wp.first];
-        w.orient = e->affine ? 3 : 2;  // PairView::layout
+        w.orient = e->affine && pr.int_path ? 3 : 2;  // PairView::layout
         w.S = kWarpRows;
         items2.push_back(w);
         cls2.push_back(kNumClasses);  // marks a warp item
@@ -2450,7 +2465,7 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         // (the score sweep's checkpoints, when it kept them, are not the wave's)
         bytes2.push_back(tile_form ? (p1ck ? 0 : tile_checkpoint_ints(qlen[wp.first], tlen[wp.second]) * 4) +
                                          align_up(((int64_t)qlen[wp.first] * tlen[wp.second] + 31) / 32 * 4, 16)
-                                   : align_up(e->affine ? affine_code_bytes(qlen[wp.first], tlen[wp.second])
+                                   : align_up(e->affine && pr.int_path ? affine_code_bytes(qlen[wp.first], tlen[wp.second])
                                                          : warp_code_bytes(qlen[wp.first], tlen[wp.second], hstore), 16));
         qmax_warp = std::max(qmax_warp, qlen[wp.first]);
     }
