@@ -447,6 +447,20 @@ extern "C" int pw_set_scoring(pw_engine* e, const float* matrix, int dim, int ch
     return PW_OK;
 }
 
+// dst = src with ASCII letters upper-cased; whether dst held that already.
+// (restrict: the compiler takes 16 bytes at a time; one at a time a 75 MB read
+// set took 9.5 ms on 16 threads, a 3.8 MB target set 3.2 ms on one)
+static bool upper_bytes(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src, int64_t n) {
+    uint8_t diff = 0;
+    for (int64_t i = 0; i < n; ++i) {
+        const uint8_t c = src[i];
+        const uint8_t u = (uint8_t)(c - ((uint8_t)(c - 'a') < 26u ? 32 : 0));
+        diff = (uint8_t)(diff | (dst[i] ^ u));
+        dst[i] = u;
+    }
+    return diff == 0;
+}
+
 // The residues as the engine keeps them: ASCII letters upper-cased (the
 // reference upper-cases every sequence before its kernels see it), on host
 // threads.  Returns whether dst already held exactly that.
@@ -456,16 +470,8 @@ static bool copy_upper(HostBuf<uint8_t>& dst, const uint8_t* src, int64_t n, boo
     *ok = same_size || dst.resize((size_t)n, kDirectBytes);
     if (!*ok) return false;
     parallel_for(n, [&](int64_t i0, int64_t i1) {
-        uint8_t* d = dst.data();
-        bool diff = false;
-        for (int64_t i = i0; i < i1; ++i) {
-            const uint8_t c = src[i];
-            const uint8_t u = (uint8_t)(c - (((uint8_t)(c - 'a') < 26u) ? 32 : 0));
-            diff |= d[i] != u;
-            d[i] = u;
-        }
-        if (diff) differ.store(true, std::memory_order_relaxed);
-    }, (int64_t)1 << 22);
+        if (!upper_bytes(dst.data() + i0, src + i0, i1 - i0)) differ.store(true, std::memory_order_relaxed);
+    }, (int64_t)1 << 20);
     return !differ.load();
 }
 
