@@ -1470,78 +1470,115 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
 }
 
 
-// Orders the n accumulated hits (acc_hits / acc_ops) as the reference's
-// HitList and spells their strings on the device; the records land in
-// h_hits / h_strings.
-static cudaError_t finish_hits(pw_engine* e, int64_t n, int64_t* str_bytes) {
+// Bits that hold values 0 .. v.
+static int bits_for(uint64_t v) {
+    int b = 0;
+    while (b < 64 && (v >> b) != 0) ++b;
+    return b;
+}
+
+// Orders the n accumulated hits (acc_hits / acc_ops, n_ops column operations
+// in all) as the reference's HitList and spells their strings on the device;
+// the records land in h_hits / h_strings.  max_score: no hit scores higher
+// (integer scores).
+static cudaError_t finish_hits(pw_engine* e, int64_t n, int64_t n_ops, int64_t max_score, int64_t* str_bytes) {
     *str_bytes = 0;
     e->h_hits.clear();
     e->h_strings.clear();
     if (n <= 0) return cudaSuccess;
     if (n > (int64_t)INT32_MAX) return cudaErrorInvalidValue;
     cudaError_t c;
+    const Prepared& pr = e->pr;
+    const int64_t total = 3 * n_ops;
     const size_t k8 = (size_t)n * sizeof(uint64_t), k4 = (size_t)n * sizeof(int32_t);
-    if ((c = e->fk_a.reserve(e->stream, k8)) != cudaSuccess || (c = e->fk_b.reserve(e->stream, k8)) != cudaSuccess ||
-        (c = e->fk_c.reserve(e->stream, k8)) != cudaSuccess || (c = e->fk_t.reserve(e->stream, k8)) != cudaSuccess ||
-        (c = e->fk_g.reserve(e->stream, k8)) != cudaSuccess || (c = e->fi_a.reserve(e->stream, k4)) != cudaSuccess ||
-        (c = e->fi_b.reserve(e->stream, k4)) != cudaSuccess || (c = e->f_len.reserve(e->stream, k8)) != cudaSuccess ||
-        (c = e->f_soff.reserve(e->stream, k8)) != cudaSuccess)
-        return c;
-    const DevHit* h = e->acc_hits.as<DevHit>();
-    uint64_t *ka = e->fk_a.as<uint64_t>(), *kb = e->fk_b.as<uint64_t>(), *kc = e->fk_c.as<uint64_t>();
-    uint64_t *kt = e->fk_t.as<uint64_t>(), *kg = e->fk_g.as<uint64_t>();
-    int32_t *ia = e->fi_a.as<int32_t>(), *ib = e->fi_b.as<int32_t>();
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)e->sm_count * 16));
-    PW_LAUNCH(hit_key_kernel, grid, 256, 0, e->stream, h, n, ka, kb, kc, ia);
-    size_t tmp = 0;
-    if ((c = cub::DeviceRadixSort::SortPairs(nullptr, tmp, kc, kt, ia, ib, (int)n, 0, 64, e->stream)) != cudaSuccess ||
-        (c = e->scan_tmp.reserve(e->stream, std::max<size_t>(tmp, 16))) != cudaSuccess)
-        return c;
-    tmp = e->scan_tmp.bytes;
-    // three stable passes, least significant word first
-    if ((c = cub::DeviceRadixSort::SortPairs(e->scan_tmp.p, tmp, kc, kt, ia, ib, (int)n, 0, 64, e->stream)) !=
-        cudaSuccess)
-        return c;
-    PW_LAUNCH(gather_key_kernel, grid, 256, 0, e->stream, kb, ib, n, kg);
-    tmp = e->scan_tmp.bytes;
-    if ((c = cub::DeviceRadixSort::SortPairs(e->scan_tmp.p, tmp, kg, kt, ib, ia, (int)n, 0, 64, e->stream)) !=
-        cudaSuccess)
-        return c;
-    PW_LAUNCH(gather_key_kernel, grid, 256, 0, e->stream, ka, ia, n, kg);
-    tmp = e->scan_tmp.bytes;
-    if ((c = cub::DeviceRadixSort::SortPairs(e->scan_tmp.p, tmp, kg, kt, ia, ib, (int)n, 0, 64, e->stream)) !=
-        cudaSuccess)
-        return c;
-    // string offsets in the final order
-    int64_t *len = e->f_len.as<int64_t>(), *soff = e->f_soff.as<int64_t>();
-    PW_LAUNCH(hit_len_kernel, grid, 256, 0, e->stream, h, ib, n, len);
-    size_t stmp = 0;
-    if ((c = cub::DeviceScan::ExclusiveSum(nullptr, stmp, len, soff, (int64_t)n, e->stream)) != cudaSuccess) return c;
-    if (stmp > e->scan_tmp.bytes && (c = e->scan_tmp.reserve(e->stream, stmp)) != cudaSuccess) return c;
-    stmp = e->scan_tmp.bytes;
-    if ((c = cub::DeviceScan::ExclusiveSum(e->scan_tmp.p, stmp, len, soff, (int64_t)n, e->stream)) != cudaSuccess)
-        return c;
-    int64_t tail[2] = {0, 0};
-    if ((c = copy_d2h(e, &tail[0], soff + n - 1, sizeof(int64_t))) !=
-            cudaSuccess ||
-        (c = copy_d2h(e, &tail[1], len + n - 1, sizeof(int64_t))) !=
-            cudaSuccess ||
-        (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
-        return c;
-    const int64_t total = tail[0] + tail[1];
-    if ((c = e->f_out.reserve(e->stream, (size_t)n * sizeof(pw_hit))) != cudaSuccess ||
+    if ((c = e->fi_a.reserve(e->stream, k4)) != cudaSuccess || (c = e->fi_b.reserve(e->stream, k4)) != cudaSuccess ||
+        (c = e->f_len.reserve(e->stream, k8)) != cudaSuccess || (c = e->f_soff.reserve(e->stream, k8)) != cudaSuccess ||
+        (c = e->f_out.reserve(e->stream, (size_t)n * sizeof(pw_hit))) != cudaSuccess ||
         (c = e->f_str.reserve(e->stream, (size_t)std::max<int64_t>(total, 16))) != cudaSuccess)
         return c;
-    PW_LAUNCH(hit_out_kernel, grid, 256, 0, e->stream, h, ib, soff, n, e->acc_ops.as<char>(), e->q_raw.as<uint8_t>(),
+    const DevHit* h = e->acc_hits.as<DevHit>();
+    int32_t *ia = e->fi_a.as<int32_t>(), *ib = e->fi_b.as<int32_t>();
+    int64_t *len = e->f_len.as<int64_t>(), *soff = e->f_soff.as<int64_t>();
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)e->sm_count * 16));
+    HitKeyBits kb;
+    kb.x_top = (uint32_t)(pr.maxlq >> 3);
+    kb.diag_top = kb.x_top + (uint32_t)(pr.maxlt >> 3);
+    kb.x = bits_for(kb.x_top);
+    kb.diag = bits_for(kb.diag_top);
+    kb.target = bits_for((uint64_t)e->T.n);
+    kb.query = bits_for((uint64_t)e->Q.n);
+    kb.is_float = pr.int_path ? 0 : 1;
+    const int score_bits = pr.int_path ? bits_for((uint64_t)std::max<int64_t>(max_score, 1)) : 32;
+    const int key_bits = score_bits + kb.diag + kb.x + kb.target + kb.query + 7;
+    const int32_t* order = ib;  // hits in their final order
+    if (key_bits <= 64 && n <= kSmallHits) {
+        PW_LAUNCH(hit_small_kernel, 1, kSmallHits, 0, e->stream, h, (int)n, kb, ib, len, soff);
+        e->launches++;
+    } else {
+        if ((c = e->fk_a.reserve(e->stream, k8)) != cudaSuccess || (c = e->fk_t.reserve(e->stream, k8)) != cudaSuccess)
+            return c;
+        uint64_t *ka = e->fk_a.as<uint64_t>(), *kt = e->fk_t.as<uint64_t>();
+        size_t tmp = 0, stmp = 0;
+        if ((c = cub::DeviceRadixSort::SortPairs(nullptr, tmp, ka, kt, ia, ib, (int)n, 0, 64, e->stream)) != cudaSuccess ||
+            (c = cub::DeviceScan::ExclusiveSum(nullptr, stmp, len, soff, (int64_t)n, e->stream)) != cudaSuccess ||
+            (c = e->scan_tmp.reserve(e->stream, std::max<size_t>({tmp, stmp, 16}))) != cudaSuccess)
+            return c;
+        tmp = e->scan_tmp.bytes;
+        if (key_bits <= 64) {
+            PW_LAUNCH(hit_pack_kernel, grid, 256, 0, e->stream, h, n, kb, ka, ia);
+            e->launches++;
+            if ((c = cub::DeviceRadixSort::SortPairs(e->scan_tmp.p, tmp, ka, kt, ia, ib, (int)n, 0, key_bits, e->stream)) !=
+                cudaSuccess)
+                return c;
+        } else {
+            // three stable passes, least significant word first
+            if ((c = e->fk_b.reserve(e->stream, k8)) != cudaSuccess || (c = e->fk_c.reserve(e->stream, k8)) != cudaSuccess ||
+                (c = e->fk_g.reserve(e->stream, k8)) != cudaSuccess)
+                return c;
+            uint64_t *kbw = e->fk_b.as<uint64_t>(), *kc = e->fk_c.as<uint64_t>(), *kg = e->fk_g.as<uint64_t>();
+            PW_LAUNCH(hit_key_kernel, grid, 256, 0, e->stream, h, n, ka, kbw, kc, ia);
+            if ((c = cub::DeviceRadixSort::SortPairs(e->scan_tmp.p, tmp, kc, kt, ia, ib, (int)n, 0, 64, e->stream)) !=
+                cudaSuccess)
+                return c;
+            PW_LAUNCH(gather_key_kernel, grid, 256, 0, e->stream, kbw, ib, n, kg);
+            tmp = e->scan_tmp.bytes;
+            if ((c = cub::DeviceRadixSort::SortPairs(e->scan_tmp.p, tmp, kg, kt, ib, ia, (int)n, 0, 64, e->stream)) !=
+                cudaSuccess)
+                return c;
+            PW_LAUNCH(gather_key_kernel, grid, 256, 0, e->stream, ka, ia, n, kg);
+            tmp = e->scan_tmp.bytes;
+            if ((c = cub::DeviceRadixSort::SortPairs(e->scan_tmp.p, tmp, kg, kt, ia, ib, (int)n, 0, 64, e->stream)) !=
+                cudaSuccess)
+                return c;
+            e->launches += 3;
+        }
+        // string offsets in the final order
+        PW_LAUNCH(hit_len_kernel, grid, 256, 0, e->stream, h, order, n, len);
+        e->launches++;
+        stmp = e->scan_tmp.bytes;
+        if ((c = cub::DeviceScan::ExclusiveSum(e->scan_tmp.p, stmp, len, soff, (int64_t)n, e->stream)) != cudaSuccess)
+            return c;
+    }
+    PW_LAUNCH(hit_out_kernel, grid, 256, 0, e->stream, h, order, soff, n, e->acc_ops.as<char>(), e->q_raw.as<uint8_t>(),
               e->q_raw_off.as<int64_t>(), e->t_raw.as<uint8_t>(), e->t_raw_off.as<int64_t>(), e->f_out.as<pw_hit>(),
               e->f_str.as<char>());
-    {
-        const int wgrid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 127) / 128, (int64_t)e->sm_count * 16));
-        PW_LAUNCH(hit_strings_warp_kernel, wgrid, 128, 0, e->stream, h, ib, soff, n, e->acc_ops.as<char>(),
-                  e->q_raw.as<uint8_t>(), e->q_raw_off.as<int64_t>(), e->t_raw.as<uint8_t>(),
+    e->launches++;
+    const int64_t longest = std::min(pr.maxlq + pr.maxlt, n_ops);  // no hit has more columns
+    if (longest > kWarpStringCols) {
+        const int64_t warps = (int64_t)e->sm_count * 64;
+        const int group = (int)std::max<int64_t>(1, std::min<int64_t>(kWarp, n / warps));
+        const int wgrid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 4 * group - 1) / (4 * group), warps / 4));
+        PW_LAUNCH(hit_strings_warp_kernel, wgrid, 128, 0, e->stream, h, order, soff, len, n, group,
+                  e->acc_ops.as<char>(), e->q_raw.as<uint8_t>(), e->q_raw_off.as<int64_t>(), e->t_raw.as<uint8_t>(),
                   e->t_raw_off.as<int64_t>(), e->f_str.as<char>());
+        e->launches++;
     }
-    e->launches += 6;  // this library's kernels (the CUB sorts and scan are not counted)
+    if (longest > kBlockStringCols) {
+        PW_LAUNCH(hit_strings_block_kernel, (int)std::min<int64_t>(n, (int64_t)e->sm_count * 4), 512, 0, e->stream, h,
+                  order, soff, len, n, e->acc_ops.as<char>(), e->q_raw.as<uint8_t>(), e->q_raw_off.as<int64_t>(),
+                  e->t_raw.as<uint8_t>(), e->t_raw_off.as<int64_t>(), e->f_str.as<char>());
+        e->launches++;
+    }
     if ((c = cudaGetLastError()) != cudaSuccess) return c;
     if (!e->h_hits.resize((size_t)n) || !e->h_strings.resize((size_t)total)) return cudaErrorMemoryAllocation;
     if ((c = copy_d2h(e, e->h_hits.data(), e->f_out.p, (size_t)n * sizeof(pw_hit))) != cudaSuccess ||
@@ -3032,7 +3069,7 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
     // (pw_finish.cuh), then both to the host
     const double t_finish = wall_ms();
     int64_t str_bytes = 0;
-    if ((c = finish_hits(e, acc_n, &str_bytes)) != cudaSuccess) return cuda_fail(e, c, "order hits");
+    if ((c = finish_hits(e, acc_n, acc_ops, max_pass, &str_bytes)) != cudaSuccess) return cuda_fail(e, c, "order hits");
     ht.mark("hit order + strings");
     inf.starting_points = total_starts;
     inf.hits = (int64_t)e->h_hits.size();
