@@ -284,7 +284,14 @@ struct pw_engine {
     HostBuf<int64_t> h_sel;
     HostBuf<int32_t> h_ptq, h_p2order;  // phase-2 pair lists (kept across calls: no page faults, no zero fill)
     HostBuf<uint8_t> h_stage[4];        // page-locked staging of the sets' blocks and tables (Staged)
-    HostBuf<uint8_t> h_seen;
+    HostBuf<uint8_t> h_small;           // page-locked landing place of small results (SmallReads)
+    std::vector<cudaEvent_t> idle_events;
+    struct Interval {                   // kernel time still to be read (settle_times)
+        cudaEvent_t a, b;
+        double* ms;
+    };
+    std::vector<Interval> intervals;
+    bool abort_unread = false;          // a band sweep was launched whose abort flag has not been read
     int64_t free_mem = 0;    // free device memory plus this engine's kept wave buffers, as last queried
     double free_mem_t = -1;  // wall_ms() of that query
     DevBuf chain_info, chain_prog, chain_max, chain_ring_off, chain_ring, chain_abort, p1_items, p1_grid;
@@ -371,6 +378,70 @@ static cudaError_t copy_d2h(pw_engine* e, void* dst, const void* src, size_t n) 
         if (_c != cudaSuccess) return cuda_fail(e, _c, what); \
     } while (0)
 
+// Small device results read together: one synchronisation, page-locked landing
+// place (a copy to pageable memory waits for the stream by itself, ~10 us each).
+struct SmallReads {
+    struct Item {
+        void* dst;
+        const void* src;
+        size_t n;
+    };
+    std::vector<Item> items;
+    void add(void* dst, const void* src, size_t n) { items.push_back({dst, src, n}); }
+    cudaError_t run(pw_engine* e) {
+        size_t total = 0;
+        for (const Item& it : items) total += (it.n + 15) & ~(size_t)15;
+        if (!e->h_small.resize(std::max<size_t>(total, 1024))) return cudaErrorMemoryAllocation;
+        size_t off = 0;
+        cudaError_t c;
+        for (const Item& it : items) {
+            if ((c = copy_d2h(e, e->h_small.data() + off, it.src, it.n)) != cudaSuccess) return c;
+            off += (it.n + 15) & ~(size_t)15;
+        }
+        if ((c = cudaStreamSynchronize(e->stream)) != cudaSuccess) return c;
+        off = 0;
+        for (const Item& it : items) {
+            std::memcpy(it.dst, e->h_small.data() + off, it.n);
+            off += (it.n + 15) & ~(size_t)15;
+        }
+        return cudaSuccess;
+    }
+};
+
+// Kernel times: an interval's events are recorded around its launches and read
+// after the next synchronisation (settle_times), so that timing costs no
+// synchronisation of its own.
+static cudaEvent_t idle_event(pw_engine* e) {
+    cudaEvent_t ev = nullptr;
+    if (!e->idle_events.empty()) {
+        ev = e->idle_events.back();
+        e->idle_events.pop_back();
+    } else {
+        cudaEventCreate(&ev);
+    }
+    return ev;
+}
+static cudaEvent_t time_from(pw_engine* e) {
+    const cudaEvent_t ev = idle_event(e);
+    cudaEventRecord(ev, e->stream);
+    return ev;
+}
+static void time_until(pw_engine* e, cudaEvent_t from, double* ms) {
+    const cudaEvent_t ev = idle_event(e);
+    cudaEventRecord(ev, e->stream);
+    e->intervals.push_back({from, ev, ms});
+}
+// After a synchronisation: adds the intervals' times to their sums.
+static void settle_times(pw_engine* e, bool read = true) {
+    for (const pw_engine::Interval& i : e->intervals) {
+        float ms = 0;
+        if (read && cudaEventElapsedTime(&ms, i.a, i.b) == cudaSuccess && i.ms) *i.ms += ms;
+        e->idle_events.push_back(i.a);
+        e->idle_events.push_back(i.b);
+    }
+    e->intervals.clear();
+}
+
 extern "C" int pw_create(int device, pw_engine** out) {
     if (!out) return PW_ERR_ARG;
     *out = nullptr;
@@ -403,6 +474,8 @@ extern "C" void pw_destroy(pw_engine* e) {
     if (!e) return;
     cudaSetDevice(e->device);
     if (e->stream) cudaStreamSynchronize(e->stream);
+    settle_times(e, false);
+    for (cudaEvent_t ev : e->idle_events) cudaEventDestroy(ev);
     for (auto& ev : e->ev)
         if (ev) cudaEventDestroy(ev);
     if (e->stream) cudaStreamDestroy(e->stream);
@@ -779,12 +852,10 @@ static int prepare_set(pw_engine* e, const HostSeqs& S, const SetBuffers& B, flo
         PW_LAUNCH(present_kernel, grid, 256, 0, e->stream, (const uint8_t*)B.raw_buf->as<uint8_t>(), (int64_t)raw_bytes,
                   e->seen_flags.as<uint8_t>());
         e->launches++;
-        if (!e->h_seen.resize(256)) return fail(e, PW_ERR_NOMEM, "host memory for the sequences");
-        if ((c = cudaGetLastError()) != cudaSuccess ||
-            (c = copy_d2h(e, e->h_seen.data(), e->seen_flags.p, 256)) != cudaSuccess ||
-            (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
+        SmallReads r;
+        r.add(seen, e->seen_flags.p, 256);
+        if ((c = cudaGetLastError()) != cudaSuccess || (c = r.run(e)) != cudaSuccess)
             return cuda_fail(e, c, "residues present");
-        std::memcpy(seen, e->h_seen.data(), 256);
     } else {
         for (size_t k = 0; k < raw_bytes; ++k) seen[S.raw[k]] = 1;
     }
@@ -944,12 +1015,12 @@ static KernelArgs base_args(pw_engine* e) {
 // Launches a sweep phase over items already sorted by strip class and uploaded
 // as one array; class c covers [cls_begin[c], cls_begin[c + 1]).  Each class
 // gets its own work counter, so there is no host synchronisation in between.
-// Kernel time per launch is accumulated into *kernel_ms after the phase.
+// Kernel time per launch is accumulated into *kernel_ms at the next
+// settle_times; nothing here waits for the launches.
 template <int PH>
 static int run_phase(pw_engine* e, KernelArgs A, const WorkItem* dev_items, const int (&cls_begin)[kNumClasses + 1],
                      int xmax_multi4, double* kernel_ms, int* n_launch, bool trans = false) {
     cudaError_t c;
-    std::vector<std::pair<cudaEvent_t, cudaEvent_t>> evs;
     if (cls_begin[kS32Multi + 1] > cls_begin[kS32Multi]) {
         // one boundary slot per resident warp (at most 16 blocks of 4 warps per SM)
         const int64_t slot = (int64_t)xmax_multi4 * kWarp;
@@ -967,27 +1038,15 @@ static int run_phase(pw_engine* e, KernelArgs A, const WorkItem* dev_items, cons
         if (n <= 0) continue;
         A.items = dev_items + cls_begin[cls];
         A.n_items = n;
-        cudaEvent_t a, b;
-        cudaEventCreate(&a);
-        cudaEventCreate(&b);
-        cudaEventRecord(a, e->stream);
+        const cudaEvent_t from = time_from(e);
         if constexpr (PH == 3)
             c = launch_class<int, 3>(e, cls, false, A, e->counter.as<int>() + cls, trans);
         else
             c = e->pr.int_path ? launch_class<int, PH>(e, cls, e->affine, A, e->counter.as<int>() + cls, trans)
                                : launch_class<float, PH>(e, cls, e->affine, A, e->counter.as<int>() + cls, trans);
-        cudaEventRecord(b, e->stream);
-        evs.push_back({a, b});
+        time_until(e, from, kernel_ms);
         if (c != cudaSuccess) return cuda_fail(e, c, "sweep kernel launch");
         if (n_launch) ++*n_launch;
-    }
-    if ((c = cudaStreamSynchronize(e->stream)) != cudaSuccess) return cuda_fail(e, c, "sweep kernel");
-    for (auto& ab : evs) {
-        float ms = 0;
-        cudaEventElapsedTime(&ms, ab.first, ab.second);
-        if (kernel_ms) *kernel_ms += ms;
-        cudaEventDestroy(ab.first);
-        cudaEventDestroy(ab.second);
     }
     return PW_OK;
 }
@@ -1353,10 +1412,7 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
             (c = cudaMemsetAsync(e->chain_abort.p, 0, sizeof(int), e->stream)) != cudaSuccess)
             return cuda_fail(e, c, "clear chain state");
     }
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    cudaEventRecord(a, e->stream);
+    const cudaEvent_t from = time_from(e);
     for (int k = 0; k < kNumClasses; ++k) {
         const int n = begin[k + 1] - begin[k];
         if (n <= 0) continue;
@@ -1403,19 +1459,12 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
         if (c != cudaSuccess) return cuda_fail(e, c, "score16 launch");
         inf.score_launches++;
     }
-    cudaEventRecord(b, e->stream);
+    time_until(e, from, &inf.score_kernel_ms);
     int status[2] = {0, 0};  // overflow count, chain abort flag
-    if ((c = copy_d2h(e, &status[0], S.ovf_count, sizeof(int))) != cudaSuccess ||
-        (chained &&
-         (c = copy_d2h(e, &status[1], e->chain_abort.p, sizeof(int))) !=
-             cudaSuccess) ||
-        (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
-        return cuda_fail(e, c, "read score status");
-    float ms = 0;
-    cudaEventElapsedTime(&ms, a, b);
-    inf.score_kernel_ms += ms;
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
+    SmallReads rd;
+    rd.add(&status[0], S.ovf_count, sizeof(int));
+    if (chained) rd.add(&status[1], e->chain_abort.p, sizeof(int));
+    if ((c = rd.run(e)) != cudaSuccess) return cuda_fail(e, c, "read score status");
     if (status[1]) return fail(e, PW_ERR_KERNEL, "chained score sweep: a strip waited too long for its predecessor");
     // the maxima stay on the device (pruning reads them there); the host
     // copy is needed only to find the pairs that reached the 16-bit limit
@@ -1632,6 +1681,8 @@ static int block_warps(int warp_smem) {
 // pairs (cell codes), 2: the same storing H (linear gap), 3: the checkpoint
 // sweep of the tile form (linear gap, checkpoints into tile_ck); 0: pair
 // maxima into band_out (indexed by BandPair.slot).
+// DIRS 1 to 3 do not wait for the launch: the caller reads the abort flag with
+// its next results (abort_unread).
 template <int DIRS>
 static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pairs, double* kernel_ms,
                           int* n_launch) {
@@ -1719,24 +1770,21 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
     B.ck = DIRS == 3 ? e->tile_ck.as<int>() : nullptr;
     B.wait_ns = wait_limit(e);
     const int grid = std::max(1, std::min(grid_cap(e, per_sm), (int)((n + bw - 1) / bw)));
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    cudaEventRecord(a, e->stream);
+    const cudaEvent_t from = time_from(e);
     PW_LAUNCH(kern, grid, bw * kWarp, smem, e->stream, A, B);
     e->launches++;
-    cudaEventRecord(b, e->stream);
-    if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "band sweep launch");
-    int aborted = 0;
-    if ((c = copy_d2h(e, &aborted, e->chain_abort.p, sizeof(int))) != cudaSuccess ||
-        (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
-        return cuda_fail(e, c, "band sweep");
-    float ms = 0;
-    cudaEventElapsedTime(&ms, a, b);
-    if (kernel_ms) *kernel_ms += ms;
+    time_until(e, from, kernel_ms);
     if (n_launch) ++*n_launch;
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
+    if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "band sweep launch");
+    if (DIRS != 0) {
+        e->abort_unread = true;
+        return PW_OK;
+    }
+    int aborted = 0;
+    SmallReads rd;
+    rd.add(&aborted, e->chain_abort.p, sizeof(int));
+    if ((c = rd.run(e)) != cudaSuccess) return cuda_fail(e, c, "band sweep");
+    settle_times(e);
     if (aborted) return fail(e, PW_ERR_KERNEL, "band sweep: a band waited too long for the band above");
     return PW_OK;
 }
@@ -1812,24 +1860,17 @@ static int run_band_ck_phase(pw_engine* e, KernelArgs A, const std::vector<BandC
     B.limit = limit;
     B.wait_ns = wait_limit(e);
     const int grid = std::max(1, std::min(grid_cap(e, per_sm), (int)((n + bw - 1) / bw)));
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    cudaEventRecord(a, e->stream);
+    const cudaEvent_t from = time_from(e);
     PW_LAUNCH(kern, grid, bw * kWarp, smem, e->stream, A, B);
     e->launches++;
-    cudaEventRecord(b, e->stream);
+    time_until(e, from, kernel_ms);
+    if (n_launch) ++*n_launch;
     if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "band sweep launch");
     int aborted = 0;
-    if ((c = copy_d2h(e, &aborted, e->chain_abort.p, sizeof(int))) != cudaSuccess ||
-        (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
-        return cuda_fail(e, c, "band sweep");
-    float ms = 0;
-    cudaEventElapsedTime(&ms, a, b);
-    if (kernel_ms) *kernel_ms += ms;
-    if (n_launch) ++*n_launch;
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
+    SmallReads rd;
+    rd.add(&aborted, e->chain_abort.p, sizeof(int));
+    if ((c = rd.run(e)) != cudaSuccess) return cuda_fail(e, c, "band sweep");
+    settle_times(e);
     if (aborted) return fail(e, PW_ERR_KERNEL, "band sweep: a band waited too long for the band above");
     return PW_OK;
 }
@@ -1857,10 +1898,7 @@ static int run_tile_cands(pw_engine* e, KernelArgs A, TileArgs T, const TilePair
         (c = cudaFuncSetAttribute(tile_cand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tsmem)) != cudaSuccess)
         return cuda_fail(e, c, "tile kernels smem");
     int* cnt = e->tile_cnt.as<int>();
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    cudaEventRecord(a, e->stream);
+    const cudaEvent_t from = time_from(e);
     const int n = (int)list.size();
     PW_LAUNCH(tile_select_kernel, n, 256, 0, e->stream, A, T, dev_list, e->tile_sel.as<int2>(), cnt, (int)tiles);
     int per_sm = 0;
@@ -1870,15 +1908,9 @@ static int run_tile_cands(pw_engine* e, KernelArgs A, TileArgs T, const TilePair
               (const int2*)e->tile_sel.as<int2>(), (const int*)cnt, cnt + 1);
     PW_LAUNCH(tile_cand_count_kernel, (n + 127) / 128, 128, 0, e->stream, A, dev_list, n);
     e->launches += 3;
-    cudaEventRecord(b, e->stream);
-    if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "tile candidates launch");
-    if ((c = cudaEventSynchronize(b)) != cudaSuccess) return cuda_fail(e, c, "tile candidates");
-    float ms = 0;
-    cudaEventElapsedTime(&ms, a, b);
-    if (kernel_ms) *kernel_ms += ms;
+    time_until(e, from, kernel_ms);
     if (n_launch) *n_launch += 3;
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
+    if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "tile candidates launch");
     return PW_OK;
 }
 
@@ -1919,6 +1951,11 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
     if (!e->Q.set || !e->T.set) return fail(e, PW_ERR_STATE, "queries and targets must be set");
     if (cudaSetDevice(e->device) != cudaSuccess) return fail(e, PW_ERR_DEVICE, "cudaSetDevice failed");
     e->err.clear();
+    if (!e->intervals.empty()) {  // left by a call that failed
+        cudaStreamSynchronize(e->stream);
+        settle_times(e, false);
+    }
+    e->abort_unread = false;
     e->h_hits.clear();
     e->h_strings.clear();
     e->h_starts.clear();
@@ -2190,14 +2227,10 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         cudaEventElapsedTime(&ms, e->ev[0], e->ev[1]);
         inf.score_ms = ms;
     } else if (use_s16) {
-        cudaEventRecord(e->ev[0], e->stream);
+        const cudaEvent_t from = time_from(e);
         rc = phase1_s16(e, A, inf, flags);
         if (rc != PW_OK) return rc;
-        cudaEventRecord(e->ev[1], e->stream);
-        cudaStreamSynchronize(e->stream);
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e->ev[0], e->ev[1]);
-        inf.score_ms = ms;
+        time_until(e, from, &inf.score_ms);
         ht0.mark("score phase (16-bit, wall)");
     } else {
         inf.score_path = 1;
@@ -2234,7 +2267,7 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         int xm = 4;
         for (int k = begin[kS32Multi]; k < begin[kS32Multi + 1]; ++k) xm = std::max(xm, (int)align_up(it2[k].xmax, 4));
         if ((c = upload(e, e->items, it2)) != cudaSuccess) return cuda_fail(e, c, "upload items");
-        cudaEventRecord(e->ev[0], e->stream);
+        const cudaEvent_t from = time_from(e);
         if (plain) {
             // the unbatched form: one launch per (query, target) pair
             for (size_t k = 0; k < it2.size(); ++k) {
@@ -2243,17 +2276,17 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
                 rc = run_phase<1>(e, A, e->items.as<WorkItem>() + k, b1, xm, &inf.score_kernel_ms,
                                   &inf.score_launches);
                 if (rc != PW_OK) return rc;
+                if ((c = cudaStreamSynchronize(e->stream)) != cudaSuccess) return cuda_fail(e, c, "score sweep");
+                settle_times(e);
             }
         } else {
             rc = run_phase<1>(e, A, e->items.as<WorkItem>(), begin, xm, &inf.score_kernel_ms, &inf.score_launches);
             if (rc != PW_OK) return rc;
         }
-        cudaEventRecord(e->ev[1], e->stream);
-        if ((c = cudaEventSynchronize(e->ev[1])) != cudaSuccess) return cuda_fail(e, c, "score sweep");
+        time_until(e, from, &inf.score_ms);
+        if ((c = cudaStreamSynchronize(e->stream)) != cudaSuccess) return cuda_fail(e, c, "score sweep");
+        settle_times(e);
         e->pm_stale = true;
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e->ev[0], e->ev[1]);
-        inf.score_ms = ms;
     }
     if ((band1 || plain_band) && !pair_mode) {
         // the band sweep wrote host maxima only: the trace kernels read them on the device
@@ -2273,6 +2306,7 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
             return cuda_fail(e, c, "upload pair maxima");
     }
     if (flags & PW_FLAG_SCORE_ONLY) {
+        settle_times(e);
         inf.kernel_launches = (int32_t)e->launches;
         inf.total_ms = wall_ms() - t_call;
         inf.h2d_bytes = e->h2d;
@@ -2312,10 +2346,11 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
                   e->q_trace_set ? (const uint8_t*)e->q_trace.as<uint8_t>() : (const uint8_t*)nullptr,
                   e->prune_flags.as<uint8_t>(), e->prune_cnt.as<unsigned long long>());
         e->launches++;
-        if ((c = cudaGetLastError()) != cudaSuccess ||
-            (c = copy_d2h(e, cnt, e->prune_cnt.p, sizeof(cnt))) != cudaSuccess ||
-            (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
+        SmallReads rd;
+        rd.add(cnt, e->prune_cnt.p, sizeof(cnt));
+        if ((c = cudaGetLastError()) != cudaSuccess || (c = rd.run(e)) != cudaSuccess)
             return cuda_fail(e, c, "prune pairs");
+        settle_times(e);
         min_pass = (int64_t)cnt[0];
         n_pass = (int64_t)cnt[1];
         max_pass = (int64_t)cnt[3];
@@ -2425,10 +2460,9 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         PW_LAUNCH(group_bound_kernel, g2, 256, 0, e->stream, (const int32_t*)e->q_count.as<int32_t>(), nq,
                   e->q_len.as<int32_t>(), per_item, e->prune_cnt.as<unsigned long long>());
         e->launches += 2;
-        if ((c = cudaGetLastError()) != cudaSuccess ||
-            (c = copy_d2h(e, &lb_units, e->prune_cnt.p, sizeof(lb_units))) !=
-                cudaSuccess ||
-            (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
+        SmallReads rd;
+        rd.add(&lb_units, e->prune_cnt.p, sizeof(lb_units));
+        if ((c = cudaGetLastError()) != cudaSuccess || (c = rd.run(e)) != cudaSuccess)
             return cuda_fail(e, c, "query counts");
         const double lb_q = (double)lb_units * tmin;
         if (lb_q < cost_t) {
@@ -2720,7 +2754,7 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         Aw.cand_base = A.cand_base;
         Aw.cand_cap = A.cand_cap;
         Aw.n_cand = A.n_cand;
-        cudaEventRecord(e->ev[0], e->stream);
+        const cudaEvent_t trace_from = time_from(e);
         if ((c = cudaMemsetAsync(A.n_cand, 0, n_pairs * sizeof(int32_t), e->stream)) != cudaSuccess)
             return cuda_fail(e, c, "reset candidate counts");
         if (!wi.empty()) {
@@ -2748,10 +2782,15 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         PW_LAUNCH(cand_overflow_kernel, gslot, 256, 0, e->stream, (const int32_t*)A.n_cand, (const int32_t*)A.cand_cap,
                   n_pairs, e->prune_cnt.as<unsigned long long>());
         e->launches++;
-        if ((c = copy_d2h(e, &n_over, e->prune_cnt.p, sizeof(n_over))) !=
-                cudaSuccess ||
-            (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
-            return cuda_fail(e, c, "candidate overflow count");
+        int aborted = 0;
+        {
+            SmallReads rd;
+            rd.add(&n_over, e->prune_cnt.p, sizeof(n_over));
+            if (e->abort_unread) rd.add(&aborted, e->chain_abort.p, sizeof(int));
+            if ((c = rd.run(e)) != cudaSuccess) return cuda_fail(e, c, "direction sweep");
+            e->abort_unread = false;
+        }
+        if (aborted) return fail(e, PW_ERR_KERNEL, "band sweep: a band waited too long for the band above");
         ht.mark("direction sweep");
         std::vector<int32_t> ncand;
         std::vector<int64_t> cbase;
@@ -2828,6 +2867,13 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
                      : hstore  ? run_band_phase<2>(e, Aw, bp, &inf.trace_kernel_ms, &inf.trace_launches)
                                : run_band_phase<1>(e, Aw, bp, &inf.trace_kernel_ms, &inf.trace_launches);
                 if (rc != PW_OK) return rc;
+                if (e->abort_unread) {  // before anything walks the codes
+                    SmallReads rd;
+                    rd.add(&aborted, e->chain_abort.p, sizeof(int));
+                    if ((c = rd.run(e)) != cudaSuccess) return cuda_fail(e, c, "band sweep");
+                    e->abort_unread = false;
+                    if (aborted) return fail(e, PW_ERR_KERNEL, "band sweep: a band waited too long for the band above");
+                }
             }
         }
 
@@ -2928,15 +2974,18 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
                                                     cub::Sum(), (int64_t)0, (int)n_pairs, e->stream)) != cudaSuccess)
                 return cuda_fail(e, c, "scan start counts");
         }
-        cudaEventRecord(e->ev[2], e->stream);
+        time_until(e, trace_from, &trace_ms);
+        const cudaEvent_t walk_from = time_from(e);
         int64_t last_off = 0;
         int32_t last_n = 0;
         unsigned long long tile_bound = 0;  // tile form: bytes of operations its walks can reserve at most
-        if ((c = copy_d2h(e, &last_off, e->start_off.as<int64_t>() + n_pairs - 1, sizeof(int64_t))) != cudaSuccess ||
-            (c = copy_d2h(e, &last_n, TA.n_starts + n_pairs - 1, sizeof(int32_t))) != cudaSuccess ||
-            (n_tile > 0 && (c = copy_d2h(e, &tile_bound, TT.ops_bound, sizeof(tile_bound))) != cudaSuccess) ||
-            (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
-            return cuda_fail(e, c, "collect");
+        {
+            SmallReads rd;
+            rd.add(&last_off, e->start_off.as<int64_t>() + n_pairs - 1, sizeof(int64_t));
+            rd.add(&last_n, TA.n_starts + n_pairs - 1, sizeof(int32_t));
+            if (n_tile > 0) rd.add(&tile_bound, TT.ops_bound, sizeof(tile_bound));
+            if ((c = rd.run(e)) != cudaSuccess) return cuda_fail(e, c, "collect");
+        }
         // the tile walks spell their hits' operations themselves unless that
         // bound is large (more than 1 GiB); else tile_ops_kernel walks the
         // hits again
@@ -2956,11 +3005,12 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
             if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "gather launch");
             if (!e->h_starts.resize_keep(first_rec + (size_t)wave_starts))
                 return fail(e, PW_ERR_NOMEM, "host memory for the starting points");
-            if ((c = copy_d2h(e, e->h_starts.data() + first_rec, e->starts.p, wave_starts * sizeof(StartRec))) != cudaSuccess ||
-                (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
+            if ((c = copy_d2h(e, e->h_starts.data() + first_rec, e->starts.p, wave_starts * sizeof(StartRec))) != cudaSuccess)
                 return cuda_fail(e, c, "copy starts");
         }
         total_starts += wave_starts;
+        if (start_cap >= 0 && total_starts >= start_cap && (c = cudaStreamSynchronize(e->stream)) != cudaSuccess)
+            return cuda_fail(e, c, "copy starts");  // the host reads them below
         ht.mark("starting points");
         TA.allowed = nullptr;
         if (start_cap >= 0 && total_starts >= start_cap) {
@@ -3015,13 +3065,13 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
                 e->launches++;
             }
             if ((c = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, c, "walk launch");
-            std::vector<int64_t> cnt;
-            if ((c = download(e, cnt, TA.hit_count, 2)) != cudaSuccess) return cuda_fail(e, c, "walk");
-            const int nh = (int)std::min<int64_t>((int32_t)(cnt[0] & 0xffffffff), wave_starts);
+            int64_t cnt[2] = {0, 0};
             unsigned long long tile_ops_n = 0;
-            if (TT.ops && (c = copy_d2h(e, &tile_ops_n, TT.ops_total, sizeof(tile_ops_n))) != cudaSuccess)
-                return cuda_fail(e, c, "walk");
-            if (TT.ops && (c = cudaStreamSynchronize(e->stream)) != cudaSuccess) return cuda_fail(e, c, "walk");
+            SmallReads rd;
+            rd.add(cnt, TA.hit_count, sizeof(cnt));
+            if (TT.ops) rd.add(&tile_ops_n, TT.ops_total, sizeof(tile_ops_n));
+            if ((c = rd.run(e)) != cudaSuccess) return cuda_fail(e, c, "walk");
+            const int nh = (int)std::min<int64_t>((int32_t)(cnt[0] & 0xffffffff), wave_starts);
             const int64_t strip_end = cnt[1];
             const int64_t ops_end = strip_end + (int64_t)tile_ops_n;
             if (nh) {
@@ -3055,14 +3105,12 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
                 acc_ops = ops_end;
             }
         }
-        cudaEventRecord(e->ev[3], e->stream);
-        cudaStreamSynchronize(e->stream);
+        time_until(e, walk_from, &walk_ms);
         ht.mark("walk");
-        float t1 = 0, t2 = 0;
-        cudaEventElapsedTime(&t1, e->ev[0], e->ev[2]);
-        cudaEventElapsedTime(&t2, e->ev[2], e->ev[3]);
-        trace_ms += t1;
-        walk_ms += t2;
+        if (wv + 1 < waves.size()) {  // the next wave reuses this one's buffers and staging
+            if ((c = cudaStreamSynchronize(e->stream)) != cudaSuccess) return cuda_fail(e, c, "walk");
+            settle_times(e);
+        }
     }
 
     // hits in the reference's HitList order and their strings, on the device
@@ -3070,6 +3118,8 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
     const double t_finish = wall_ms();
     int64_t str_bytes = 0;
     if ((c = finish_hits(e, acc_n, acc_ops, max_pass, &str_bytes)) != cudaSuccess) return cuda_fail(e, c, "order hits");
+    if (acc_n == 0 && (c = cudaStreamSynchronize(e->stream)) != cudaSuccess) return cuda_fail(e, c, "walk");
+    settle_times(e);
     ht.mark("hit order + strings");
     inf.starting_points = total_starts;
     inf.hits = (int64_t)e->h_hits.size();
