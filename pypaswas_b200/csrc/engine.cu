@@ -1806,7 +1806,9 @@ static int run_band_ck_phase(pw_engine* e, KernelArgs A, const std::vector<BandC
     int per_sm = 0;
     if ((c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bw * kWarp, smem)) != cudaSuccess)
         return cuda_fail(e, c, "occupancy");
-    per_sm = std::max(1, std::min(per_sm, 16));
+    int64_t bands = 0;
+    for (const BandCk& p : pairs) bands += std::max(1, p.nbands);
+    per_sm = std::max(1, std::min(per_sm, band_ck_sm_warps(bands, e->sm_count) / bw));
     const int warps = grid_cap(e, per_sm) * bw;
     std::vector<int> order(pairs.size());
     std::iota(order.begin(), order.end(), 0);

@@ -26,6 +26,18 @@
 // storing warp for the latency of its outstanding stores each time).  Each
 // poll is bounded in time, as every wait here.
 //
+// Blocks per SM (kBandCkBlocks, band_ck_sm_warps).  A chain goes at the pace of
+// its slowest band, the one whose SM sub-partition has most warps at work, and
+// one warp alone keeps the ALU pipe three quarters busy: with 4 blocks of 4
+// warps an SM, bands waited for the band above 40% of their time and the pipe
+// was 66% busy.  64 pairs of 10 to 50 kb (3900 bands): 17.6 ms with 4 blocks,
+// 15.9 with 3, 15.1 with 2, 17.4 with 1.  With few bands one block an SM is
+// better, all bands then going at one pace; pairs of 20 to 30 kb with 1 and 2
+// blocks: 8 pairs 2.7 and 4.2 ms, 16 3.7 and 4.6, 24 (2350 bands) 5.1 and 5.3,
+// 32 (3100) 6.9 and 6.7; the line is drawn at four bands a warp.  Blocks of 8
+// columns a lane (half the steps, twice the skew) were slower: 16.1 ms for the
+// 64 pairs.
+//
 // Steps past a lane's ends run on padding codes: before its first block H
 // stays 0, after its last one it only decays, so no step is predicated except
 // the stores.
@@ -68,12 +80,16 @@ struct BandCkArgs {
 
 constexpr int kBlkCols = 4;   // columns a lane sweeps per step
 constexpr int kBlkGroup = 8;  // steps between two loads of the row above
+constexpr int kBandCkBlocks = 2; // blocks of 4 warps an SM at most
 constexpr int kBandCkLead = 48;  // planning lead between bands (steps): the lanes' skew, a group and the hand-over
 
 __host__ __device__ __forceinline__ int band_ck_warp_smem(int alpha1) {
     // profile, the row above's blocks, the tile's last column, its maxima, code words
     return alpha1 * 2 * kWarp * 16 + kBlkGroup * 16 + 2 * kWarp * 16 + kWarp * 4 + 2 * kWarp * 4;
 }
+
+// Warps in flight an SM for `bands` bands on `sms` SMs.
+inline int band_ck_sm_warps(int64_t bands, int sms) { return bands < (int64_t)4 * 4 * sms ? 4 : 4 * kBandCkBlocks; }
 
 __device__ __forceinline__ int lo16(uint32_t v) { return (int)(int16_t)(v & 0xffffu); }
 __device__ __forceinline__ int hi16(uint32_t v) { return (int)(int16_t)(v >> 16); }
@@ -106,7 +122,7 @@ __device__ __forceinline__ uint32_t ck_cell(uint32_t diag, uint32_t s, uint32_t 
 }
 
 template <bool PAIR>
-__global__ void __launch_bounds__(128, 4) band_ck_kernel(KernelArgs A, BandCkArgs B) {
+__global__ void __launch_bounds__(128, kBandCkBlocks) band_ck_kernel(KernelArgs A, BandCkArgs B) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
