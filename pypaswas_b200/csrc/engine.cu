@@ -780,7 +780,7 @@ static std::vector<int> listed_bytes(const uint8_t* seen) {
 
 // One sequence set on the device: residues as given, and the two encodings (the
 // host loops that wrote them, with two copies of the padded set over PCIe, took
-// 18 ms for 500,000 reads and 9 ms for 5.8 Mb of long DNA; 1.9 and 0.4 ms now) --
+// 18 ms for 500,000 reads and 9 ms for 5.8 Mb of long DNA; 6 and 0.3 ms now) --
 // compact codes (codes: the distinct residues numbered, padding coded as one
 // more) and matrix indices (res) -- written by encode_kernel, each sequence
 // 16-byte aligned and padded.  Queries and targets are prepared separately and
@@ -1705,6 +1705,11 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
     if ((c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bw * kWarp, smem)) != cudaSuccess)
         return cuda_fail(e, c, "occupancy");
     per_sm = std::max(1, std::min(per_sm, 16));
+    if (aff_ints) {
+        int64_t bands = 0;
+        for (const BandPair& p : pairs) bands += std::max(1, p.nbands);
+        per_sm = std::min(per_sm, std::max(1, band_affine_sm_warps(bands, (int64_t)pairs.size(), e->sm_count) / bw));
+    }
     const int warps = grid_cap(e, per_sm) * bw;
     // queue: the bands of each pair form a chain (pw_plan.h), longest pairs first
     std::vector<int> order(pairs.size());

@@ -49,6 +49,20 @@ __host__ __device__ __forceinline__ int band_affine_warp_smem(int alpha1) {
     // profile, the row above's blocks, code pairs of the last 64 blocks
     return alpha1 * kWarp * 8 + kAffGroup * 16 + 2 * kWarp * 2;
 }
+// Warps in flight an SM for `bands` bands of `pairs` pairs on `sms` SMs: a block
+// of 4 for each four bands a warp, up to the 4 that fit, and two at least for
+// short chains (fewer than 3 bands a pair).  A chain goes at the pace of its most
+// crowded band, so that more blocks than the bands need make all of them wait;
+// one warp alone keeps a sub-partition's ALU pipe 40% busy, four 85%.  Cell
+// codes, with 4 blocks and with 1 / 2, proteins of 2 to 8 thousand residues: 48
+// pairs (900 bands) 3.3 and 2.2 / 3.3 ms, 96 5.9 and 3.4 / 3.6, 200 (3600) 7.2
+// and 7.3 / 5.8, 300 9.3 and 10.4 / 8.9, 500 14.1 and 16.9 / 13.8; two bands a
+// pair: 1200 pairs .38 and .43 / .32; the 12,600 traced pairs of a 200 x 2000
+// protein batch 5.2 and 9.2 / 6.5.
+inline int band_affine_sm_warps(int64_t bands, int64_t pairs, int sms) {
+    const int64_t blocks = 1 + bands / (16 * sms);
+    return 4 * (int)std::min<int64_t>(bands < 3 * pairs ? std::max<int64_t>(blocks, 2) : blocks, 4);
+}
 // The epoch of a band's row: 1 .. 63, never that of bands b - 2 .. b - 124,
 // whose words its slot may still hold.
 __device__ __forceinline__ uint32_t affine_epoch(int band) { return 1u + (uint32_t)(band >> 1) % 63u; }

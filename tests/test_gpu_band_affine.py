@@ -103,3 +103,40 @@ def test_walks_with_many_candidates(engine_lib, oracle_mod, affine, limit):
         e.close()
     assert info.warp_pairs > 0 and info.starting_points > info.traced_pairs
     assert hits == ref["hits"]
+
+
+def test_many_chains(engine_lib, oracle_mod):
+    """More bands than warps in flight with one block an SM (two and more blocks,
+    warps that take band after band): maxima and hits of a sample."""
+    st = cases.Settings(matrix_name="BLOSUM62", gap_score="-11", gap_extension="-1", minimum_score="25",
+                        filter_factor="0.01")
+    score = scores.make_score(st)
+    rng = np.random.default_rng(77)
+
+    def rs(n):
+        return "".join(cases.PROTEIN[i] for i in rng.integers(0, len(cases.PROTEIN), n))
+
+    n = 900
+    q = [rs(int(rng.integers(20, 60))) for _ in range(n)]
+    t = [rs(int(rng.integers(600, 1000))) for _ in range(8)]  # three or four bands
+    t = [s[:250] + q[k][:20] + s[270:510] + q[k + 8][:20] + s[530:] for k, s in enumerate(t)]
+    pairs = [(i, i % 8) for i in range(n)]
+    e = _native.Engine(0, lib=engine_lib)
+    try:
+        configure(e, score, st)
+        e.set_queries([s.encode() for s in q], np.arange(n))
+        e.set_targets([s.encode() for s in t], np.arange(8) + n)
+        e.set_pairs([a for a, _ in pairs], [b for _, b in pairs])
+        info = e.align()
+        pm = e.pair_max()
+        hits = decode_hits(*e.hits())
+    finally:
+        e.close()
+    assert info.score_path == 2
+    for k in [*range(16), *range(16, n, 59)]:
+        a, b = pairs[k]
+        ref = oracle_mod.run(cases.oracle_params(oracle_mod, score), [q[a]], [t[b]],
+                             cases.pos_scores(score, st, [q[a]], [t[b]]), float(st.minimum_score))
+        assert pm[a, b] == ref["pair_max"][0, 0]
+        assert [h for h in hits if (h["query"], h["target"]) == (a, b)] == \
+            [dict(h, query=a, target=b) for h in ref["hits"]]
