@@ -288,8 +288,9 @@ def roofline(e, w, score, infos, steps):
     sixteen = last["score_path"] == 0 and last["overflow_pairs"] == 0 and last["score_launches"] > 0
     if trace_ms >= score_ms:
         wp, tp = last["warp_pairs"], last["traced_pairs"]
-        which = "band_kernel, one pair per warp" if wp >= tp else (
-            "sweep_kernel phase 2" if wp == 0 else "sweep_kernel phase 2 + band_kernel")
+        band = "band_affine_kernel" if mode == "affine" else "band_kernel"
+        which = band + ", one pair per warp" if wp >= tp else (
+            "sweep_kernel phase 2" if wp == 0 else "sweep_kernel phase 2 + " + band)
         dom, dom_ms, launches = "direction sweep (%s)" % which, trace_ms, sum(i["trace_launches"] for i in infos)
         ops = sum(i["traced_cells"] for i in infos) * OPS_PER_CELL[(mode, "dirs")]
         per_cell = OPS_PER_CELL[(mode, "dirs")]
@@ -299,10 +300,10 @@ def roofline(e, w, score, infos, steps):
                1: "score sweep (sweep_kernel phase 1, 32-bit lanes)",
                2: "score sweep (band_kernel, bands chained across warps)"}.get(last["score_path"], "score sweep")
         if last["score_path"] == 2 and last.get("tile_pairs"):
-            dom = "score sweep (band_kernel, bands chained across warps, keeping the tile form's checkpoints)"
+            dom = "score sweep (band_ck_kernel, bands chained across warps, keeping the tile form's checkpoints)"
         if last["score_path"] == 2 and 2 * last.get("paired_cells", 0) >= last["cells"]:
             # most cells on the 16x2 band sweep: its DPX issue peak is the 16x2 one
-            dom = ("score sweep (band16_kernel: a pair and its reverse-complement pair in 16-bit halves, bands "
+            dom = ("score sweep (band_ck_kernel: a pair and its reverse-complement pair in 16-bit halves, bands "
                    "chained across warps, keeping the tile form's checkpoints)")
             sixteen = True
         dom_ms, launches = score_ms, sum(i["score_launches"] for i in infos)

@@ -11,6 +11,10 @@
 //   walk_kernel      the host walk of SmithWaterman._print_alignments
 //                    (SmithWaterman.py:699-838), one thread per pair
 //   ops_kernel       writes the column operations of every kept hit
+//   warp_collect_kernel, warp_walk_kernel, warp_ops_kernel
+//                    the same for the band sweep's pairs, one warp per pair
+//   present_kernel, encode_kernel
+//                    residues that occur in a set, and its two encodings
 #pragma once
 #include <type_traits>
 
