@@ -291,6 +291,7 @@ struct pw_engine {
         double* ms;
     };
     std::vector<Interval> intervals;
+    std::vector<cudaEvent_t> started;   // intervals without an end yet
     bool abort_unread = false;          // a band sweep was launched whose abort flag has not been read
     int64_t free_mem = 0;    // free device memory plus this engine's kept wave buffers, as last queried
     double free_mem_t = -1;  // wall_ms() of that query
@@ -424,14 +425,17 @@ static cudaEvent_t idle_event(pw_engine* e) {
 static cudaEvent_t time_from(pw_engine* e) {
     const cudaEvent_t ev = idle_event(e);
     cudaEventRecord(ev, e->stream);
+    e->started.push_back(ev);
     return ev;
 }
 static void time_until(pw_engine* e, cudaEvent_t from, double* ms) {
     const cudaEvent_t ev = idle_event(e);
     cudaEventRecord(ev, e->stream);
     e->intervals.push_back({from, ev, ms});
+    e->started.erase(std::find(e->started.begin(), e->started.end(), from));
 }
-// After a synchronisation: adds the intervals' times to their sums.
+// After a synchronisation: adds the intervals' times to their sums (read), or
+// forgets what a failed call left.
 static void settle_times(pw_engine* e, bool read = true) {
     for (const pw_engine::Interval& i : e->intervals) {
         float ms = 0;
@@ -440,6 +444,10 @@ static void settle_times(pw_engine* e, bool read = true) {
         e->idle_events.push_back(i.b);
     }
     e->intervals.clear();
+    if (!read) {
+        e->idle_events.insert(e->idle_events.end(), e->started.begin(), e->started.end());
+        e->started.clear();
+    }
 }
 
 extern "C" int pw_create(int device, pw_engine** out) {
@@ -1958,7 +1966,7 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
     if (!e->Q.set || !e->T.set) return fail(e, PW_ERR_STATE, "queries and targets must be set");
     if (cudaSetDevice(e->device) != cudaSuccess) return fail(e, PW_ERR_DEVICE, "cudaSetDevice failed");
     e->err.clear();
-    if (!e->intervals.empty()) {  // left by a call that failed
+    if (!e->intervals.empty() || !e->started.empty()) {  // left by a call that failed
         cudaStreamSynchronize(e->stream);
         settle_times(e, false);
     }
