@@ -1684,6 +1684,9 @@ static int block_warps(int warp_smem) {
     return 4 * warp_smem <= kBlockSmem ? 4 : 2 * warp_smem <= kBlockSmem ? 2 : 1;
 }
 
+// Boundary rows of a band sweep's pairs at most (two rows a pair are always given).
+constexpr int64_t kRingBytes = (int64_t)8 << 30;
+
 // Launches band_kernel over `pairs` (one warp per band, the bands of a pair
 // chained across warps, pw_band.cuh).  DIRS 1: the direction sweep of traced
 // pairs (cell codes), 2: the same storing H (linear gap), 3: the checkpoint
@@ -1739,14 +1742,42 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
         sorted[k] = pairs[order[k]];
         nstr[k] = sorted[k].nbands;
         xm[k] = steps[order[k]];
-        if constexpr (DIRS < 3) {
-            sorted[k].ring_off = ring_elems;
-            const int lq = e->pr.qlen[sorted[k].q];
-            if (sorted[k].nbands > 1) ring_elems += 2 * (int64_t)(aff_ints ? affine_blocks(lq) : lq);
+    }
+    // the pairs' boundary rows, `most` a pair at most
+    auto place_rings = [&](int most) {
+        int64_t elems = 0;
+        for (BandPair& p : sorted) {
+            const int lq = e->pr.qlen[p.q];
+            p.rows = aff_ints ? std::min(most, affine_ring_rows(p.nbands, warps)) : 2;
+            p.ring_off = elems;
+            if (p.nbands > 1) elems += p.rows * (int64_t)(aff_ints ? affine_blocks(lq) : lq);
+        }
+        return elems;
+    };
+    if constexpr (DIRS < 3) {
+        // two rows a pair where the rows that hold no band back take more than
+        // kRingBytes (or are not to be had): fewer bands of a pair run at a time
+        ring_elems = place_rings(INT32_MAX);
+        if (ring_elems > kRingBytes / (int64_t)sizeof(int4) ||
+            e->band_ring.reserve(e->stream, (size_t)std::max<int64_t>(ring_elems, 1) * sizeof(int4)) != cudaSuccess) {
+            cudaGetLastError();
+            ring_elems = place_rings(2);
         }
     }
     std::vector<int4> entries = band_queue(nstr, xm, warps, aff_ints ? kAffLead : kBandLead);
     const size_t n = entries.size();
+    if (aff_ints) {
+        // the band that must have finished before an entry's band reads its row above
+        for (int4& v : entries) v.w = -1;
+        std::vector<std::vector<int>> at;  // per pair: queue indices by band (queued in order)
+        for (size_t k = 0; k < n; ++k) {
+            const int pair = entries[k].x, hold = affine_hold(sorted[pair].rows);
+            if (sorted[pair].nbands <= hold) continue;
+            at.resize(sorted.size());
+            at[pair].push_back((int)k);
+            if (entries[k].y >= hold) entries[k].w = at[pair][entries[k].y - hold];
+        }
+    }
     if (e->tune[PW_TUNE_STALL_TEST]) {
         // one band below another waits on the spare flag (index n) instead
         for (int4& v : entries)

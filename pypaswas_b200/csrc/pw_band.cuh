@@ -84,14 +84,16 @@ struct BandPair {
     int32_t q, t;        // query / target index (reference orientation)
     int32_t nbands;
     int32_t meta_item;   // DIRS: value for PairMeta.item (the pair's work item in the wave)
-    int64_t ring_off;    // int4 offset of the pair's two boundary rows (2 x lq; affine: 2 x affine_blocks)
+    int32_t rows;        // boundary rows of the pair (affine integer sweep; two elsewhere)
+    int64_t ring_off;    // int4 offset of the pair's boundary rows (2 x lq; affine: rows x affine_blocks)
     int64_t dir_base;    // DIRS 1, 2: byte offset of the pair's cell codes; 3: int offset of its checkpoints
                          // (rows, then columns)
     int64_t slot;        // DIRS: pair slot (metas, candidates); score sweep: pair_max index
 };
 
 struct BandArgs {
-    const int4* entries;  // per queue entry: (pair, band, queue index of the band above, 0)
+    const int4* entries;  // per queue entry: (pair, band, queue index of the band above, affine integer
+                          // sweep: that of the band to be finished first, or -1)
     const BandPair* pairs;
     int n_entries;
     int* counter;

@@ -17,13 +17,14 @@
 // for only in a column whose maximum reaches the threshold.
 //
 // Handing a row down: lane 31 stores its bottom row block by block into the
-// pair's ring (two rows, alternating by band parity), each word with the
-// band's epoch in its top 6 bits; the ring is zeroed before the launch and an
-// epoch differs from the ones that the slot's earlier bands left there, so a
-// word that shows the epoch is valid by itself and neither side fences.  The
-// band below loads 16 blocks ahead and polls, bounded in time, while a word is
-// missing.  A row is overwritten by band b + 2 only in columns that band b + 1
-// has handed down, i.e. after it has read them.
+// pair's ring (band b: row b % rows), each word with the band's epoch in its top
+// 6 bits; the ring is zeroed before the launch.  A word that shows the epoch is
+// the band's, so neither side fences: the band below loads 16 blocks ahead and
+// polls, bounded in time, while a word is missing.  All bands of a pair may be
+// in flight together, so a band may poll a row whose band has not been taken
+// yet: rows, epochs and the wait of a band for an earlier one to finish (the
+// queue entry's w) are such that no word of another band ever shows the epoch
+// waited for (affine_hold, pw_plan.h).
 //   word 0 of a column: B (< 2^24) | (M <= 0) << 25 | epoch << 26
 //   word 1: Y of the row below + 2^24 | epoch << 26
 //
@@ -36,6 +37,7 @@
 #pragma once
 #include "pw_band.cuh"
 #include "pw_band_ck.cuh"
+#include "pw_plan.h"
 
 namespace pw {
 
@@ -63,9 +65,6 @@ inline int band_affine_sm_warps(int64_t bands, int64_t pairs, int sms) {
     const int64_t blocks = 1 + bands / (16 * sms);
     return 4 * (int)std::min<int64_t>(bands < 3 * pairs ? std::max<int64_t>(blocks, 2) : blocks, 4);
 }
-// The epoch of a band's row: 1 .. 63, never that of bands b - 2 .. b - 124,
-// whose words its slot may still hold.
-__device__ __forceinline__ uint32_t affine_epoch(int band) { return 1u + (uint32_t)(band >> 1) % 63u; }
 
 template <int DIRS>
 __global__ void __launch_bounds__(128, 4) band_affine_kernel(KernelArgs A, BandArgs B) {
@@ -87,7 +86,7 @@ __global__ void __launch_bounds__(128, 4) band_affine_kernel(KernelArgs A, BandA
         if (it >= B.n_entries) break;
         const int4 en = B.entries[it];
         const BandPair BP = B.pairs[en.x];
-        const int band = en.y, pred = en.z;
+        const int band = en.y, pred = en.z, held = en.w;
         const int q = BP.q, t = BP.t;
         const int lq = A.q.len[q], lt = A.t.len[t];
         const int nblk = affine_blocks(lq);
@@ -143,9 +142,14 @@ __global__ void __launch_bounds__(128, 4) band_affine_kernel(KernelArgs A, BandA
         __syncwarp();
         if (lane < kAffGroup) codes[lane] = (uint16_t)load_code(0);
         uint32_t code_n = load_code(kAffGroup);
-        const uint4* in = (const uint4*)B.ring + BP.ring_off + (int64_t)((band + 1) & 1) * nblk;
-        uint4* out = (uint4*)B.ring + BP.ring_off + (int64_t)(band & 1) * nblk;
-        const uint32_t ep_in = affine_epoch(band - 1) << 26, ep_out = affine_epoch(band) << 26;
+        // (the row of band 0 - 1 is not read)
+        const int rows = BP.rows;
+        const uint4* in = (const uint4*)B.ring + BP.ring_off + (int64_t)((band + rows - 1) % rows) * nblk;
+        uint4* out = (uint4*)B.ring + BP.ring_off + (int64_t)(band % rows) * nblk;
+        const uint32_t ep_in = (has_up ? affine_epoch(band - 1, rows) : 0u) << 26;
+        const uint32_t ep_out = affine_epoch(band, rows) << 26;
+        // an earlier band whose words must be gone from the row above
+        if (held >= 0 && chain_wait(B.progress + held, kChainDone, B.abort_flag, B.wait_ns) < 0) break;
         // the row above band 0 (and past the query): B = 0, Y = -inf
         const uint4 none = make_uint4(ep_in, ep_in, ep_in, ep_in);
         auto load_above = [&](int first) -> uint4 {

@@ -1,6 +1,7 @@
 // pw_plan.h -- host-side queue planning of the chained 16-bit score sweep
-// (score16_chain_kernel).  Plain C++, no CUDA: the plan is a pure function of
-// the items' shapes, so it is tested and timed without a GPU.
+// (score16_chain_kernel) and of the band sweeps, and the rules of the affine
+// band sweep's boundary rows.  Plain C++, no CUDA: pure functions of the items'
+// shapes, so they are tested and timed without a GPU.
 #pragma once
 #include <algorithm>
 #include <cstdint>
@@ -8,7 +9,36 @@
 #include <utility>
 #include <vector>
 
+#ifdef __CUDACC__
+#define PW_PLAN_HD __host__ __device__
+#else
+#define PW_PLAN_HD
+#endif
+
 namespace pw {
+
+// Boundary rows of the affine band sweep (pw_band_affine.cuh).  Band b hands its
+// bottom row down in row b % rows of its pair's ring, in words that show the
+// band's epoch (1 .. 63; 0 is a cleared word).  A row's earlier words are those
+// of bands b - rows, b - 2 rows, ...; the epoch comes round again after 63 of
+// them, with band b - 63 rows.  The band that reads b's row is b + 1, and it may
+// look at the row long before b has run.  So band c reads only after band
+// c - affine_hold(rows) = (c - 1) - 62 rows has finished: that one has then
+// written over every word of band (c - 1) - 63 rows.  A row is written over
+// where the band below has read it: band b + rows stores a column after the
+// bands b + 1 .. b + rows - 1 have handed it down one after another.
+constexpr int kAffineEpochs = 63;
+PW_PLAN_HD inline uint32_t affine_epoch(int band, int rows) { return 1u + (uint32_t)(band / rows) % kAffineEpochs; }
+PW_PLAN_HD inline int affine_hold(int rows) { return (kAffineEpochs - 1) * rows + 1; }
+
+// Rows of a pair of `nbands` bands with `warps` warps in flight: as many as let
+// no band be held back.  A warp has one band, a band finishes after the band
+// above, so that the unfinished bands of a pair are at most `warps` consecutive
+// ones; a pair with no more bands than affine_hold(2) needs two rows.
+inline int affine_ring_rows(int nbands, int warps) {
+    const int together = std::min(nbands, warps);
+    return std::max(2, (together - 1 + kAffineEpochs - 2) / (kAffineEpochs - 1));
+}
 
 struct PlanEntry {
     int32_t item;   // index of the source item (in the order given)
