@@ -1646,34 +1646,14 @@ static cudaError_t finish_hits(pw_engine* e, int64_t n, int64_t n_ops, int64_t m
     return cudaSuccess;
 }
 
-// Queue entries (pair, band, queue index of the band above) of band chains:
-// pair k has nbands[k] bands of steps[k] steps, pairs in priority order.
+// Queue entries (pair, band, queue index of the band above, 0) of band chains
+// (plan_band_queue).
 static std::vector<int4> band_queue(const std::vector<int>& nbands, const std::vector<int64_t>& steps, int warps,
                                     int lead) {
-    std::vector<int4> entries;
-    if ((int64_t)nbands.size() * 2 >= warps) {
-        // many pairs: band-major order (every band 0, then every band 1, ...,
-        // longest pairs first within a band); a band's predecessor was handed
-        // out at least a whole band generation earlier, so nobody waits long
-        int maxb = 0;
-        for (int nb : nbands) maxb = std::max(maxb, nb);
-        std::vector<int32_t> last(nbands.size(), -1);
-        for (int b = 0; b < maxb; ++b)
-            for (size_t k = 0; k < nbands.size(); ++k)
-                if (b < nbands[k]) {
-                    entries.push_back(make_int4((int)k, b, last[k], 0));
-                    last[k] = (int32_t)entries.size() - 1;
-                }
-    } else {
-        // few (long) pairs: a list-scheduling plan pipelines each pair's bands
-        ChainPlan plan;
-        plan_chain_queue(nbands, steps, warps, 1, lead, plan);
-        entries.resize(plan.queue.size());
-        for (size_t k = 0; k < plan.queue.size(); ++k) {
-            const PlanEntry& p = plan.queue[k];
-            entries[k] = make_int4(p.item, p.chain >= 0 ? p.strip : 0, p.pred, 0);
-        }
-    }
+    std::vector<PlanEntry> plan;
+    plan_band_queue(nbands, steps, warps, lead, plan);
+    std::vector<int4> entries(plan.size());
+    for (size_t k = 0; k < plan.size(); ++k) entries[k] = make_int4(plan[k].item, plan[k].strip, plan[k].pred, 0);
     return entries;
 }
 

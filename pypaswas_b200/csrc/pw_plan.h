@@ -173,4 +173,34 @@ inline void plan_chain_queue(const std::vector<int>& nstr, const std::vector<int
     for (; wnext < whole.size(); ++wnext) out.queue.push_back(PlanEntry{whole[wnext], -1, -1, -1});
 }
 
+// The queue of a band sweep: one entry per band (item: the pair, strip: the
+// band), pair k of nbands[k] bands of steps[k] steps, pairs in priority order.
+// Every band is queued, after the band above it.
+inline void plan_band_queue(const std::vector<int>& nbands, const std::vector<int64_t>& steps, int warps, int lead,
+                            std::vector<PlanEntry>& out) {
+    out.clear();
+    if ((int64_t)nbands.size() * 2 >= warps) {
+        // many pairs: band-major order (every band 0, then every band 1, ...,
+        // longest pairs first within a band); a band's predecessor was handed
+        // out at least a whole band generation earlier, so nobody waits long
+        int maxb = 0;
+        for (int nb : nbands) maxb = std::max(maxb, nb);
+        std::vector<int32_t> last(nbands.size(), -1);
+        for (int b = 0; b < maxb; ++b)
+            for (size_t k = 0; k < nbands.size(); ++k)
+                if (b < nbands[k]) {
+                    out.push_back(PlanEntry{(int32_t)k, (int32_t)k, b, last[k]});
+                    last[k] = (int32_t)out.size() - 1;
+                }
+    } else {
+        // few (long) pairs: a list-scheduling plan pipelines each pair's bands.
+        // Every pair of several bands is a chain, however short beside the
+        // others (no threshold): a warp takes one band, not a whole pair.
+        ChainPlan plan;
+        plan_chain_queue(nbands, steps, warps, 0, lead, plan);
+        out.swap(plan.queue);
+        for (PlanEntry& p : out) p.strip = std::max(p.strip, 0);  // pairs of one band
+    }
+}
+
 }  // namespace pw
