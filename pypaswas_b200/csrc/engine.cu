@@ -2084,8 +2084,9 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
         if (p1ck) {
             // pairs that share their query and their target's length go two
             // to a 16x2 sweep and share their checkpoint words; the others,
-            // and pairs whose maximum passes the 16-bit limit, run on 32-bit lanes
-            if (!(flags & PW_FLAG_INT32) && limit > 0) {
+            // pairs whose maximum passes the 16-bit limit, and all pairs when the
+            // gap itself is no 16-bit number, run on 32-bit lanes
+            if (!(flags & PW_FLAG_INT32) && limit > 0 && e->gap >= -32768.0f) {
                 std::map<std::pair<int32_t, int32_t>, size_t> open;
                 std::vector<char> paired(np, 0);
                 for (size_t k = 0; k < np; ++k) {
