@@ -2080,13 +2080,14 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
             p.slot[0] = p.slot[1] = (int64_t)j;
             return p;
         };
-        const int limit = 32767 - (int)std::ceil(A.P.highest);
+        // (by the matrix itself: the caller's highest score may be below it)
+        const int limit = 32767 - (int)pr.maxabs;
         if (p1ck) {
             // pairs that share their query and their target's length go two
             // to a 16x2 sweep and share their checkpoint words; the others,
             // pairs whose maximum passes the 16-bit limit, and all pairs when the
             // gap itself is no 16-bit number, run on 32-bit lanes
-            if (!(flags & PW_FLAG_INT32) && limit > 0 && e->gap >= -32768.0f) {
+            if (!(flags & PW_FLAG_INT32) && e->gap >= -32768.0f) {
                 std::map<std::pair<int32_t, int32_t>, size_t> open;
                 std::vector<char> paired(np, 0);
                 for (size_t k = 0; k < np; ++k) {

@@ -45,8 +45,8 @@
 // A block's columns past the query hold decayed values; checkpoint rows are
 // (lq + 3) & ~3 wide and nothing reads those columns.
 //
-// 16-bit halves hold H exactly while every value stays at or below
-// 32767 - highest (no add can then wrap); a pair whose maximum passes that
+// 16-bit halves hold H exactly while every value stays at or below 32767 - the
+// matrix's highest score (no add can then wrap); a pair whose maximum passes that
 // limit is reported in `over` and swept again on 32-bit lanes by the host.
 #pragma once
 #include "pw_band.cuh"
@@ -74,7 +74,7 @@ struct BandCkArgs {
     float* max_out;       // pair maxima, indexed by BandCk.slot
     int* over;            // PAIR: per pair-list index, 1 when its maximum passed the 16-bit limit
     int* ck;              // checkpoints and tile maxima
-    int limit;            // PAIR: 32767 - highest substitution score
+    int limit;            // PAIR: 32767 - the matrix's largest absolute score
     unsigned long long wait_ns;
 };
 

@@ -1,6 +1,7 @@
 """The 16-bit halves of the checkpointing band sweep: gaps at and past the 16-bit
 range (listed pairs that share a query and a target length, and the same pairs
-as an unlisted call of few long sequences), against the oracle."""
+as an unlisted call of few long sequences), against the oracle; maxima around the
+16-bit limit when the caller's highest score is not the matrix's."""
 import numpy as np
 import pytest
 
@@ -8,7 +9,6 @@ from engine_helpers import decode_hits
 from pypaswas_b200 import _native
 
 pytestmark = pytest.mark.gpu
-BYTES = {c: k for k, c in enumerate(b"ACGT")}
 
 
 def _matrix(match, mismatch):
@@ -56,3 +56,18 @@ def test_gaps_past_16_bits(engine_lib, oracle_mod, gap, listed):
         ref = oracle_mod.run(p, [q[a].decode()], [t[b].decode()], pos, 60.0)
         assert pm[a, b] == ref["pair_max"][0, 0]
         assert [h for h in hits if h["target"] == b] == [dict(h, query=a, target=b) for h in ref["hits"]]
+
+
+@pytest.mark.parametrize("highest", [-3.0, 1.0, 127.0, 1.0e6, 1.0e12])
+@pytest.mark.parametrize("length", [256, 257, 258, 259, 400])
+def test_limit_is_the_matrix_own(engine_lib, highest, length):
+    # identical sequences: the maximum is 127 a residue; 258 of them are past the limit
+    q = [_bases(np.random.default_rng(length), length)]
+    e = _engine(engine_lib, q, [q[0], q[0]], _matrix(127.0, -100.0), -100.0, 1.0e9, highest, [(0, 0), (0, 1)])
+    try:
+        info = e.align(score_only=True)
+        pm = e.pair_max()
+    finally:
+        e.close()
+    assert info.overflow_pairs == (2 if length >= 258 else 0)
+    assert pm.tolist() == [[127.0 * length] * 2]
