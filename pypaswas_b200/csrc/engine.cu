@@ -439,7 +439,10 @@ static void time_until(pw_engine* e, cudaEvent_t from, double* ms) {
 static void settle_times(pw_engine* e, bool read = true) {
     for (const pw_engine::Interval& i : e->intervals) {
         float ms = 0;
-        if (read && cudaEventElapsedTime(&ms, i.a, i.b) == cudaSuccess && i.ms) *i.ms += ms;
+        if (read && cudaEventElapsedTime(&ms, i.a, i.b) != cudaSuccess)
+            cudaGetLastError();  // no later check takes it for its own
+        else if (read && i.ms)
+            *i.ms += ms;
         e->idle_events.push_back(i.a);
         e->idle_events.push_back(i.b);
     }
@@ -2334,6 +2337,8 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
             return cuda_fail(e, c, "upload pair maxima");
     }
     if (flags & PW_FLAG_SCORE_ONLY) {
+        // the closing event, and the 32-bit sweep of pairs past the 16-bit limit, are still under way
+        if ((c = cudaStreamSynchronize(e->stream)) != cudaSuccess) return cuda_fail(e, c, "score sweep");
         settle_times(e);
         inf.kernel_launches = (int32_t)e->launches;
         inf.total_ms = wall_ms() - t_call;
