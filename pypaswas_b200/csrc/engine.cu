@@ -752,7 +752,7 @@ static cudaError_t download(pw_engine* e, std::vector<HT>& v, const void* src, s
 // Small arrays gathered into a page-locked staging buffer and copied with one
 // call into one device block; each gets its place in the block.  The staging
 // buffer is not reused before the stream has been synchronised (every pw_align
-// ends so, and a set is prepared at most once in it).
+// ends so, failed ones too, and a set is prepared at most once in it).
 struct Staged {
     struct Item {
         DevView* dst;
@@ -1973,17 +1973,12 @@ static int emit_key_less(const StartRec& a, const StartRec& b) {
 }
 
 
-extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_info* info) {
-    if (!e) return PW_ERR_ARG;
+static int align_call(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_info* info) {
     const double t_call = wall_ms();
     if (!e->scoring_set) return fail(e, PW_ERR_STATE, "pw_set_scoring was not called");
     if (!e->Q.set || !e->T.set) return fail(e, PW_ERR_STATE, "queries and targets must be set");
     if (cudaSetDevice(e->device) != cudaSuccess) return fail(e, PW_ERR_DEVICE, "cudaSetDevice failed");
     e->err.clear();
-    if (!e->intervals.empty() || !e->started.empty()) {  // left by a call that failed
-        cudaStreamSynchronize(e->stream);
-        settle_times(e, false);
-    }
     e->abort_unread = false;
     e->h_hits.clear();
     e->h_strings.clear();
@@ -3167,6 +3162,18 @@ extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_
     inf.reuse = e->reuse;
     if (info) *info = inf;
     return PW_OK;
+}
+
+// A call ends with its stream idle, also where it failed with copies and
+// kernels under way: the next one writes to the page-locked arrays they read.
+extern "C" int pw_align(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_info* info) {
+    if (!e) return PW_ERR_ARG;
+    const int rc = align_call(e, flags, start_cap, info);
+    if (rc != PW_OK && cudaSetDevice(e->device) == cudaSuccess) {
+        cudaStreamSynchronize(e->stream);
+        settle_times(e, false);
+    }
+    return rc;
 }
 
 extern "C" int pw_set_query_trace(pw_engine* e, const uint8_t* mask, int32_t n) {
