@@ -2190,11 +2190,19 @@ static int align_call(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_in
                     inf.paired_cells -= (int64_t)lq * lt;
                 }
                 if (!again.empty()) {
-                    if ((c = e->p1_ck.grow_keep(e->stream, (size_t)ck_ints * sizeof(int), (size_t)end * sizeof(int))) !=
-                            cudaSuccess ||
-                        (c = cudaMemsetAsync(e->p1_ck.as<int>() + ck_ints, 0, (size_t)(end - ck_ints) * sizeof(int),
-                                             e->stream)) != cudaSuccess)
+                    // (their words are not shared: up to three times the paired layout's in
+                    // all, within the same share of the memory or not kept)
+                    if ((double)end * (double)sizeof(int) > 0.35 * (double)e->p1_free) {
+                        p1ck = false;
+                    } else if ((c = e->p1_ck.grow_keep(e->stream, (size_t)ck_ints * sizeof(int),
+                                                       (size_t)end * sizeof(int))) == cudaErrorMemoryAllocation) {
+                        cudaGetLastError();
+                        p1ck = false;
+                    } else if (c != cudaSuccess ||
+                               (c = cudaMemsetAsync(e->p1_ck.as<int>() + ck_ints, 0,
+                                                    (size_t)(end - ck_ints) * sizeof(int), e->stream)) != cudaSuccess) {
                         return cuda_fail(e, c, "alloc checkpoints");
+                    }
                     for (BandCk& p : again) {
                         pw_engine::P1Ck& o = e->p1_pairs[(size_t)p.slot[0]];
                         o.rows = p.rows;
@@ -2205,7 +2213,15 @@ static int align_call(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_in
                     }
                 }
             }
-            rc = run_band_ck_phase<false>(e, A, bp1, limit, &inf.score_kernel_ms, &inf.score_launches);
+            if (p1ck) {
+                rc = run_band_ck_phase<false>(e, A, bp1, limit, &inf.score_kernel_ms, &inf.score_launches);
+            } else {
+                // no room for these pairs' checkpoints: their maxima alone, and the
+                // traced pairs of the call get the checkpoint sweep
+                std::vector<BandPair> rest;
+                for (const BandCk& p : bp1) rest.push_back(bp[(size_t)p.slot[0]]);
+                rc = run_band_phase<0>(e, A, rest, &inf.score_kernel_ms, &inf.score_launches);
+            }
         } else {
             rc = run_band_phase<0>(e, A, bp, &inf.score_kernel_ms, &inf.score_launches);
         }
