@@ -230,7 +230,10 @@ int pw_set_wave_limit(pw_engine* e, int64_t bytes);
 /*   PW_TUNE_STALL_TEST  1: the next chained launch makes one queue entry wait
  *                       on a progress flag that nothing sets, so that its wait
  *                       runs out (PW_TUNE_WAIT_NS) and pw_align reports the
- *                       failure; a test of the bounded waits.  0: off */
+ *                       failure; 2: the next sweep of listed or affine pairs
+ *                       makes one band read its row above where nothing is
+ *                       stored, with the same end; tests of the bounded waits.
+ *                       0: off */
 #define PW_TUNE_STALL_TEST 6
 /*   PW_TUNE_LANES       score sweep lane width: 32 runs it on 32-bit lanes as
  *                       PW_FLAG_INT32 does; 0 the 16x2 sweep wherever the

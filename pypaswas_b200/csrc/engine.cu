@@ -1406,7 +1406,7 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
         S.run_max = e->chain_max.as<uint32_t>();
         S.abort_flag = e->chain_abort.as<int>();
         S.n_chain_items = P1.n_chain_items;
-        if (e->tune[PW_TUNE_STALL_TEST]) {
+        if (e->tune[PW_TUNE_STALL_TEST] == 1) {
             // one entry with a predecessor waits on the spare flag instead
             e->tune[PW_TUNE_STALL_TEST] = 0;
             std::vector<int4> info = e->h_chain_info;
@@ -1660,6 +1660,23 @@ static std::vector<int4> band_queue(const std::vector<int>& nbands, const std::v
     return entries;
 }
 
+// PW_TUNE_STALL_TEST 2: the first entry whose band is the last of several of its
+// pair gets a pair record of its own (appended to `pairs`), whose row above the
+// caller places where nothing is stored; -1: no such entry.
+template <typename Pair>
+static int stalled_row(pw_engine* e, std::vector<int4>& entries, std::vector<Pair>& pairs) {
+    if (e->tune[PW_TUNE_STALL_TEST] != 2) return -1;
+    for (int4& v : entries)
+        if (v.y > 0 && v.y + 1 == pairs[v.x].nbands) {
+            e->tune[PW_TUNE_STALL_TEST] = 0;
+            const Pair p = pairs[v.x];
+            pairs.push_back(p);
+            v.x = (int)pairs.size() - 1;
+            return v.x;
+        }
+    return -1;
+}
+
 // Warps of a block whose warps take `warp_smem` bytes of shared memory each:
 // four, fewer where large alphabets' profiles leave room for fewer.
 constexpr int kBlockSmem = 227 * 1024;
@@ -1761,7 +1778,7 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
             if (entries[k].y >= hold) entries[k].w = at[pair][entries[k].y - hold];
         }
     }
-    if (e->tune[PW_TUNE_STALL_TEST]) {
+    if (e->tune[PW_TUNE_STALL_TEST] == 1) {
         // one band below another waits on the spare flag (index n) instead
         for (int4& v : entries)
             if (v.y > 0) {
@@ -1769,6 +1786,14 @@ static int run_band_phase(pw_engine* e, KernelArgs A, std::vector<BandPair>& pai
                 v.z = (int)n;
                 break;
             }
+    }
+    if (aff_ints) {
+        const int x = stalled_row(e, entries, sorted);
+        if (x >= 0) {  // a row behind the rings, cleared like them
+            const int64_t nblk = affine_blocks(e->pr.qlen[sorted[x].q]);
+            sorted[x].ring_off = ring_elems - (sorted[x].nbands - 2) % sorted[x].rows * nblk;
+            ring_elems += nblk;
+        }
     }
     if ((c = upload(e, e->band_pairs, sorted)) != cudaSuccess) return cuda_fail(e, c, "upload band pairs");
     if ((c = upload(e, e->band_entries, entries)) != cudaSuccess) return cuda_fail(e, c, "upload band queue");
@@ -1855,7 +1880,7 @@ static int run_band_ck_phase(pw_engine* e, KernelArgs A, const std::vector<BandC
     }
     std::vector<int4> entries = band_queue(nstr, xm, warps, kBandCkLead);
     const size_t n = entries.size();
-    if (e->tune[PW_TUNE_STALL_TEST]) {
+    if (e->tune[PW_TUNE_STALL_TEST] == 1) {
         // one band below another waits on the spare flag (index n) instead
         for (int4& v : entries)
             if (v.y > 0) {
@@ -1863,6 +1888,14 @@ static int run_band_ck_phase(pw_engine* e, KernelArgs A, const std::vector<BandC
                 v.z = (int)n;
                 break;
             }
+    }
+    const int x = stalled_row(e, entries, sorted);
+    if (x >= 0) {  // a cleared row behind the checkpoints
+        const int64_t stride = tile_row_stride(e->pr.qlen[sorted[x].q]), at = align_up((int64_t)e->p1_ck.bytes, 16);
+        if ((c = e->p1_ck.grow_keep(e->stream, e->p1_ck.bytes, (size_t)(at + stride * 4))) != cudaSuccess ||
+            (c = cudaMemsetAsync(e->p1_ck.as<char>() + at, 0, (size_t)stride * 4, e->stream)) != cudaSuccess)
+            return cuda_fail(e, c, "alloc a silent row");
+        sorted[x].rows = at / 4 - (sorted[x].nbands - 2) * stride;
     }
     if ((c = upload(e, e->band_pairs, sorted)) != cudaSuccess) return cuda_fail(e, c, "upload band pairs");
     if ((c = upload(e, e->band_entries, entries)) != cudaSuccess) return cuda_fail(e, c, "upload band queue");
