@@ -1147,10 +1147,8 @@ static cudaError_t launch_s16(pw_engine* e, int form, int rows, const Score16Arg
 // Plans the multi-strip launch.  Items whose sweep cost (columns x strips)
 // reaches `min_permille`/1000 of the mean per-warp load are cut into chains of
 // one-strip entries (score16_chain_kernel); the others stay whole.  The queue
-// order comes from a list-scheduling simulation of `warps` equally fast warps:
-// a free warp takes the next strip of the largest chain whose predecessor is
-// at least kChainLead columns ahead, else the next whole item (longest first),
-// else the strip that becomes ready first.  Every strip is queued after its
+// order is plan_chain_queue's (pw_plan.h): by levels with enough chains, else
+// the chain with the longest way to go first.  Every strip is queued after its
 // predecessor, which is what the kernel's waits rely on.
 static int setup_chains(pw_engine* e, const std::vector<WorkItem>& items, int i0, int i1,
                         const std::vector<int32_t>& strip_len, int warps, int* n_entries) {
@@ -1687,8 +1685,9 @@ static int block_warps(int warp_smem) {
 // Boundary rows of a band sweep's pairs at most (two rows a pair are always given).
 constexpr int64_t kRingBytes = (int64_t)8 << 30;
 
-// Launches band_kernel over `pairs` (one warp per band, the bands of a pair
-// chained across warps, pw_band.cuh).  DIRS 1: the direction sweep of traced
+// Launches the band sweep of `pairs` (one warp per band, the bands of a pair
+// chained across warps): band_kernel for linear, band_affine_kernel for affine
+// integer scores, band_float_kernel for others.  DIRS 1: the direction sweep of traced
 // pairs (cell codes), 2: the same storing H (linear gap), 3: the checkpoint
 // sweep of the tile form (linear gap, checkpoints into tile_ck); 0: pair
 // maxima into band_out (indexed by BandPair.slot).
@@ -2729,7 +2728,7 @@ static int align_call(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_in
                 } else {
                     tp.rows = ck_ints;
                     tp.cols = ck_ints + tile_row_ints(lq_, lt_);
-                    wi[k].dir_base = ck_ints;  // band_kernel<false, 3>: the pair's checkpoints
+                    wi[k].dir_base = ck_ints;  // band_kernel<3>: the pair's checkpoints
                     ck_ints += tile_checkpoint_ints(lq_, lt_);
                 }
                 tps.push_back(tp);

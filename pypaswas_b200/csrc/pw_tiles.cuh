@@ -3,8 +3,8 @@
 // The band direction sweep of a long pair stores a 4-bit code for every cell
 // (a 30 kb x 30 kb pair: 450 MB), and the walks then follow their paths one
 // dependent global load a step.  The tile form stores no cell codes: the
-// checkpoint sweep (band_kernel<false, 3>, or the score sweep of listed pairs
-// itself, pw_band_ck.cuh) keeps every band's bottom row and, per band, the H
+// checkpoint sweep (band_kernel<3>, or the score sweep of listed pairs itself,
+// pw_band_ck.cuh) keeps every band's bottom row and, per band, the H
 // column at every kTileW-th column.  From those, one warp recomputes the codes
 // of any 256 x kTileW tile -- the same codes, bit for bit, as the direction
 // sweep (same recurrence, same boundary values, same classification): 16 KB,
