@@ -1220,9 +1220,10 @@ static double dual_cost(const std::vector<int32_t>& strip_len, const std::vector
 // rows instead of one 128-bit load).
 constexpr double kDualSlotCost = 1.15;
 
-// Pair maxima with the 16-bit dual-pair sweep.  Returns the device time of
-// the sweep launches in *kernel_ms.  Pairs whose maximum could overflow
-// 16-bit halves come back as NaN; they are recomputed by the 32-bit sweep.
+// Pair maxima with the 16-bit dual-pair sweep.  Pairs whose maximum could
+// overflow 16-bit halves come back as NaN; they are recomputed by the 32-bit
+// sweep.  The phase's interval (score_ms) closes before the read that ends it,
+// which leaves the stream idle (a further synchronisation cost a 0.38 ms call 10 us).
 static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uint32_t flags) {
     const Prepared& pr = e->pr;
     const int nq = e->Q.n, nt = e->T.n;
@@ -1233,6 +1234,7 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
                        P1.flags == pflags && P1.tune == e->tune[PW_TUNE_CHAIN_MIN] &&
                        P1.share == e->tune[PW_TUNE_GRID_SHARE] && P1.dual_mode == e->tune[PW_TUNE_DUAL];
     cudaError_t c;
+    const cudaEvent_t phase_from = time_from(e);
     if (reuse) e->reuse |= PW_REUSE_PLAN;
     if (!reuse) {
         const double t_plan = wall_ms();
@@ -1469,6 +1471,7 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
         inf.score_launches++;
     }
     time_until(e, from, &inf.score_kernel_ms);
+    time_until(e, phase_from, &inf.score_ms);
     int status[2] = {0, 0};  // overflow count, chain abort flag
     SmallReads rd;
     rd.add(&status[0], S.ovf_count, sizeof(int));
@@ -1478,15 +1481,15 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
     // the maxima stay on the device (pruning reads them there); the host
     // copy is needed only to find the pairs that reached the 16-bit limit
     e->pm_stale = true;
-    if (status[0] > 0) {
-        const int rc = sync_pair_max(e, A32.pair_max);
-        if (rc != PW_OK) return rc;
-    }
+    if (status[0] <= 0) return PW_OK;
+    const cudaEvent_t again_from = time_from(e);
+    int rc = sync_pair_max(e, A32.pair_max);
+    if (rc != PW_OK) return rc;
 
     // pairs that reached the 16-bit limit: the 32-bit sweep, per target
     std::vector<std::vector<int32_t>> ovf(nt);
     int64_t n_ovf = 0;
-    for (int sp = 0; sp < nq && status[0] > 0; ++sp) {
+    for (int sp = 0; sp < nq; ++sp) {
         const int q = pr.order[sp];
         for (int t = 0; t < nt; ++t)
             if (std::isnan(e->h_pair_max[(size_t)q * nt + t])) {
@@ -1495,7 +1498,6 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
             }
     }
     inf.overflow_pairs = n_ovf;
-    if (n_ovf == 0) return PW_OK;
     std::vector<int32_t> order2;
     std::vector<WorkItem> its;
     std::vector<int> cl;
@@ -1521,9 +1523,11 @@ static int phase1_s16(pw_engine* e, const KernelArgs& A32, pw_run_info& inf, uin
     if ((c = upload(e, e->items, its)) != cudaSuccess) return cuda_fail(e, c, "upload items");
     KernelArgs A = A32;
     A.q_order = e->q_order2.as<int32_t>();
-    int rc = run_phase<1>(e, A, e->items.as<WorkItem>(), bg, xm, &inf.score_kernel_ms, &inf.score_launches);
+    rc = run_phase<1>(e, A, e->items.as<WorkItem>(), bg, xm, &inf.score_kernel_ms, &inf.score_launches);
     if (rc != PW_OK) return rc;
+    time_until(e, again_from, &inf.score_ms);
     e->pm_stale = true;
+    if ((c = cudaStreamSynchronize(e->stream)) != cudaSuccess) return cuda_fail(e, c, "score sweep");
     return PW_OK;
 }
 
@@ -2301,10 +2305,8 @@ static int align_call(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_in
         cudaEventElapsedTime(&ms, e->ev[0], e->ev[1]);
         inf.score_ms = ms;
     } else if (use_s16) {
-        const cudaEvent_t from = time_from(e);
         rc = phase1_s16(e, A, inf, flags);
         if (rc != PW_OK) return rc;
-        time_until(e, from, &inf.score_ms);
         ht0.mark("score phase (16-bit, wall)");
     } else {
         inf.score_path = 1;
@@ -2380,9 +2382,7 @@ static int align_call(pw_engine* e, uint32_t flags, int64_t start_cap, pw_run_in
             return cuda_fail(e, c, "upload pair maxima");
     }
     if (flags & PW_FLAG_SCORE_ONLY) {
-        // the closing event, and the 32-bit sweep of pairs past the 16-bit limit, are still under way
-        if ((c = cudaStreamSynchronize(e->stream)) != cudaSuccess) return cuda_fail(e, c, "score sweep");
-        settle_times(e);
+        settle_times(e);  // (every form of the score phase ends with the stream idle)
         inf.kernel_launches = (int32_t)e->launches;
         inf.total_ms = wall_ms() - t_call;
         inf.h2d_bytes = e->h2d;
